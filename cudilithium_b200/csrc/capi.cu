@@ -75,13 +75,12 @@ __global__ void __launch_bounds__(kBlock) k_derive_rhoprime(uint8_t *out, size_t
 // would take 64 registers.
 __global__ void __launch_bounds__(kBlock) k_ntt_mul(const int32_t *a, const int32_t *b, int32_t *out, long long npolys) {
     __shared__ int32_t sm[kGroupsPerBlock * NTT_SMEM_WORDS];
-    // twiddle rows (forward, inverse) of the 16 group positions; chunk c (16 bytes) of row t is
-    // stored at chunk (c + t) mod 8, so that the positions' reads of one chunk spread over the banks
-    __shared__ __align__(16) int4 s_tw[2][16][8];
+    // twiddle chunks (forward, inverse) of the 16 group positions, as in the table: the positions'
+    // reads of one chunk are contiguous
+    __shared__ __align__(16) int4 s_tw[2][8][16];
     for (int k = threadIdx.x; k < 2 * 16 * 8; k += blockDim.x) {
-        const int dir = k >> 7, t = (k >> 3) & 15, c = k & 7;
-        const int4 *src = reinterpret_cast<const int4 *>(dir ? g_group_tw.inv[t] : g_group_tw.fwd[t]);
-        s_tw[dir][t][(c + t) & 7] = src[c];
+        const int dir = k >> 7, c = (k >> 4) & 7, t = k & 15;
+        s_tw[dir][c][t] = dir ? g_group_tw.inv[c][t] : g_group_tw.fwd[c][t];
     }
     __syncthreads();
     const long long groups = (long long)gridDim.x * (blockDim.x >> 4);
@@ -91,7 +90,7 @@ __global__ void __launch_bounds__(kBlock) k_ntt_mul(const int32_t *a, const int3
     auto tw_row = [&](int dir, int2 (&tw)[16]) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            const int4 v = s_tw[dir][g.t][(c + g.t) & 7];
+            const int4 v = s_tw[dir][c][g.t];
             tw[2 * c] = make_int2(v.x, v.y);
             tw[2 * c + 1] = make_int2(v.z, v.w);
         }

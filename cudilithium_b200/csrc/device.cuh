@@ -58,7 +58,7 @@ __device__ __forceinline__ void expand_a_stream(const uint2 (&rho)[4], int i, in
     }
 }
 
-// The same entry written to out[0..255].  Where out is 16-byte aligned, a group of eight
+// The same entry, times the inverse transform's factor f (scale_f), written to out[0..255].  Where out is 16-byte aligned, a group of eight
 // candidates that are all accepted while the count is a multiple of four goes out as two 16-byte
 // stores; anything else is stored coefficient by coefficient (a candidate is rejected with
 // probability (2^23 - q) / 2^23 < 0.1%, so nearly every group takes the wide path).
@@ -91,14 +91,17 @@ __device__ __forceinline__ void expand_a_row(const uint2 (&rho)[4], int i, int j
             }
             if (wide && all && (ctr & 3) == 0 && ctr + 8 <= N) {
                 int4 *o = reinterpret_cast<int4 *>(out + ctr);
-                o[0] = make_int4((int)c[0], (int)c[1], (int)c[2], (int)c[3]);
-                o[1] = make_int4((int)c[4], (int)c[5], (int)c[6], (int)c[7]);
+                int32_t v[8];
+#pragma unroll
+                for (int m = 0; m < 8; ++m) v[m] = scale_f((int32_t)c[m]);
+                o[0] = make_int4(v[0], v[1], v[2], v[3]);
+                o[1] = make_int4(v[4], v[5], v[6], v[7]);
                 ctr += 8;
             } else {
 #pragma unroll
                 for (int m = 0; m < 8; ++m) {
                     if (c[m] < (uint32_t)Q && ctr < N) {
-                        out[ctr] = (int32_t)c[m];
+                        out[ctr] = scale_f((int32_t)c[m]);
                         ++ctr;
                     }
                 }
@@ -219,12 +222,30 @@ __device__ __forceinline__ void strided_to_contig(const Group &g, const int32_t 
     __syncwarp(g.gmask);
 }
 
+// Fields t + 16 i (i = 0..15) of a packed array of BITS-bit fields, BITS even: sixteen fields are
+// BITS / 2 whole words, so all the fields of position t sit at the same shift in words BITS / 2 apart,
+// and two word loads and a funnel shift read one (three or four byte loads, shifts and ORs before).
+// The array may start at any byte: the words are the aligned ones that hold it.  A word is read only if
+// it holds bits of the field, so nothing past the array's last aligned word is touched.
+template <int BITS>
+__device__ __forceinline__ void unpack_strided(uint32_t (&v)[16], const uint8_t *packed, int t) {
+    static_assert(BITS % 2 == 0 && BITS <= 20, "whole words every sixteen fields");
+    const unsigned mis = (unsigned)(reinterpret_cast<uintptr_t>(packed) & 3u);
+    const unsigned bit = 8u * mis + (unsigned)(BITS * t), sh = bit & 31u;
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(packed - mis) + (bit >> 5);
+    const int second = sh + BITS > 32u ? 1 : 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        v[i] = __funnelshift_r(w[(BITS / 2) * i], w[(BITS / 2) * i + second], sh) & ((1u << BITS) - 1u);
+}
+
 // z coefficients a[t + 16 i] from a packed (gamma1 - z) polynomial.
 template <int MODE>
 __device__ __forceinline__ void unpack_z_strided(int32_t (&x)[16], const uint8_t *packed, int t) {
-    constexpr int ZB = P<MODE>::Z_BITS;
+    uint32_t v[16];
+    unpack_strided<P<MODE>::Z_BITS>(v, packed, t);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) x[i] = Params<MODE>::GAMMA1 - (int32_t)get_bits(packed, (t + 16 * i) * ZB, ZB);
+    for (int i = 0; i < 16; ++i) x[i] = Params<MODE>::GAMMA1 - (int32_t)v[i];
 }
 
 // z coefficients a[16 t + i] (the contiguous slice of group thread t) from a packed (gamma1 - z)
@@ -244,16 +265,6 @@ __device__ __forceinline__ void unpack_z_contig(int32_t (&x)[16], const uint8_t 
         const uint32_t r = __funnelshift_r(v[wi], v[wi + 1], sh) & ((1u << ZB) - 1u);
         x[i] = Params<MODE>::GAMMA1 - (int32_t)r;
     }
-}
-
-// Inverse of strided_to_contig: y[i] = a[16 t + i] -> x[i] = a[t + 16 i].
-__device__ __forceinline__ void contig_to_strided(const Group &g, const int32_t (&y)[16], int32_t (&x)[16]) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) g.sm[17 * g.t + i] = y[i];
-    __syncwarp(g.gmask);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) x[i] = g.sm[g.t + 17 * i];
-    __syncwarp(g.gmask);
 }
 
 // c coefficients a[t + 16 i] from the challenge masks (occupied bits, negative bits).

@@ -168,11 +168,18 @@ __global__ void __launch_bounds__(kBlock) k_cache_pk_t1(const uint8_t *pk, uint8
     Group g = make_group(sm, threadIdx.x >> 4);
     const uint8_t *t1p = pk + (size_t)it * PM::PK_BYTES + SEEDBYTES + (size_t)i * POLYT1_PACKED;
     int32_t x[16];
+    if ((reinterpret_cast<uintptr_t>(t1p) & 3u) == 0u) {
+        uint32_t v[16];
+        unpack_strided<10>(v, t1p, g.t);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-        const int bit = (g.t + 16 * m) * 10, byte = bit >> 3, sh = bit & 7;
-        const uint32_t v = ((uint32_t)t1p[byte] | ((uint32_t)t1p[byte + 1] << 8)) >> sh;  // sh + 10 <= 16
-        x[m] = (int32_t)((v & 0x3FFu) << D);
+        for (int m = 0; m < 16; ++m) x[m] = (int32_t)(v[m] << D);
+    } else {  // the last key's words would reach past the buffer
+#pragma unroll
+        for (int m = 0; m < 16; ++m) {
+            const int bit = (g.t + 16 * m) * 10, byte = bit >> 3, sh = bit & 7;
+            const uint32_t v = ((uint32_t)t1p[byte] | ((uint32_t)t1p[byte + 1] << 8)) >> sh;  // sh + 10 <= 16
+            x[m] = (int32_t)((v & 0x3FFu) << D);
+        }
     }
     ntt16s(x, g.sm, g.gmask, g.t);
     store16_contig(reinterpret_cast<int32_t *>(rows + (size_t)it * pitch + C::PK_T1 + (size_t)i * C::POLY) + 16 * g.t, x);
@@ -589,6 +596,8 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
         int32_t ch[16];
         challenge_strided(ch, masks, g.t);
         fwd(ch);
+#pragma unroll
+        for (int m = 0; m < 16; ++m) ch[m] = scale_f(ch[m]);
         const int32_t *s1 = reinterpret_cast<const int32_t *>(row + C::SK_S1);
         const int32_t *s2 = reinterpret_cast<const int32_t *>(row + C::SK_S2);
         const int32_t *t0 = reinterpret_cast<const int32_t *>(row + C::SK_T0);
@@ -782,35 +791,14 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
 #pragma unroll 1
         for (int i = 0; i < K; ++i) {
             int32_t acc[16];
-#pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] = 0;
-            // A row entries in chunks of up to four polynomials: their loads are all in flight
-            // before the first one is consumed
-#pragma unroll 1
-            for (int j0 = 0; j0 < L; j0 += 4) {
-                int32_t av[4][16];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj)
-                    if (j0 + jj < L) load16_contig(av[jj], mat0 + ((size_t)i * L + j0 + jj) * N + 16 * g.t);
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    if (j0 + jj < L) {
-                        int32_t yv[16];
-                        load16_smem(yv, yh + (j0 + jj) * N, g.t);
-#pragma unroll
-                        for (int m = 0; m < 16; ++m) acc[m] += montmul(av[jj][m], yv[m]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] = reduce32(acc[m]);
+            dot16<L, (L + 1) / 2>(acc, yh, g.t, [&](int j) { return mat0 + ((size_t)i * L + j) * N; });
             inv(acc);
             int32_t *w0 = reinterpret_cast<int32_t *>(slot + C::SL_W0) + (size_t)i * N;
             int32_t w1[16];
 #pragma unroll
             for (int m = 0; m < 16; ++m) {
                 int32_t a0;
-                w1[m] = decompose<MODE>(a0, caddq(acc[m]));
+                w1[m] = decompose<MODE>(a0, caddq(reduce32(acc[m])));
                 w0[g.t + 16 * m] = a0;
             }
             int32_t w1c[16];
@@ -1002,14 +990,9 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_verify(const u
 #pragma unroll 1
                 for (int j = 0; j < L; ++j) {
                     int32_t x[16];
+                    unpack_z_strided<MODE>(x, s + PM::SIG_Z + (size_t)j * PM::POLYZ_PACKED, g.t);
 #pragma unroll
-                    for (int m = 0; m < 16; ++m) {
-                        const int bit = (g.t + 16 * m) * PM::Z_BITS;
-                        const uint8_t *pz = s + PM::SIG_Z + (size_t)j * PM::POLYZ_PACKED + (bit >> 3);
-                        const uint32_t v = ((uint32_t)pz[0] | ((uint32_t)pz[1] << 8) | ((uint32_t)pz[2] << 16)) >> (bit & 7);
-                        x[m] = PM::GAMMA1 - (int32_t)(v & ((1u << PM::Z_BITS) - 1u));
-                        zbad |= exceeds(x[m], PM::GAMMA1 - PM::BETA);
-                    }
+                    for (int m = 0; m < 16; ++m) zbad |= exceeds(x[m], PM::GAMMA1 - PM::BETA);
                     ntt16s(x, g.sm, g.gmask, g.t);
                     store16_smem(zh + j * N, x, g.t);
                 }
@@ -1028,6 +1011,9 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_verify(const u
                     int32_t x[16];
                     challenge_strided(x, masks, g.t);
                     ntt16s(x, g.sm, g.gmask, g.t);
+                    // -c_hat with the inverse transform's factor (A_hat carries it already)
+#pragma unroll
+                    for (int m = 0; m < 16; ++m) x[m] = -scale_f(x[m]);
                     store16_smem(zh + L * N, x, g.t);
                 }
                 __syncwarp(g.gmask);
@@ -1042,54 +1028,16 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_verify(const u
                     for (int j = start + g.t; j < end; j += 16) atomicOr(&hbits[h[j] >> 5], 1u << (h[j] & 31));
                     __syncwarp(g.gmask);
                     const int32_t *mat = reinterpret_cast<const int32_t *>(row + C::PK_MAT) + (size_t)i * L * N;
-                    int32_t acc[16];
-#pragma unroll
-                    for (int m = 0; m < 16; ++m) acc[m] = 0;
-                    // sum_j A_ij z_j - c t1_i, the key operands in chunks of up to four polynomials
-                    // whose loads are all in flight before the first one is consumed (one memory
-                    // round trip per chunk).  When L is not a multiple of four, t1_i joins the last
-                    // chunk of A row entries as operand L (its shared-memory vector, after
-                    // z_hat_0..L-1, is c_hat); otherwise it would start a chunk of its own, and
-                    // the separate load below measured faster.  The int32 sum is exact
-                    // (|acc| < (L+1) q), so both forms give the same result.
+                    // sum_j A_ij z_j - c t1_i: t1_i is operand L, whose shared-memory vector is -c_hat
                     const int32_t *t1 = reinterpret_cast<const int32_t *>(row + C::PK_T1) + (size_t)i * N;
-                    constexpr int LAST = (L % 4 == 0) ? L - 1 : L;  // last operand in the chunks
-#pragma unroll 1
-                    for (int j0 = 0; j0 <= LAST; j0 += 4) {
-                        int32_t av[4][16];
-#pragma unroll
-                        for (int jj = 0; jj < 4; ++jj)
-                            if (j0 + jj <= LAST) load16_contig(av[jj], (j0 + jj < L ? mat + (size_t)(j0 + jj) * N : t1) + 16 * g.t);
-#pragma unroll
-                        for (int jj = 0; jj < 4; ++jj) {
-                            if (j0 + jj <= LAST) {
-                                int32_t zv[16];
-                                load16_smem(zv, zh + (j0 + jj) * N, g.t);
-                                if (j0 + jj < L) {
-#pragma unroll
-                                    for (int m = 0; m < 16; ++m) acc[m] += montmul(av[jj][m], zv[m]);
-                                } else {
-#pragma unroll
-                                    for (int m = 0; m < 16; ++m) acc[m] -= montmul(zv[m], av[jj][m]);
-                                }
-                            }
-                        }
-                    }
-                    if constexpr (LAST < L) {
-                        int32_t cv[16], tv[16];
-                        load16_smem(cv, zh + L * N, g.t);
-                        load16_contig(tv, t1 + 16 * g.t);
-#pragma unroll
-                        for (int m = 0; m < 16; ++m) acc[m] -= montmul(cv[m], tv[m]);
-                    }
-#pragma unroll
-                    for (int m = 0; m < 16; ++m) acc[m] = reduce32(acc[m]);
+                    int32_t acc[16];
+                    dot16<L + 1, (L + 2) / 2>(acc, zh, g.t, [&](int j) { return j < L ? mat + (size_t)j * N : t1; });
                     intt16s(acc, g.sm, g.gmask, g.t);
                     int32_t w1[16];
 #pragma unroll
                     for (int m = 0; m < 16; ++m) {
                         const int c = g.t + 16 * m;
-                        w1[m] = use_hint<MODE>(caddq(acc[m]), (hbits[c >> 5] >> (c & 31)) & 1u);
+                        w1[m] = use_hint<MODE>(caddq(reduce32(acc[m])), (hbits[c >> 5] >> (c & 31)) & 1u);
                     }
                     int32_t w1c[16];
                     strided_to_contig(g, w1, w1c);

@@ -275,9 +275,8 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512) ? 1 : 512 / THREADS)
         for (int j0 = 0; j0 < L; j0 += 2) {
             const int j = j0 + half;
             if (j < L) {
-                int32_t yc[16], x[16];
-                unpack_z_contig<MODE>(yc, slot + C::SL_Y + (size_t)j * PM::POLYZ_PACKED, g.t);
-                contig_to_strided(g, yc, x);
+                int32_t x[16];
+                unpack_z_strided<MODE>(x, slot + C::SL_Y + (size_t)j * PM::POLYZ_PACKED, g.t);
                 ntt16_ool(x, g.sm, g.gmask, g.t);
                 store16_smem(yh + j * N, x, g.t);
             }
@@ -288,32 +287,13 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512) ? 1 : 512 / THREADS)
         for (int i0 = 0; i0 < K; i0 += 2) {
             const int i = i0 + half;  // K is even
             int32_t acc[16];
-#pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] = 0;
-#pragma unroll 1
-            for (int j0 = 0; j0 < L; j0 += 4) {
-                int32_t av[4][16];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj)
-                    if (j0 + jj < L) load16_contig(av[jj], mat0 + ((size_t)i * L + j0 + jj) * N + 16 * g.t);
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    if (j0 + jj < L) {
-                        int32_t yv[16];
-                        load16_smem(yv, yh + (j0 + jj) * N, g.t);
-#pragma unroll
-                        for (int m = 0; m < 16; ++m) acc[m] += montmul(av[jj][m], yv[m]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] = reduce32(acc[m]);
+            dot16<L, (L + 1) / 2>(acc, yh, g.t, [&](int j) { return mat0 + ((size_t)i * L + j) * N; });
             intt16_ool(acc, g.sm, g.gmask, g.t);
             // w0 and w1 bytes thread-major (thread t's strided coefficients t + 16 m contiguous)
             int4 *w0t = reinterpret_cast<int4 *>(slot + C::SL_W0 + (size_t)i * C::POLY) + 4 * g.t;
             int32_t w1[16], a0[16];
 #pragma unroll
-            for (int m = 0; m < 16; ++m) w1[m] = decompose<MODE>(a0[m], caddq(acc[m]));
+            for (int m = 0; m < 16; ++m) w1[m] = decompose<MODE>(a0[m], caddq(reduce32(acc[m])));
 #pragma unroll
             for (int k = 0; k < 4; ++k) w0t[k] = make_int4(a0[4 * k], a0[4 * k + 1], a0[4 * k + 2], a0[4 * k + 3]);
             {
@@ -364,6 +344,8 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512) ? 1 : 512 / THREADS)
         int32_t ch[16];
         challenge_strided(ch, masks, g.t);
         ntt16_ool(ch, g.sm, g.gmask, g.t);
+#pragma unroll
+        for (int m = 0; m < 16; ++m) ch[m] = scale_f(ch[m]);
         const int32_t *s1 = reinterpret_cast<const int32_t *>(row + C::SK_S1);
         const int32_t *s2 = reinterpret_cast<const int32_t *>(row + C::SK_S2);
         const int32_t *t0 = reinterpret_cast<const int32_t *>(row + C::SK_T0);

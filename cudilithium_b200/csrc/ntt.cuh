@@ -2,14 +2,15 @@
 // threads (16 coefficients each, two groups per warp).
 //
 // Arithmetic: the same Cooley-Tukey (forward) and Gentleman-Sande (inverse) butterfly network
-// as the reference (src/ntt.cu:58-207, include/ntt.cuh:74-306), and the inverse ends with a
-// Montgomery multiplication of every coefficient by f = 41978 (src/ntt.cu:201-205).  Two forms:
+// as the reference (src/ntt.cu:58-207, include/ntt.cuh:74-306), whose inverse ends with a Montgomery
+// multiplication of every coefficient by f = 41978 (src/ntt.cu:201-205).  Two forms:
 //   ntt16 / intt16   every butterfly is a +/- montmul(zeta, b) with the reference's Montgomery
 //                    zetas, so outputs are bit-identical to the reference's radix-8 kernels and to
 //                    the CPU oracle (key generation, the NTT microbench);
 //   ntt16s / intt16s the butterflies multiply by the true zetas with precomputed quotients
 //                    (shoup_mul): the same residues mod q in other representatives, for the
-//                    signing and verification paths, which reduce every output before use.
+//                    signing and verification paths, which reduce every output before use and
+//                    carry f in an operand of the products (scale_f).
 //
 // Layout (radix-16, one shared-memory transpose per transform instead of two):
 //   forward: in  x[i] = a[t + 16 i]  -> levels len 128..16 in registers
@@ -29,29 +30,36 @@
 namespace cudil {
 
 // Per-thread twiddles of the register-local half: 15 (zeta, zeta*qinv) pairs for each group
-// position t, padded to 16 pairs (128 bytes) so a thread reads them with 8 x 128-bit loads.
+// position t, padded to 16 pairs, read as eight 128-bit chunks of two pairs.  Chunk c of the 16
+// positions is contiguous (256 bytes), so one load instruction of a warp touches two cache lines; with
+// a position's row contiguous it touched sixteen.
 struct GroupTwiddles {
-    int2 fwd[16][16];  // levels len 8,4,2,1 of the forward transform
-    int2 inv[16][16];  // levels len 1,2,4,8 of the inverse transform (negated zetas)
+    int4 fwd[8][16];  // levels len 8,4,2,1 of the forward transform
+    int4 inv[8][16];  // levels len 1,2,4,8 of the inverse transform (negated zetas)
 };
 
 __host__ __device__ constexpr GroupTwiddles make_group_twiddles(const TwiddleTables &tw) {
     GroupTwiddles g{};
     for (int t = 0; t < 16; ++t) {
+        int32_t f[32] = {}, v[32] = {};  // (zeta, zeta*qinv) pairs of position t
         int n = 0;
         // forward: len 8: zeta[16+t]; len 4: zeta[32+2t+m]; len 2: zeta[64+4t+m]; len 1: zeta[128+8t+m]
-        g.fwd[t][n++] = int2{tw.zeta[16 + t], tw.zeta_q[16 + t]};
-        for (int m = 0; m < 2; ++m) g.fwd[t][n++] = int2{tw.zeta[32 + 2 * t + m], tw.zeta_q[32 + 2 * t + m]};
-        for (int m = 0; m < 4; ++m) g.fwd[t][n++] = int2{tw.zeta[64 + 4 * t + m], tw.zeta_q[64 + 4 * t + m]};
-        for (int m = 0; m < 8; ++m) g.fwd[t][n++] = int2{tw.zeta[128 + 8 * t + m], tw.zeta_q[128 + 8 * t + m]};
-        g.fwd[t][15] = int2{0, 0};
+        for (int h = 1; h <= 8; h *= 2)
+            for (int m = 0; m < h; ++m, ++n) {
+                f[2 * n] = tw.zeta[16 * h + h * t + m];
+                f[2 * n + 1] = tw.zeta_q[16 * h + h * t + m];
+            }
         n = 0;
         // inverse: len 1: -zeta[255-8t-m]; len 2: -zeta[127-4t-m]; len 4: -zeta[63-2t-m]; len 8: -zeta[31-t]
-        for (int m = 0; m < 8; ++m) g.inv[t][n++] = int2{tw.izeta[255 - 8 * t - m], tw.izeta_q[255 - 8 * t - m]};
-        for (int m = 0; m < 4; ++m) g.inv[t][n++] = int2{tw.izeta[127 - 4 * t - m], tw.izeta_q[127 - 4 * t - m]};
-        for (int m = 0; m < 2; ++m) g.inv[t][n++] = int2{tw.izeta[63 - 2 * t - m], tw.izeta_q[63 - 2 * t - m]};
-        g.inv[t][n++] = int2{tw.izeta[31 - t], tw.izeta_q[31 - t]};
-        g.inv[t][15] = int2{0, 0};
+        for (int h = 8; h >= 1; h /= 2)
+            for (int m = 0; m < h; ++m, ++n) {
+                v[2 * n] = tw.izeta[32 * h - 1 - h * t - m];
+                v[2 * n + 1] = tw.izeta_q[32 * h - 1 - h * t - m];
+            }
+        for (int c = 0; c < 8; ++c) {
+            g.fwd[c][t] = int4{f[4 * c], f[4 * c + 1], f[4 * c + 2], f[4 * c + 3]};
+            g.inv[c][t] = int4{v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]};
+        }
     }
     return g;
 }
@@ -99,18 +107,17 @@ __device__ __forceinline__ const TwiddleTables &utw() {
     return S ? c_tw_s : c_tw;
 }
 
-__device__ __forceinline__ void load_tw16(int2 (&tw)[16], const int2 *src) {
-    const int4 *p = reinterpret_cast<const int4 *>(src);
+__device__ __forceinline__ void load_tw16(int2 (&tw)[16], const int4 (&src)[8][16], int t) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        int4 v = __ldg(p + i);
+        const int4 v = __ldg(&src[i][t]);
         tw[2 * i] = make_int2(v.x, v.y);
         tw[2 * i + 1] = make_int2(v.z, v.w);
     }
 }
 
 // Forward NTT with the thread's register-local twiddles already loaded (tw = the group position's
-// row of GroupTwiddles::fwd); sm = this group's NTT_SMEM_WORDS-word region, gmask = its lanes.
+// pairs of GroupTwiddles::fwd); sm = this group's NTT_SMEM_WORDS-word region, gmask = its lanes.
 template <bool S>
 __device__ __forceinline__ void ntt16_tw(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t, const int2 (&tw)[16]) {
     // len 128: (i, i+8), zeta[1]
@@ -156,13 +163,15 @@ __device__ __forceinline__ void ntt16_tw(int32_t (&x)[16], int32_t *sm, unsigned
 template <bool S>
 __device__ __forceinline__ void ntt16_t(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) {
     int2 tw[16];
-    load_tw16(tw, (S ? g_group_tw_s : g_group_tw).fwd[t]);
+    load_tw16(tw, (S ? g_group_tw_s : g_group_tw).fwd, t);
     ntt16_tw<S>(x, sm, gmask, t, tw);
 }
 
 // Inverse NTT including the final multiplication by f (invntt_tomont), register-local twiddles
-// already loaded (tw = the group position's row of GroupTwiddles::inv).
-template <bool S>
+// already loaded (tw = the group position's pairs of GroupTwiddles::inv).  FIN = false leaves the
+// final multiplication out: for inputs that carry the factor already.  Then |x| <= q at the input
+// keeps every intermediate within 256 q < 2^31; the outputs are bounded by 256 max |x|.
+template <bool S, bool FIN = true>
 __device__ __forceinline__ void intt16_tw(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t, const int2 (&tw)[16]) {
     // len 1: block 8t + (i>>1): -zeta[255 - 8t - (i>>1)]
 #pragma unroll
@@ -200,15 +209,17 @@ __device__ __forceinline__ void intt16_tw(int32_t (&x)[16], int32_t *sm, unsigne
     // len 128: -zeta[1]
 #pragma unroll
     for (int i = 0; i < 8; ++i) gs_bfly<S>(x[i], x[i + 8], utw<S>().izeta[1], utw<S>().izeta_q[1]);
+    if constexpr (FIN) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) x[i] = montmul_pre(x[i], F_INV, F_INV_Q);
+        for (int i = 0; i < 16; ++i) x[i] = montmul_pre(x[i], F_INV, F_INV_Q);
+    }
 }
 
-template <bool S>
+template <bool S, bool FIN = true>
 __device__ __forceinline__ void intt16_t(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) {
     int2 tw[16];
-    load_tw16(tw, (S ? g_group_tw_s : g_group_tw).inv[t]);
-    intt16_tw<S>(x, sm, gmask, t, tw);
+    load_tw16(tw, (S ? g_group_tw_s : g_group_tw).inv, t);
+    intt16_tw<S, FIN>(x, sm, gmask, t, tw);
 }
 
 // Montgomery transforms: the reference's exact output representatives (key generation, the NTT
@@ -216,9 +227,15 @@ __device__ __forceinline__ void intt16_t(int32_t (&x)[16], int32_t *sm, unsigned
 __device__ __forceinline__ void ntt16(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { ntt16_t<false>(x, sm, gmask, t); }
 __device__ __forceinline__ void intt16(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { intt16_t<false>(x, sm, gmask, t); }
 // Precomputed-quotient transforms: the same residues, cheaper butterflies (signing, verification,
-// the engine's key caches -- every consumer reduces the outputs before use).
+// the engine's key caches -- every consumer reduces the outputs before use).  The inverse has no final
+// multiplication: its callers' products carry the factor f (scale_f below).
 __device__ __forceinline__ void ntt16s(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { ntt16_t<true>(x, sm, gmask, t); }
-__device__ __forceinline__ void intt16s(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { intt16_t<true>(x, sm, gmask, t); }
+__device__ __forceinline__ void intt16s(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { intt16_t<true, false>(x, sm, gmask, t); }
+
+// The inverse transform's factor f, put into one operand of the products it will transform -- A_hat
+// when it is sampled, c_hat once per challenge -- instead of into all 256 outputs of every inverse
+// transform (16 multiplications of a thread's ~90 per transform).
+__device__ __forceinline__ int32_t scale_f(int32_t a) { return montmul_pre(a, F_INV, F_INV_Q); }
 
 // Out-of-line forms of the two transforms for large kernels that call them from many places: one
 // copy of each transform instead of one per call site keeps the instruction working set small.
@@ -291,6 +308,47 @@ __device__ __forceinline__ void load16_smem(int32_t (&x)[16], const int32_t *pol
         x[4 * i + 1] = v.y;
         x[4 * i + 2] = v.z;
         x[4 * i + 3] = v.w;
+    }
+}
+
+// out[i] = sum_j op(j)[16 t + i] * y_j[16 t + i] mod q (Montgomery-reduced once) over NOPS operand
+// polynomials op(j) in global memory and vectors y_j in shared memory (store16_smem layout, y_j =
+// yh + j N).  The products accumulate in 64 bits: |sum| < NOPS * q * 2^27 < 2^53, so |out| < 0.67 q.
+// Eight coefficients at a time, CH operands' loads in flight before the first is consumed.
+template <int NOPS, int CH, typename Op>
+__device__ __forceinline__ void dot16(int32_t (&out)[16], const int32_t *yh, int t, Op op) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        int64_t acc[8];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) acc[m] = 0;
+#pragma unroll
+        for (int j0 = 0; j0 < NOPS; j0 += CH) {
+            int4 a[CH][2];
+#pragma unroll
+            for (int j = 0; j < CH; ++j)
+                if (j0 + j < NOPS) {
+                    const int4 *p = reinterpret_cast<const int4 *>(op(j0 + j) + 16 * t) + 2 * h;
+                    a[j][0] = p[0];
+                    a[j][1] = p[1];
+                }
+#pragma unroll
+            for (int j = 0; j < CH; ++j)
+                if (j0 + j < NOPS) {
+                    const int4 *q = reinterpret_cast<const int4 *>(yh + (j0 + j) * N + 16 * t);
+                    const int4 y0 = q[(2 * h + t) & 3], y1 = q[(2 * h + 1 + t) & 3];
+                    acc[0] += (int64_t)a[j][0].x * y0.x;
+                    acc[1] += (int64_t)a[j][0].y * y0.y;
+                    acc[2] += (int64_t)a[j][0].z * y0.z;
+                    acc[3] += (int64_t)a[j][0].w * y0.w;
+                    acc[4] += (int64_t)a[j][1].x * y1.x;
+                    acc[5] += (int64_t)a[j][1].y * y1.y;
+                    acc[6] += (int64_t)a[j][1].z * y1.z;
+                    acc[7] += (int64_t)a[j][1].w * y1.w;
+                }
+        }
+#pragma unroll
+        for (int m = 0; m < 8; ++m) out[8 * h + m] = montred(acc[m]);
     }
 }
 

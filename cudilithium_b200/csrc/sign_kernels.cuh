@@ -179,18 +179,7 @@ __global__ void __launch_bounds__(kBlock) k_sign_compute_w(const uint8_t *sign_p
         if (!bc_ok(item < (uint32_t)nitems, BC_STAGE_ITEM)) continue;
         const int32_t *mat = reinterpret_cast<const int32_t *>(sign_pool + (size_t)item * sp + LY::sg_mat(mlen)) + (size_t)i * L * N;
         int32_t acc[16];
-#pragma unroll
-        for (int m = 0; m < 16; ++m) acc[m] = 0;
-#pragma unroll
-        for (int j = 0; j < L; ++j) {
-            int32_t av[16], yv[16];
-            load16_contig(av, mat + (size_t)j * N + 16 * g.t);
-            load16_smem(yv, &s_yhat[a][j][0], g.t);
-#pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] += montmul(av[m], yv[m]);
-        }
-#pragma unroll
-        for (int m = 0; m < 16; ++m) acc[m] = reduce32(acc[m]);
+        dot16<L, (L + 1) / 2>(acc, &s_yhat[a][0][0], g.t, [&](int j) { return mat + (size_t)j * N; });
         intt16s(acc, g.sm, g.gmask, g.t);
         uint8_t *trow = temp_pool + (size_t)e * tp;
         int32_t *w0 = reinterpret_cast<int32_t *>(trow + LY::TP_W0) + (size_t)i * N;
@@ -198,7 +187,7 @@ __global__ void __launch_bounds__(kBlock) k_sign_compute_w(const uint8_t *sign_p
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
             int32_t a0;
-            w1[m] = decompose<MODE>(a0, caddq(acc[m]));
+            w1[m] = decompose<MODE>(a0, caddq(reduce32(acc[m])));
             w0[g.t + 16 * m] = a0;
         }
         int32_t w1c[16];
@@ -337,6 +326,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_sign_reject(const uint8_t *sign_p
     int32_t ch[16];
     challenge_strided(ch, masks, g.t);
     ntt16s(ch, g.sm, g.gmask, g.t);
+#pragma unroll
+    for (int m = 0; m < 16; ++m) ch[m] = scale_f(ch[m]);
 
     // Acceptance needs every check to pass (src/sign.cu:1026-1144 checks z, then r0, then ct0);
     // here the most selective runs first: pair steps of the r0_i (r0 replaces w0 in the temp row,

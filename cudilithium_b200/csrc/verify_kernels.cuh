@@ -127,6 +127,10 @@ __global__ void __launch_bounds__(kBlock) k_verify_w(uint8_t *pool, size_t pitch
             challenge_strided(x, masks, g.t);
         }
         ntt16s(x, g.sm, g.gmask, g.t);
+        if (j == L) {  // -c_hat with the inverse transform's factor (A_hat carries it already)
+#pragma unroll
+            for (int m = 0; m < 16; ++m) x[m] = -scale_f(x[m]);
+        }
         store16_smem(&s_hat[a][j][0], x, g.t);
     }
     __syncthreads();
@@ -137,33 +141,28 @@ __global__ void __launch_bounds__(kBlock) k_verify_w(uint8_t *pool, size_t pitch
         uint8_t *row = pool + (size_t)it * pitch;
         // t1_i * 2^d, NTT
         int32_t t1[16];
-        const uint8_t *t1p = row + LY::VF_PK + SEEDBYTES + (size_t)i * POLYT1_PACKED;
+        {
+            uint32_t v[16];
+            unpack_strided<10>(v, row + LY::VF_PK + SEEDBYTES + (size_t)i * POLYT1_PACKED, g.t);
 #pragma unroll
-        for (int m = 0; m < 16; ++m) t1[m] = (int32_t)(get_bits(t1p, (g.t + 16 * m) * 10, 10) << D);
+            for (int m = 0; m < 16; ++m) t1[m] = (int32_t)(v[m] << D);
+        }
         ntt16s(t1, g.sm, g.gmask, g.t);
         const int32_t *mat = reinterpret_cast<const int32_t *>(row + LY::vf_mat(mlen)) + (size_t)i * L * N;
         int32_t acc[16];
-#pragma unroll
-        for (int m = 0; m < 16; ++m) acc[m] = 0;
-#pragma unroll
-        for (int j = 0; j < L; ++j) {
-            int32_t av[16], zv[16];
-            load16_contig(av, mat + (size_t)j * N + 16 * g.t);
-            load16_smem(zv, &s_hat[a][j][0], g.t);
-#pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] += montmul(av[m], zv[m]);
-        }
+        dot16<L, (L + 1) / 2>(acc, &s_hat[a][0][0], g.t, [&](int j) { return mat + (size_t)j * N; });
         int32_t cv[16];
         load16_smem(cv, &s_hat[a][L][0], g.t);
+        // + (-c) t1: |sum| < 1.2 q, reduced below q for the inverse transform
 #pragma unroll
-        for (int m = 0; m < 16; ++m) acc[m] = reduce32(acc[m] - montmul(cv[m], t1[m]));
+        for (int m = 0; m < 16; ++m) acc[m] = reduce32(acc[m] + montmul(cv[m], t1[m]));
         intt16s(acc, g.sm, g.gmask, g.t);
         int32_t w1[16];
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
             const int c = g.t + 16 * m;
             const unsigned hb = (s_hint[a][i][c >> 5] >> (c & 31)) & 1u;
-            w1[m] = use_hint<MODE>(caddq(acc[m]), hb);
+            w1[m] = use_hint<MODE>(caddq(reduce32(acc[m])), hb);
         }
         int32_t w1c[16];
         strided_to_contig(g, w1, w1c);
