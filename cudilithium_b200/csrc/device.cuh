@@ -22,10 +22,12 @@ __device__ __forceinline__ void ld_lanes(uint2 (&v)[NL], const uint8_t *p) {
 
 // ExpandA entry A[i][j] (NTT domain): SHAKE128(rho || j || i), 23-bit little-endian candidates
 // accepted below q (src/sign.cu:98-163, src/keypair.cu:139-190; the stream is extended until 256
-// coefficients are accepted, as benches/bench_rej_sampling.cu:571-593 does).  `emit(ctr, v)` is
-// called for every accepted coefficient in order.
-template <typename Emit>
-__device__ __forceinline__ void expand_a_stream(const uint2 (&rho)[4], int i, int j, Emit emit) {
+// coefficients are accepted, as benches/bench_rej_sampling.cu:571-593 does).  Eight candidates that are
+// all accepted while the count is a multiple of four go out together, emit8(ctr, v); anything else
+// coefficient by coefficient, emit1(ctr, v) (a candidate is rejected with probability
+// (2^23 - q) / 2^23 < 0.1%, so nearly every group takes the wide path).
+template <typename Emit8, typename Emit1>
+__device__ __forceinline__ void expand_a_groups(const uint2 (&rho)[4], int i, int j, Emit8 emit8, Emit1 emit1) {
     uint32_t al[25], ah[25];
     shake_absorb_seed_nonce<SHAKE128_RATE, 4>(al, ah, rho, (uint32_t)((i << 8) | j));
     int ctr = 0;
@@ -46,62 +48,20 @@ __device__ __forceinline__ void expand_a_stream(const uint2 (&rho)[4], int i, in
             c[5] = __funnelshift_r(w3, w4, 24);
             c[6] = __funnelshift_r(w4, w5, 16);
             c[7] = w5 >> 8;
-#pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                const uint32_t v = c[m] & 0x7FFFFFu;
-                if (v < (uint32_t)Q && ctr < N) {
-                    emit(ctr, (int32_t)v);
-                    ++ctr;
-                }
-            }
-        }
-    }
-}
-
-// The same entry, times the inverse transform's factor f (scale_f), written to out[0..255].  Where out is 16-byte aligned, a group of eight
-// candidates that are all accepted while the count is a multiple of four goes out as two 16-byte
-// stores; anything else is stored coefficient by coefficient (a candidate is rejected with
-// probability (2^23 - q) / 2^23 < 0.1%, so nearly every group takes the wide path).
-__device__ __forceinline__ void expand_a_row(const uint2 (&rho)[4], int i, int j, int32_t *out) {
-    uint32_t al[25], ah[25];
-    shake_absorb_seed_nonce<SHAKE128_RATE, 4>(al, ah, rho, (uint32_t)((i << 8) | j));
-    const bool wide = (reinterpret_cast<uintptr_t>(out) & 15u) == 0u;
-    int ctr = 0;
-#pragma unroll 1
-    while (ctr < N) {
-        keccak_f1600(al, ah);
-#pragma unroll
-        for (int g = 0; g < 7; ++g) {
-            const uint32_t w0 = al[3 * g], w1 = ah[3 * g], w2 = al[3 * g + 1];
-            const uint32_t w3 = ah[3 * g + 1], w4 = al[3 * g + 2], w5 = ah[3 * g + 2];
-            uint32_t c[8];
-            c[0] = w0;
-            c[1] = __funnelshift_r(w0, w1, 24);
-            c[2] = __funnelshift_r(w1, w2, 16);
-            c[3] = w2 >> 8;
-            c[4] = w3;
-            c[5] = __funnelshift_r(w3, w4, 24);
-            c[6] = __funnelshift_r(w4, w5, 16);
-            c[7] = w5 >> 8;
             bool all = true;
 #pragma unroll
             for (int m = 0; m < 8; ++m) {
                 c[m] &= 0x7FFFFFu;
                 all &= c[m] < (uint32_t)Q;
             }
-            if (wide && all && (ctr & 3) == 0 && ctr + 8 <= N) {
-                int4 *o = reinterpret_cast<int4 *>(out + ctr);
-                int32_t v[8];
-#pragma unroll
-                for (int m = 0; m < 8; ++m) v[m] = scale_f((int32_t)c[m]);
-                o[0] = make_int4(v[0], v[1], v[2], v[3]);
-                o[1] = make_int4(v[4], v[5], v[6], v[7]);
+            if (all && (ctr & 3) == 0 && ctr + 8 <= N) {
+                emit8(ctr, c);
                 ctr += 8;
             } else {
 #pragma unroll
                 for (int m = 0; m < 8; ++m) {
                     if (c[m] < (uint32_t)Q && ctr < N) {
-                        out[ctr] = scale_f((int32_t)c[m]);
+                        emit1(ctr, c[m]);
                         ++ctr;
                     }
                 }
@@ -110,40 +70,17 @@ __device__ __forceinline__ void expand_a_row(const uint2 (&rho)[4], int i, int j
     }
 }
 
-// ExpandS entry: SHAKE256(rho' || nonce), nibbles < 15 (eta 2) or < 9 (eta 4), low nibble first
-// (src/keypair.cu:84-114).  emit(ctr, s) with s in [-eta, eta].
-template <int MODE, typename Emit>
-__device__ __forceinline__ void expand_s_stream(const uint2 (&rhoprime)[8], int nonce, Emit emit) {
-    constexpr int ETA = Params<MODE>::ETA;
-    uint32_t al[25], ah[25];
-    shake_absorb_seed_nonce<SHAKE256_RATE, 8>(al, ah, rhoprime, (uint32_t)nonce);
-    int ctr = 0;
-#pragma unroll 1
-    while (ctr < N) {
-        keccak_f1600(al, ah);
-#pragma unroll
-        for (int w = 0; w < 17; ++w) {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const uint32_t word = half ? ah[w] : al[w];
-#pragma unroll
-                for (int nb = 0; nb < 8; ++nb) {
-                    const uint32_t t = (word >> (4 * nb)) & 15u;
-                    if constexpr (ETA == 2) {
-                        if (t < 15 && ctr < N) {
-                            emit(ctr, 2 - (int32_t)(t - (205 * t >> 10) * 5));
-                            ++ctr;
-                        }
-                    } else {
-                        if (t < 9 && ctr < N) {
-                            emit(ctr, 4 - (int32_t)t);
-                            ++ctr;
-                        }
-                    }
-                }
-            }
-        }
-    }
+// The same entry, times the inverse transform's factor f (scale_f), written to out[0..255], a group of
+// eight as two 16-byte stores.  Rows start 16-byte aligned (pool rows and key-cache rows are).
+__device__ __forceinline__ void expand_a_row(const uint2 (&rho)[4], int i, int j, int32_t *out) {
+    expand_a_groups(
+        rho, i, j,
+        [&](int c, const uint32_t (&v)[8]) {
+            int4 *o = reinterpret_cast<int4 *>(out + c);
+            o[0] = make_int4(scale_f((int32_t)v[0]), scale_f((int32_t)v[1]), scale_f((int32_t)v[2]), scale_f((int32_t)v[3]));
+            o[1] = make_int4(scale_f((int32_t)v[4]), scale_f((int32_t)v[5]), scale_f((int32_t)v[6]), scale_f((int32_t)v[7]));
+        },
+        [&](int c, uint32_t v) { out[c] = scale_f((int32_t)v); });
 }
 
 // ExpandMask entry y_j: SHAKE256(rho' || kappa) with kappa = L*nonce + j (src/sign.cu:488-499);

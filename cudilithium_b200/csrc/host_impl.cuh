@@ -49,9 +49,8 @@ struct Impl {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
     static constexpr int K = PM::K, L = PM::L;
-    // keys per keypair block, attempts per compute_w block, signatures per verify_w block:
-    // chosen so that the 8 groups of a block have whole units of work in every phase.
-    static constexpr int KPI = MODE == 2 ? 8 : (MODE == 3 ? 4 : 2);
+    // attempts per compute_w block, signatures per verify_w block: chosen so that the 8 groups of a
+    // block have whole units of work in every phase.
     static constexpr int AW = MODE == 2 ? 2 : (MODE == 3 ? 4 : 1);
     static constexpr int AV = MODE == 2 ? 2 : (MODE == 3 ? 4 : 1);
 
@@ -62,13 +61,14 @@ struct Impl {
         if (!pk || !sk || !pool || pitch < LY::ref_keypair_row() || misaligned(pool, pitch) || n > (size_t)INT_MAX / 64)
             return CUDIL_ERR_INVALID;
         const int nn = (int)n;
-        CUDIL_CK(cudaMemset2DAsync(pool + LY::KP_TACC, pitch, 0, (size_t)K * LY::POLY, n, st));
         if (seeds) CUDIL_CK(cudaMemcpy2DAsync(pool + LY::KP_SK + PM::SK_TR, pitch, seeds, SEEDBYTES, SEEDBYTES, n, in_kind, st));
         CUDIL_LAUNCH(KID_KP_SEED, st, k_kp_seed<MODE><<<blocks_for(n, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, nn, (unsigned long long)rand_index, seeds ? 1 : 0));
         CUDIL_CK_LAUNCH();
-        const size_t smem = KpSmem<MODE>::bytes(KPI);
-        CUDIL_CK(cudaFuncSetAttribute(k_kp_main<MODE, KPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CUDIL_LAUNCH(KID_KP_MAIN, st, k_kp_main<MODE, KPI><<<(unsigned)((n + KPI - 1) / KPI), kBlock, smem, st>>>(pool, pitch, nn));
+        CUDIL_LAUNCH(KID_KP_S, st, k_kp_s<MODE><<<blocks_for(n * (K + L)), kBlock, 0, st>>>(pool, pitch, nn));
+        CUDIL_CK_LAUNCH();
+        CUDIL_LAUNCH(KID_KP_S1, st, k_kp_s1<MODE><<<blocks_for(n * L * 16), kBlock, 0, st>>>(pool, pitch, nn));
+        CUDIL_CK_LAUNCH();
+        CUDIL_LAUNCH(KID_KP_T, st, k_kp_t<MODE><<<blocks_for(n * K, kBlock / L), kBlock, 0, st>>>(pool, pitch, nn));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_KP_TR, st, k_kp_tr<MODE><<<blocks_for(n, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, nn));
         CUDIL_CK_LAUNCH();

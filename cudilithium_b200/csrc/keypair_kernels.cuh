@@ -1,9 +1,12 @@
-// Batched key generation (reference: gpu_keypair, src/keypair.cu:35-311, one warp per key).
+// Batched key generation (reference: gpu_keypair, src/keypair.cu:35-311, one warp per key), one kernel
+// per parallel shape so that every Keccak stage has all its threads on streams:
 //   k_kp_seed  one thread per key: seed (from the counter scheme of src/keypair.cu:53-59 or
 //              caller-provided) -> (rho, rho', K) = SHAKE256(seed, 128)
-//   k_kp_main  KPI keys per block: ExpandS streams (one thread each), eta packing and NTT(s1)
-//              (16-thread groups), ExpandA streams accumulating A_ij * s1_hat_j straight into
-//              t_hat (no A matrix is stored), then invNTT, + s2, Power2Round, t1/t0 packing
+//   k_kp_s     one thread per secret polynomial: ExpandS stream, eta fields packed into sk as sampled
+//   k_kp_s1    16-thread group per s1 polynomial: s1_hat = NTT(s1), with the inverse transform's factor
+//   k_kp_t     one thread per ExpandA entry, products A_ij * s1_hat_j summed into the block's rows of
+//              t_hat in shared memory (no A matrix is stored), then per row invNTT, + s2, Power2Round,
+//              t1/t0 packing
 //   k_kp_tr    one thread per key: tr = SHAKE256(pk, 32)
 #pragma once
 
@@ -75,92 +78,157 @@ __device__ __forceinline__ void pack16_halves(uint16_t *out, const uint32_t (&v)
     for (int i = 0; i < BITS; ++i) out[i] = (uint16_t)w[i];
 }
 
+// ExpandS (src/keypair.cu:84-114): s1 (nonces 0..L-1) then s2 (nonces L..L+K-1), one thread per
+// polynomial, SHAKE256(rho' || nonce); nibbles, low one first, below 15 (eta 2) or 9 (eta 4) are
+// accepted.  The fields go straight into sk: a table of the 256 byte values gives a byte's accepted
+// fields, already packed, and their bits, so two nibbles cost one lookup and one append.
 template <int MODE>
-struct KpSmem {
-    static constexpr int K = Params<MODE>::K, L = Params<MODE>::L;
-    static constexpr size_t bytes(int kpi) {
-        return (size_t)kpi * (K + L) * N                      // s (int8)
-               + (size_t)kpi * L * N * sizeof(int32_t)         // s1_hat
-               + (size_t)kGroupsPerBlock * NTT_SMEM_WORDS * 4;  // NTT transposes
-    }
-};
-
-template <int MODE, int KPI>
-__global__ void __launch_bounds__(kBlock) k_kp_main(uint8_t *pool, size_t pitch, int n) {
+__global__ void __launch_bounds__(kBlock) k_kp_s(uint8_t *pool, size_t pitch, int n) {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
-    constexpr int K = PM::K, L = PM::L;
-    extern __shared__ __align__(16) uint8_t kp_smem[];
-    int32_t *s1hat = reinterpret_cast<int32_t *>(kp_smem);                         // [KPI][L][N]
-    int32_t *sm = s1hat + (size_t)KPI * L * N;                                       // NTT scratch
-    int8_t *s = reinterpret_cast<int8_t *>(sm + kGroupsPerBlock * NTT_SMEM_WORDS);  // [KPI][L+K][N]
-    const int it0 = blockIdx.x * KPI;
-    const int gi = threadIdx.x >> 4;
-    Group g = make_group(sm, gi);
-
-    // ExpandS: s1 (nonces 0..L-1) and s2 (nonces L..L+K-1)
-    for (int u = threadIdx.x; u < KPI * (L + K); u += blockDim.x) {
-        const int a = u / (L + K), p = u % (L + K), it = it0 + a;
-        if (it >= n) continue;
-        uint2 rhop[8];
-        ld_lanes(rhop, pool + (size_t)it * pitch + LY::KP_RHOP);
-        int8_t *sp = s + ((size_t)a * (L + K) + p) * N;
-        expand_s_stream<MODE>(rhop, p, [&](int c, int32_t v) { sp[c] = (int8_t)v; });
+    constexpr int NP = PM::L + PM::K, EB = PM::ETA_BITS, NW = N * EB / 32;
+    __shared__ uint32_t lut[256];  // fields | bits << 8
+    for (int v = threadIdx.x; v < 256; v += kBlock) {
+        uint32_t f = 0, nb = 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t t = (uint32_t)(v >> (4 * h)) & 15u;
+            if (PM::ETA == 2 ? t < 15u : t < 9u) {
+                f |= (PM::ETA == 2 ? t % 5u : t) << nb;
+                nb += EB;
+            }
+        }
+        lut[v] = f | nb << 8;
     }
     __syncthreads();
+    const int u = blockIdx.x * blockDim.x + threadIdx.x, it = u / NP, p = u % NP;
+    if (it >= n) return;
+    uint8_t *row = pool + (size_t)it * pitch;
+    uint2 rhop[8];
+    ld_lanes(rhop, row + LY::KP_RHOP);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(row + LY::KP_SK + PM::SK_S1 + (size_t)p * PM::POLYETA_PACKED);
+    uint32_t al[25], ah[25];
+    shake_absorb_seed_nonce<SHAKE256_RATE, 8>(al, ah, rhop, (uint32_t)p);
+    uint32_t w = 0, nb = 0;
+    int words = 0;
+    while (words < NW) {
+        keccak_f1600(al, ah);
+#pragma unroll
+        for (int k = 0; k < 2 * (SHAKE256_RATE / 8); ++k) {
+            const uint32_t word = (k & 1) ? ah[k >> 1] : al[k >> 1];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const uint32_t e = lut[(word >> (8 * b)) & 0xFFu], f = e & 0xFFu;
+                w |= f << nb;
+                const uint32_t nn = nb + (e >> 8);
+                if (nn >= 32u) {
+                    // the field bits past the word; fields past the last word are dropped
+                    if (words < NW) dst[words] = w;
+                    ++words;
+                    w = f >> (32u - nb);
+                }
+                nb = nn & 31u;
+            }
+        }
+    }
+}
 
-    // eta packing of s1, s2 into sk; NTT(s1)
-    for (int u = gi; u < KPI * (L + K); u += kGroupsPerBlock) {
-        const int a = u / (L + K), p = u % (L + K), it = it0 + a;
-        if (it >= n) continue;
-        uint8_t *row = pool + (size_t)it * pitch;
-        const int8_t *sp = s + ((size_t)a * (L + K) + p) * N;
-        uint32_t v[16];
+// The eta field of coefficient c of a packed secret polynomial.
+template <int MODE>
+__device__ __forceinline__ int32_t eta_coef(const uint8_t *poly, int c) {
+    constexpr int EB = P<MODE>::ETA_BITS;
+    const int bit = EB * c, byte = bit >> 3, sh = bit & 7;
+    uint32_t v = poly[byte];
+    if (sh + EB > 8) v |= (uint32_t)poly[byte + 1] << 8;
+    return Params<MODE>::ETA - (int32_t)((v >> sh) & ((1u << EB) - 1u));
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kBlock) k_kp_s1(uint8_t *pool, size_t pitch, int n) {
+    using PM = P<MODE>;
+    using LY = Layout<MODE>;
+    __shared__ int32_t sm[kGroupsPerBlock * NTT_SMEM_WORDS];
+    const int gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, it = gid / PM::L, j = gid % PM::L;
+    if (it >= n) return;
+    Group g = make_group(sm, threadIdx.x >> 4);
+    uint8_t *row = pool + (size_t)it * pitch;
+    const uint8_t *src = row + LY::KP_SK + PM::SK_S1 + (size_t)j * PM::POLYETA_PACKED;
+    int32_t x[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) v[m] = (uint32_t)(PM::ETA - sp[16 * g.t + m]);
-        uint8_t *dst = row + LY::KP_SK + PM::SK_S1 + (size_t)p * PM::POLYETA_PACKED;
-        if constexpr (PM::ETA_BITS == 3)
-            pack16_halves<3>(reinterpret_cast<uint16_t *>(dst + 6 * g.t), v);
-        else
-            pack16_words<4>(reinterpret_cast<uint32_t *>(dst + 8 * g.t), v);
-        if (p < L) {
-            int32_t x[16];
+    for (int m = 0; m < 16; ++m) x[m] = eta_coef<MODE>(src, g.t + 16 * m);
+    ntt16s(x, g.sm, g.gmask, g.t);
 #pragma unroll
-            for (int m = 0; m < 16; ++m) x[m] = sp[g.t + 16 * m];
-            ntt16(x, g.sm, g.gmask, g.t);
-            store16_contig(s1hat + ((size_t)a * L + p) * N + 16 * g.t, x);
+    for (int m = 0; m < 16; ++m) x[m] = scale_f(x[m]);
+    store16_contig(reinterpret_cast<int32_t *>(row + LY::KP_S1H) + (size_t)j * N + 16 * g.t, x);
+}
+
+// A block takes kBlock / L consecutive rows (key, i) of t_hat, one thread per entry A_ij of them, and
+// sums the products in shared memory.  Coefficient c of a row sits at c + c / 16 and rows are 273 words
+// apart: the lanes of a warp -- the same j of different rows -- then add to the same coefficient in
+// different banks, and a group's reads of its contiguous slices do not collide either.
+//
+// Bound: the ALU pipe (K L 5 permutations a key).  10 000 Dilithium2 key pairs, this stage: sums by
+// shared-memory atomics with a row's L entries in neighbouring lanes (L-way collisions) 316 us; entries
+// kept in shared memory and summed by the groups (128 KiB per 128 threads, too few warps) 372 us; this
+// layout 322 us (ALU pipe 76% busy while active).  Whole call: global atomics 658 us, now 537 us.
+constexpr int KP_ROW = 273;
+
+template <int MODE>
+__global__ void __launch_bounds__(kBlock) k_kp_t(uint8_t *pool, size_t pitch, int n) {
+    using PM = P<MODE>;
+    using LY = Layout<MODE>;
+    constexpr int K = PM::K, L = PM::L, ROWS = kBlock / L;
+    __shared__ int32_t acc[ROWS * KP_ROW];
+    __shared__ int32_t sm[kGroupsPerBlock * NTT_SMEM_WORDS];
+    const long long row0 = (long long)blockIdx.x * ROWS, nrows = (long long)n * K;
+    for (int q = threadIdx.x; q < ROWS * KP_ROW; q += kBlock) acc[q] = 0;
+    __syncthreads();
+    {
+        const int j = threadIdx.x / ROWS, r = threadIdx.x % ROWS;
+        const long long gr = row0 + r;
+        if (j < L && gr < nrows) {
+            const int it = (int)(gr / K), i = (int)(gr % K);
+            const uint8_t *row = pool + (size_t)it * pitch;
+            uint2 rho[4];
+            ld_lanes(rho, row + LY::KP_PK);
+            const int32_t *sh = reinterpret_cast<const int32_t *>(row + LY::KP_S1H) + (size_t)j * N;
+            int32_t *ac = acc + r * KP_ROW;
+            expand_a_groups(
+                rho, i, j,
+                [&](int c, const uint32_t (&v)[8]) {
+                    const int4 s0 = *reinterpret_cast<const int4 *>(sh + c), s1 = *reinterpret_cast<const int4 *>(sh + c + 4);
+                    int32_t *a0 = ac + c + (c >> 4), *a1 = ac + c + 4 + ((c + 4) >> 4);
+                    atomicAdd(a0, montmul((int32_t)v[0], s0.x));
+                    atomicAdd(a0 + 1, montmul((int32_t)v[1], s0.y));
+                    atomicAdd(a0 + 2, montmul((int32_t)v[2], s0.z));
+                    atomicAdd(a0 + 3, montmul((int32_t)v[3], s0.w));
+                    atomicAdd(a1, montmul((int32_t)v[4], s1.x));
+                    atomicAdd(a1 + 1, montmul((int32_t)v[5], s1.y));
+                    atomicAdd(a1 + 2, montmul((int32_t)v[6], s1.z));
+                    atomicAdd(a1 + 3, montmul((int32_t)v[7], s1.w));
+                },
+                [&](int c, uint32_t v) { atomicAdd(ac + c + (c >> 4), montmul((int32_t)v, sh[c])); });
         }
     }
     __syncthreads();
 
-    // ExpandA fused with the matrix-vector product: t_hat_i += A_ij o s1_hat_j
-    for (int u = threadIdx.x; u < KPI * K * L; u += blockDim.x) {
-        const int a = u / (K * L), ij = u % (K * L), i = ij / L, j = ij % L, it = it0 + a;
-        if (it >= n) continue;
-        uint8_t *row = pool + (size_t)it * pitch;
-        uint2 rho[4];
-        ld_lanes(rho, row + LY::KP_PK);
-        int32_t *acc = reinterpret_cast<int32_t *>(row + LY::KP_TACC) + (size_t)i * N;
-        const int32_t *sh = s1hat + ((size_t)a * L + j) * N;
-        expand_a_stream(rho, i, j, [&](int c, int32_t v) { atomicAdd(&acc[c], montmul(v, sh[c])); });
-    }
-    __syncthreads();
-
     // t = invNTT(t_hat) + s2; Power2Round; pack t1 (pk) and t0 (sk)
-    for (int u = gi; u < KPI * K; u += kGroupsPerBlock) {
-        const int a = u / K, i = u % K, it = it0 + a;
-        if (it >= n) continue;
+    const int gi = threadIdx.x >> 4;
+    Group g = make_group(sm, gi);
+    for (int r = gi; r < ROWS; r += kGroupsPerBlock) {
+        const long long gr = row0 + r;
+        if (gr >= nrows) break;
+        const int it = (int)(gr / K), i = (int)(gr % K);
         uint8_t *row = pool + (size_t)it * pitch;
-        const int32_t *acc = reinterpret_cast<const int32_t *>(row + LY::KP_TACC) + (size_t)i * N + 16 * g.t;
         int32_t x[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) x[m] = reduce32(__ldcg(acc + m));
-        intt16(x, g.sm, g.gmask, g.t);
-        const int8_t *s2 = s + ((size_t)a * (L + K) + L + i) * N;
+        for (int m = 0; m < 16; ++m) x[m] = reduce32(acc[r * KP_ROW + 17 * g.t + m]);
+        intt16s(x, g.sm, g.gmask, g.t);
+        const uint8_t *s2 = row + LY::KP_SK + PM::SK_S2 + (size_t)i * PM::POLYETA_PACKED;
         int32_t t1[16], t0[16];
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
-            const int32_t v = caddq(x[m] + s2[g.t + 16 * m]);
+            const int32_t v = caddq(reduce32(x[m] + eta_coef<MODE>(s2, g.t + 16 * m)));
             t1[m] = power2round(t0[m], v);
         }
         int32_t c1[16], c0[16];

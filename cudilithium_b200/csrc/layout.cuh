@@ -34,11 +34,11 @@ struct Layout {
                sizeof(int);
     }
 
-    // ---- keypair row: pk | sk | t_hat accumulators (K polys, zeroed before use) ----
+    // ---- keypair row: pk | sk | s1_hat (L <= K polys) ----
     static constexpr size_t KP_PK = 0;
     static constexpr size_t KP_SK = align256(PM::PK_BYTES);
-    static constexpr size_t KP_TACC = KP_SK + align256(PM::SK_BYTES);
-    static constexpr size_t KP_END = KP_TACC + K * POLY;
+    static constexpr size_t KP_S1H = KP_SK + align256(PM::SK_BYTES);
+    static constexpr size_t KP_END = KP_S1H + L * POLY;
     // rho' is parked in pk's t1 area until t1 is packed.
     static constexpr size_t KP_RHOP = KP_PK + SEEDBYTES;
 

@@ -14,7 +14,9 @@ namespace cudil {
 
 enum KernelId : int {
     KID_KP_SEED = 0,
-    KID_KP_MAIN,
+    KID_KP_S,
+    KID_KP_S1,
+    KID_KP_T,
     KID_KP_TR,
     KID_SIGN_PREHASH,
     KID_EXPAND_A,
@@ -42,7 +44,7 @@ enum KernelId : int {
 
 inline const char *kernel_name(int id) {
     static const char *names[KID_COUNT] = {
-        "k_kp_seed", "k_kp_main", "k_kp_tr", "k_sign_prehash", "k_expand_a", "k_sign_unpack_ntt",
+        "k_kp_seed", "k_kp_s", "k_kp_s1", "k_kp_t", "k_kp_tr", "k_sign_prehash", "k_expand_a", "k_sign_unpack_ntt",
         "k_sign_expand_mask", "k_sign_compute_w", "k_sign_challenge", "k_sign_reject", "k_sig_copy",
         "k_verify_prepare", "k_verify_w", "k_verify_final", "k_ntt_mul", "k_alu_peak",
         "k_fused_sign (graph)", "k_fused_verify (graph)", "k_fused_sched", "k_cache_sk", "k_cache_pk",
