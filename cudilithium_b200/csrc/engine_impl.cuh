@@ -1,12 +1,14 @@
-// Host side of the fused engine: device buffers sized once at creation, per-key caches, and the
-// graph that runs a whole signing (or verification) batch on the device with one launch:
-//   [k_fused_init] -> [k_fused_prehash] -> [k_fused_sign]       (sign)
-//   [k_fused_init] -> [k_fused_verify_prehash] -> [k_fused_verify] (verify)
-// The batch size travels in device memory (FusedQueue::n), so one instantiated graph serves every
-// batch size up to the engine's capacity; only the per-item metadata upload precedes the launch.
+// Host side of the fused engine: device buffers sized once at creation, per-key caches, and the kernels
+// of a whole signing or verification batch, enqueued without waiting for any of them:
+//   sign    rounds of the staged signer (fused_sign_staged.cuh) after k_fused_prehash, then k_fused_sign
+//           for what they left; or k_fused_init, k_fused_prehash and one persistent signer
+//   verify  k_fused_verify_prehash, k_fused_verify
+// The batch's metadata -- queue block, message offsets and lengths, key indices, longest-first order -- go
+// up in one copy.  Buffers are kernel arguments, so a call with new buffers costs what a repeated one does.
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <numeric>
 #include <vector>
@@ -15,6 +17,7 @@
 
 #include "fused_kernels.cuh"
 #include "fused_sign_async.cuh"
+#include "fused_sign_staged.cuh"
 #include "host_impl.cuh"
 #include "profiling.cuh"
 
@@ -32,11 +35,11 @@ struct EngineBase {
     // bounds of the signer's device-side loops (FusedSignArgs)
     unsigned nonce_limit = kNonceLimit, lock_spins = kLockSpinLimit, idle_polls = kAsyncIdleLimit;
     size_t last_n = 0;  // items of the last signing batch
-    FusedQueue *q = nullptr;
-    // metadata (device) and its pinned staging
-    unsigned *d_key = nullptr, *d_mlen = nullptr, *d_order = nullptr;
-    unsigned long long *d_off = nullptr;
-    uint8_t *h_stage = nullptr;     // [FusedQueue | key | mlen | order | off]
+    // a batch's metadata (device, the queue block first) and its pinned staging:
+    // [FusedQueue, padded | off | key | mlen | order], each array as long as the batch
+    uint8_t *d_meta = nullptr, *h_stage = nullptr;
+    FusedQueue *q = nullptr;  // = d_meta
+    StagedRound *rounds = nullptr;
     FusedQueue *h_status = nullptr; // D2H copy of the queue after a batch
     cudaEvent_t stage_ev = nullptr; // recorded after a batch's metadata upload from h_stage
     // key-cache builds run their independent kernels on a side stream too (fork / join events)
@@ -45,7 +48,7 @@ struct EngineBase {
     bool stage_pending = false;
     uint8_t *scratch = nullptr;
     size_t scratch_bytes = 0;
-    int sign_grid = 0, verify_grid = 0, prehash_grid = 0;
+    int sign_grid = 0, verify_grid = 0;
     size_t sign_smem = 0, verify_smem = 0;
     // signer kernel: 0 = phased k_fused_sign (block-wide Keccak / NTT phases) with the engine's
     // block size; 1..4 = asynchronous k_fused_sign_async with (threads, slots) per block of
@@ -58,17 +61,11 @@ struct EngineBase {
     size_t async_smem[kAsyncVariants] = {0, 0, 0, 0};
     int wide_grid = 0;
     size_t wide_smem = 0;
-    // instantiated graphs, keyed by the output / message buffers they were captured with
-    cudaGraphExec_t g_sign = nullptr, g_verify = nullptr;
-    const void *g_sign_key[3] = {nullptr, nullptr, nullptr}, *g_verify_key[2] = {nullptr, nullptr};
-    // Batches of at least large_min_items items (0 = never) sign with large_kernel / large_spec
-    // through a graph of their own; smaller ones with sign_kernel / spec_slots.
+    // Batches of at least large_min_items items (0 = never) sign with large_kernel / large_spec; smaller
+    // ones with sign_kernel / spec_slots.
     size_t large_min_items = 0;
     int large_kernel = 0;
     unsigned large_spec = 0;
-    cudaGraphExec_t g_sign_large = nullptr;
-    const void *g_sign_large_key[3] = {nullptr, nullptr, nullptr};
-    cudaStream_t g_sign_stream = nullptr, g_verify_stream = nullptr;
     size_t device_bytes = 0;
     bool owns_cache = true;  // false when the key caches belong to another engine (attach_keys)
     const EngineBase *key_src = nullptr;  // that engine: its key rows are read as they stand at each call
@@ -80,7 +77,7 @@ struct EngineImpl : EngineBase {
     using PM = P<MODE>;
     using C = Cache<MODE>;
 
-    // pinned staging: [FusedQueue, padded to 64 bytes | key | mlen | order | off]
+    static constexpr int L = PM::L;
     static constexpr size_t kStageHead = (sizeof(FusedQueue) + 63) / 64 * 64;
     static size_t stage_bytes(size_t max_items) {
         return kStageHead + max_items * (3 * sizeof(unsigned) + sizeof(unsigned long long));
@@ -96,7 +93,7 @@ struct EngineImpl : EngineBase {
     // Device bytes the engine needs (the admission budget checks this before allocating).
     size_t required_bytes(size_t max_keys, size_t max_items) const {
         return max_keys * (align256(C::SK_ROW) + align256(C::PK_ROW)) + max_items * (C::ITEM_BYTES + 4 * sizeof(unsigned)) +
-               stage_bytes(max_items) + sizeof(FusedQueue) + scratch_for(max_items);
+               stage_bytes(max_items) + kStagedMaxRounds * sizeof(StagedRound) + scratch_for(max_items);
     }
     // attempt slots of the largest signer variant, or the verifier's per-signature slots
     size_t scratch_for(size_t max_items) const {
@@ -164,28 +161,20 @@ struct EngineImpl : EngineBase {
         if (rc) return rc;
         rc = configure_wide();
         if (rc) return rc;
-        prehash_grid = (int)std::min<size_t>((mi + kPrehashBlock - 1) / kPrehashBlock, (size_t)sm_count * 32);
         device_bytes = required_bytes(mk, mi);
         if (budget && device_bytes > budget) return CUDIL_ERR_BUDGET;
         sk_pitch = align256(C::SK_ROW);
         pk_pitch = align256(C::PK_ROW);
         scratch_bytes = scratch_for(mi);
         spec_slots = (unsigned)threads;
-        // large batches (about 224 items per SM and more) default to the wide phased signer
-        large_min_items = (size_t)224 * (size_t)sm_count;
-        large_kernel = kWideVariant;
-        large_spec = std::min<unsigned>(128u, 2u * (unsigned)threads);
         if ((mk && (cudaMalloc(&sk_cache, mk * sk_pitch) != cudaSuccess || cudaMalloc(&pk_cache, mk * pk_pitch) != cudaSuccess)) ||
             (mi && (cudaMalloc(&items, mi * C::ITEM_BYTES) != cudaSuccess || cudaMalloc(&best, mi * sizeof(unsigned)) != cudaSuccess ||
                     cudaMalloc(&locks, mi * sizeof(unsigned)) != cudaSuccess ||
                     cudaMalloc(&next_nonce, mi * sizeof(unsigned)) != cudaSuccess ||
                     cudaMalloc(&inflight, mi * sizeof(unsigned)) != cudaSuccess ||
-                    cudaMalloc(&d_key, mi * sizeof(unsigned)) != cudaSuccess ||
-                    cudaMalloc(&d_mlen, mi * sizeof(unsigned)) != cudaSuccess ||
-                    cudaMalloc(&d_order, mi * sizeof(unsigned)) != cudaSuccess ||
-                    cudaMalloc(&d_off, mi * sizeof(unsigned long long)) != cudaSuccess ||
                     cudaMalloc(&scratch, scratch_bytes) != cudaSuccess)) ||
-            cudaMalloc(&q, sizeof(FusedQueue)) != cudaSuccess || cudaMallocHost(&h_stage, stage_bytes(mi)) != cudaSuccess ||
+            cudaMalloc(&d_meta, stage_bytes(mi)) != cudaSuccess ||
+            cudaMalloc(&rounds, kStagedMaxRounds * sizeof(StagedRound)) != cudaSuccess || cudaMallocHost(&h_stage, stage_bytes(mi)) != cudaSuccess ||
             cudaMallocHost(&h_status, sizeof(FusedQueue)) != cudaSuccess)
             return ::cudil::cudil_record_cuda_error(cudaGetLastError(), __FILE__, __LINE__);
         std::memset(h_status, 0, sizeof(FusedQueue));
@@ -193,14 +182,12 @@ struct EngineImpl : EngineBase {
         CUDIL_CK(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
         CUDIL_CK(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming));
         CUDIL_CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        q = reinterpret_cast<FusedQueue *>(d_meta);
         CUDIL_CK(cudaMemset(q, 0, sizeof(FusedQueue)));
         return CUDIL_OK;
     }
 
     ~EngineImpl() override {
-        if (g_sign) cudaGraphExecDestroy(g_sign);
-        if (g_sign_large) cudaGraphExecDestroy(g_sign_large);
-        if (g_verify) cudaGraphExecDestroy(g_verify);
         if (owns_cache) {
             cudaFree(sk_cache);
             cudaFree(pk_cache);
@@ -210,11 +197,8 @@ struct EngineImpl : EngineBase {
         cudaFree(locks);
         cudaFree(next_nonce);
         cudaFree(inflight);
-        cudaFree(q);
-        cudaFree(d_key);
-        cudaFree(d_mlen);
-        cudaFree(d_order);
-        cudaFree(d_off);
+        cudaFree(d_meta);
+        cudaFree(rounds);
         cudaFree(scratch);
         if (h_stage) cudaFreeHost(h_stage);
         if (h_status) cudaFreeHost(h_status);
@@ -239,9 +223,6 @@ struct EngineImpl : EngineBase {
         n_sk = src->n_sk;
         n_pk = src->n_pk;
         max_keys = src->max_keys;
-        g_sign_key[0] = nullptr;  // re-capture graphs with the new cache pointers
-        g_sign_large_key[0] = nullptr;
-        g_verify_key[0] = nullptr;
         return CUDIL_OK;
     }
 
@@ -303,12 +284,13 @@ struct EngineImpl : EngineBase {
     }
 
     // ------------------------------------------------------------ metadata upload
-    int upload_meta(const unsigned long long *off, const unsigned *mlen, const unsigned *key, size_t n, size_t nkeys,
-                    size_t msgs_bytes, bool longest_first, cudaStream_t st, const uint8_t *rho_seed = nullptr,
-                    unsigned long long rho_counter = 0) {
-        // the previous batch's copies out of the staging buffer must have completed (only those:
-        // work the caller queued on the stream, such as input copies or cache builds, keeps
-        // running while this batch is prepared)
+    // Checks the batch's metadata and queues its upload; m gets the device arrays (and the caller's
+    // buffers).  An order that is the identity -- every batch of equal lengths -- does not travel.
+    int upload_meta(MsgRefs &m, const unsigned long long *off, const unsigned *mlen, const unsigned *key, size_t n, size_t nkeys,
+                    size_t msgs_bytes, cudaStream_t st, const uint8_t *rho_seed = nullptr, unsigned long long rho_counter = 0) {
+        // the previous batch's copy out of the staging buffer must have completed (only that: work the
+        // caller queued on the stream, such as input copies or cache builds, keeps running while this
+        // batch is prepared)
         if (stage_pending) CUDIL_CK(cudaEventSynchronize(stage_ev));
         FusedQueue *hq = reinterpret_cast<FusedQueue *>(h_stage);
         std::memset(hq, 0, sizeof(FusedQueue));
@@ -318,10 +300,8 @@ struct EngineImpl : EngineBase {
             hq->rho_counter = rho_counter;
             std::memcpy(hq->rho_seed, rho_seed, sizeof hq->rho_seed);
         }
-        unsigned *hk = reinterpret_cast<unsigned *>(h_stage + kStageHead);
-        unsigned *hm = hk + max_items;
-        unsigned *ho = hm + max_items;
-        unsigned long long *hoff = reinterpret_cast<unsigned long long *>(ho + max_items);
+        unsigned long long *hoff = reinterpret_cast<unsigned long long *>(h_stage + kStageHead);
+        unsigned *hk = reinterpret_cast<unsigned *>(hoff + n), *hm = hk + n, *ho = hm + n;
         bool descending = true;  // already longest first (every batch of equal lengths is)
         for (size_t i = 0; i < n; ++i) {
             if (key[i] >= nkeys || (off[i] & 7u) || off[i] > msgs_bytes || mlen[i] > msgs_bytes - off[i])
@@ -331,28 +311,26 @@ struct EngineImpl : EngineBase {
             hoff[i] = off[i];
             if (i && mlen[i] > mlen[i - 1]) descending = false;
         }
-        std::iota(ho, ho + n, 0u);
-        if (longest_first && !descending)
+        size_t bytes = kStageHead + n * (sizeof(unsigned long long) + 2 * sizeof(unsigned));
+        if (!descending) {
+            std::iota(ho, ho + n, 0u);
             std::stable_sort(ho, ho + n, [&](unsigned a, unsigned b) { return hm[a] > hm[b]; });
-        CUDIL_CK(cudaMemcpyAsync(q, hq, sizeof(FusedQueue), cudaMemcpyHostToDevice, st));
-        CUDIL_CK(cudaMemcpyAsync(d_key, hk, n * sizeof(unsigned), cudaMemcpyHostToDevice, st));
-        CUDIL_CK(cudaMemcpyAsync(d_mlen, hm, n * sizeof(unsigned), cudaMemcpyHostToDevice, st));
-        CUDIL_CK(cudaMemcpyAsync(d_order, ho, n * sizeof(unsigned), cudaMemcpyHostToDevice, st));
-        CUDIL_CK(cudaMemcpyAsync(d_off, hoff, n * sizeof(unsigned long long), cudaMemcpyHostToDevice, st));
+            bytes += n * sizeof(unsigned);
+        }
+        CUDIL_CK(cudaMemcpyAsync(d_meta, h_stage, bytes, cudaMemcpyHostToDevice, st));
         CUDIL_CK(cudaEventRecord(stage_ev, st));
         stage_pending = true;
+        m.offsets = reinterpret_cast<const unsigned long long *>(d_meta + kStageHead);
+        m.key_idx = reinterpret_cast<const unsigned *>(m.offsets + n);
+        m.mlens = m.key_idx + n;
+        m.order = descending ? nullptr : m.mlens + n;
+        m.nkeys = (unsigned)max_keys;
         return CUDIL_OK;
     }
 
-    // ------------------------------------------------------------ graphs
-    template <int T>
-    void record_sign(cudaStream_t st, uint8_t *d_sig, const uint8_t *d_msgs, const uint8_t *d_rhop, int variant,
-                     unsigned spec) {
-        MsgRefs mr{d_msgs, d_off, d_mlen, d_key, d_order, d_rhop, (unsigned)max_keys};
-        k_fused_init<<<std::max(1, sm_count * 2), 256, 0, st>>>(q, best, locks, next_nonce, inflight);
-        k_fused_prehash<MODE><<<prehash_grid, kPrehashBlock, 0, st>>>(sk_cache, sk_pitch, mr, items, q);
-        FusedSignArgs a{sk_cache, sk_pitch, d_key, items, d_sig, (size_t)PM::SIG_BYTES, scratch, q, best, locks, next_nonce,
-                        inflight, spec, nonce_limit, lock_spins, idle_polls, (unsigned)max_keys};
+    // ------------------------------------------------------------ signers
+    // one of the persistent signers, on what is pending in best[] (after k_fused_init: everything)
+    void launch_persistent(const FusedSignArgs &a, int variant, cudaStream_t st) {
         if (variant == 1)
             k_fused_sign_async<MODE, 256, 64><<<async_grid[0], 256, async_smem[0], st>>>(a);
         else if (variant == 2)
@@ -363,49 +341,80 @@ struct EngineImpl : EngineBase {
             k_fused_sign_async<MODE, 768, 192><<<async_grid[3], 768, async_smem[3], st>>>(a);
         else if (variant == kWideVariant)
             k_fused_sign<MODE, kWideThreads><<<wide_grid, kWideThreads, wide_smem, st>>>(a);
+        else if (threads == 128)
+            k_fused_sign<MODE, 128><<<sign_grid, 128, sign_smem, st>>>(a);
         else
-            k_fused_sign<MODE, T><<<sign_grid, T, sign_smem, st>>>(a);
-        cudaMemcpyAsync(h_status, q, sizeof(FusedQueue), cudaMemcpyDeviceToHost, st);
+            k_fused_sign<MODE, 256><<<sign_grid, 256, sign_smem, st>>>(a);
     }
 
-    template <int T>
-    void record_verify(cudaStream_t st, int *d_ret, const uint8_t *d_sig, const uint8_t *d_msgs) {
-        MsgRefs mr{d_msgs, d_off, d_mlen, d_key, d_order, nullptr, (unsigned)max_keys};
-        k_fused_init<<<1, 32, 0, st>>>(q, nullptr, nullptr, nullptr, nullptr);
-        k_fused_verify_prehash<MODE><<<prehash_grid, kPrehashBlock, 0, st>>>(pk_cache, pk_pitch, mr, items, q);
-        k_fused_verify<MODE, T><<<verify_grid, T, verify_smem, st>>>(pk_cache, pk_pitch, mr, d_sig, PM::SIG_BYTES, d_ret,
-                                                                    scratch, items, q);
-        cudaMemcpyAsync(h_status, q, sizeof(FusedQueue), cudaMemcpyDeviceToHost, st);
+    // Attempt slots the scratch holds beside the staged signer's lists.
+    size_t staged_cap() const {
+        const size_t lists = 2 * align256(max_items * sizeof(unsigned));
+        if (scratch_bytes <= lists) return 0;
+        return (scratch_bytes - lists) / (StagedSlot<MODE>::SIZE + 2 * sizeof(StagedAttempt));
     }
 
-    int capture(cudaStream_t st, cudaGraphExec_t *exec, bool sign, uint8_t *out, const uint8_t *sig, const uint8_t *msgs,
-                int variant = 0, unsigned spec = 0) {
-        // graphs are captured on a private stream and launched on the caller's stream
-        cudaStream_t cs;
-        CUDIL_CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-        cudaGraph_t graph;
-        cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) {
-            if (sign)
-                (threads == 128) ? record_sign<128>(cs, out, msgs, sig, variant, spec)
-                                 : record_sign<256>(cs, out, msgs, sig, variant, spec);
-            else
-                (threads == 128) ? record_verify<128>(cs, reinterpret_cast<int *>(out), sig, msgs)
-                                 : record_verify<256>(cs, reinterpret_cast<int *>(out), sig, msgs);
-            e = cudaStreamEndCapture(cs, &graph);
+    // Acceptance probability of an attempt (used only to size the enqueued rounds).
+    static constexpr double kAccept = MODE == 2 ? 0.235 : (MODE == 3 ? 0.196 : 0.26);
+
+    int sign_staged(const MsgRefs &mr, uint8_t *out, size_t n, unsigned spec, cudaStream_t st) {
+        using S = StagedSlot<MODE>;
+        StagedArgs a{};
+        a.cache = sk_cache;
+        a.cpitch = sk_pitch;
+        a.key_idx = mr.key_idx;
+        a.items = items;
+        a.sig_out = out;
+        a.sig_pitch = (size_t)PM::SIG_BYTES;
+        a.cap = (unsigned)std::min<size_t>(staged_cap(), 0x7FFFFFFFu);
+        a.pend[0] = reinterpret_cast<unsigned *>(scratch);
+        a.pend[1] = reinterpret_cast<unsigned *>(scratch + align256(max_items * sizeof(unsigned)));
+        a.slots = scratch + 2 * align256(max_items * sizeof(unsigned));
+        a.att[0] = reinterpret_cast<StagedAttempt *>(a.slots + (size_t)a.cap * S::SIZE);
+        a.att[1] = a.att[0] + a.cap;
+        a.rounds = rounds;
+        a.q = q;
+        a.best = best;
+        a.locks = locks;
+        a.next_nonce = next_nonce;
+        a.inflight = inflight;
+        a.n = (unsigned)n;
+        a.target = std::min(spec, a.cap);
+        a.nonce_limit = nonce_limit;
+        a.nkeys = (unsigned)max_keys;
+        CUDIL_CK(cudaMemsetAsync(rounds, 0, kStagedMaxRounds * sizeof(StagedRound), st));
+        CUDIL_LAUNCH(KID_ST_PREHASH, st, k_fused_prehash<MODE><<<prehash_blocks(n), kPrehashBlock, 0, st>>>(sk_cache, sk_pitch, mr, items, q));
+        CUDIL_CK_LAUNCH();
+        double p = (double)n;  // expected pending items
+        unsigned prev_slots = 0;
+        int r = 0;
+        for (; r < kStagedMaxRounds && p > 0.02; ++r) {
+            // enough blocks for a pending count four standard deviations above the expected one (kernels
+            // stride over what exceeds it)
+            const double hi = std::min((double)n, p + 4.0 * std::sqrt(p) + 4.0);
+            const double depth = std::min((double)kStagedMaxDepth, std::max(1.0, std::floor(a.target / std::max(p, 1.0))));
+            const unsigned slots = (unsigned)std::min((double)a.cap, std::max(hi, std::min((double)a.target, hi * kStagedMaxDepth)));
+            const unsigned cb = std::max(blocks_for((size_t)hi + 1, 256), std::min(blocks_for(prev_slots, 8), 8u * (unsigned)sm_count));
+            CUDIL_LAUNCH(KID_ST_CLAIM, st, k_st_claim<MODE><<<cb, 256, 0, st>>>(a, r, true));
+            const unsigned mb = (size_t)slots * L <= (size_t)sm_count * 128 ? 32u : (unsigned)kBlock;
+            CUDIL_LAUNCH(KID_ST_MASK, st, k_st_mask<MODE><<<blocks_for((size_t)slots * L, mb), mb, 0, st>>>(a, r));
+            const unsigned wb = slots <= 8u * (unsigned)sm_count ? 1u : 4u;  // warps per block
+            CUDIL_LAUNCH(KID_ST_W, st, k_st_w<MODE><<<blocks_for(slots, wb), 32 * wb, wb * S::WARP_W, st>>>(a, r));
+            CUDIL_LAUNCH(KID_ST_CHALLENGE, st, k_st_challenge<MODE><<<blocks_for(slots, kItemBlock), kItemBlock, 0, st>>>(a, r));
+            CUDIL_LAUNCH(KID_ST_REJECT, st, k_st_reject<MODE><<<blocks_for(slots, wb), 32 * wb, wb * S::WARP_R, st>>>(a, r));
+            prev_slots = slots;
+            p *= std::pow(1.0 - kAccept, depth);
         }
-        cudaStreamDestroy(cs);
-        (void)st;
-        if (e != cudaSuccess) return cudil_record_cuda_error(e, __FILE__, __LINE__);
-        if (*exec) cudaGraphExecDestroy(*exec);
-        e = cudaGraphInstantiate(exec, graph, 0);
-        cudaGraphDestroy(graph);
-        return e == cudaSuccess ? CUDIL_OK : cudil_record_cuda_error(e, __FILE__, __LINE__);
+        CUDIL_LAUNCH(KID_ST_CLAIM, st, k_st_claim<MODE><<<std::min(blocks_for(prev_slots, 8), 8u * (unsigned)sm_count), 256, 0, st>>>(a, r, false));
+        CUDIL_CK_LAUNCH();
+        return CUDIL_OK;
     }
+
+    unsigned prehash_blocks(size_t n) const { return (unsigned)std::min<size_t>(blocks_for(n, kPrehashBlock), (size_t)sm_count * 32); }
 
     // d_rhop: randomized signing seeds, 64 bytes per item (dense, device); nullptr = deterministic
     // rho_seed (host, 32 bytes): seeded randomized signing, rho' of item i derived on the device from
-    // (rho_seed, rho_counter + i); it goes up with the batch metadata, so the graph is unchanged
+    // (rho_seed, rho_counter + i); it goes up with the batch metadata
     int sign(uint8_t *d_sig, const uint8_t *d_msgs, size_t msgs_bytes, const unsigned long long *off, const unsigned *mlen,
              const unsigned *key, size_t n, cudaStream_t st, const uint8_t *d_rhop = nullptr,
              const uint8_t *rho_seed = nullptr, unsigned long long rho_counter = 0) {
@@ -418,39 +427,50 @@ struct EngineImpl : EngineBase {
             d_msgs = reinterpret_cast<const uint8_t *>(items);  // any aligned pointer; never read
         }
         if (((uintptr_t)d_msgs) & 7u) return CUDIL_ERR_INVALID;
-        const bool large = large_min_items && n >= large_min_items;
-        cudaGraphExec_t &graph = large ? g_sign_large : g_sign;
-        const void **gkey = large ? g_sign_large_key : g_sign_key;
-        const bool recapture = !graph || gkey[0] != d_sig || gkey[1] != d_msgs || gkey[2] != d_rhop;
         // The signature rows may be device memory or pinned host memory (written by the signer over
-        // PCIe as each signature is found); pageable host memory is refused before anything is queued.
+        // PCIe); pageable host memory is refused before anything is queued.
         uint8_t *out = d_sig;
-        if (recapture) {
-            cudaPointerAttributes pa{};
-            if (cudaPointerGetAttributes(&pa, d_sig) != cudaSuccess) {
-                cudaGetLastError();
-                return CUDIL_ERR_INVALID;
-            }
-            if (pa.type == cudaMemoryTypeUnregistered) return CUDIL_ERR_INVALID;
-            if (pa.type == cudaMemoryTypeHost) {
-                if (!pa.devicePointer) return CUDIL_ERR_INVALID;
-                out = static_cast<uint8_t *>(pa.devicePointer);
-            }
+        cudaPointerAttributes pa{};
+        if (cudaPointerGetAttributes(&pa, d_sig) != cudaSuccess) {
+            cudaGetLastError();
+            return CUDIL_ERR_INVALID;
         }
-        int rc = upload_meta(off, mlen, key, n, n_sk, msgs_bytes, true, st, rho_seed, rho_counter);
+        if (pa.type == cudaMemoryTypeUnregistered) return CUDIL_ERR_INVALID;
+        if (pa.type == cudaMemoryTypeHost) {
+            if (!pa.devicePointer) return CUDIL_ERR_INVALID;
+            out = static_cast<uint8_t *>(pa.devicePointer);
+        }
+        MsgRefs mr{};
+        int rc = upload_meta(mr, off, mlen, key, n, n_sk, msgs_bytes, st, rho_seed, rho_counter);
         if (rc) return rc;
-        if (recapture) {
-            // for a signing graph the `sig` argument of capture carries the randomized-signing seeds
-            rc = capture(st, &graph, true, out, d_rhop, d_msgs, large ? large_kernel : sign_kernel,
-                         large ? large_spec : spec_slots);
-            if (rc) return rc;
-            gkey[0] = d_sig;
-            gkey[1] = d_msgs;
-            gkey[2] = d_rhop;
+        mr.msgs = d_msgs;
+        mr.rhoprime = d_rhop;
+        const bool large = large_min_items && n >= large_min_items;
+        int variant = large ? large_kernel : sign_kernel;
+        unsigned spec = large ? large_spec : spec_slots;
+        // variant 0: staged rounds, then the phased kernel on what they left.  A caller that shortened the
+        // publication lock's bound gets the kernel that has that lock; more items than attempt slots go
+        // to the wide phased kernel.
+        const bool staged = variant == 0 && lock_spins == kLockSpinLimit && n <= staged_cap();
+        if (variant == 0 && lock_spins == kLockSpinLimit && !staged) {
+            variant = kWideVariant;
+            spec = std::min<unsigned>(128u, 2u * (unsigned)threads);
         }
-        CUDIL_LAUNCH(KID_FUSED_SIGN, st, cudaGraphLaunch(graph, st));
+        FusedSignArgs a{sk_cache, sk_pitch, mr.key_idx, items, out, (size_t)PM::SIG_BYTES, scratch, q, best, locks, next_nonce,
+                        inflight, spec, nonce_limit, lock_spins, idle_polls, (unsigned)max_keys};
+        cudaEvent_t ev = Profiler::get().before(st);
+        if (staged) {
+            // the target is a count per block of a four-blocks-per-SM grid, as tuned for the phased kernel
+            rc = sign_staged(mr, out, n, spec * 4u * (unsigned)sm_count, st);
+            if (rc) return rc;
+        } else {
+            k_fused_init<<<std::max(1, sm_count * 2), 256, 0, st>>>(q, best, locks, next_nonce, inflight);
+            CUDIL_LAUNCH(KID_ST_PREHASH, st, k_fused_prehash<MODE><<<prehash_blocks(n), kPrehashBlock, 0, st>>>(sk_cache, sk_pitch, mr, items, q));
+        }
+        launch_persistent(a, variant, st);
         CUDIL_CK_LAUNCH();
-        Profiler::get().launches.fetch_add(2);  // the graph holds init + prehash + sign kernels
+        Profiler::get().after(KID_FUSED_SIGN, ev, st);
+        CUDIL_CK(cudaMemcpyAsync(h_status, q, sizeof(FusedQueue), cudaMemcpyDeviceToHost, st));
         last_n = n;
         return CUDIL_OK;
     }
@@ -465,14 +485,12 @@ struct EngineImpl : EngineBase {
         return CUDIL_OK;
     }
 
-    // Bounds of the signer's loops; the signing graphs are re-captured on the next batch.
+    // Bounds of the signer's loops, from the next batch on.
     int set_limits(unsigned nonces, unsigned spins, unsigned polls) {
         if (nonces == 0 || nonces > kNonceLimit) return CUDIL_ERR_INVALID;
         nonce_limit = nonces;
         lock_spins = spins;
         idle_polls = polls;
-        g_sign_key[0] = nullptr;
-        g_sign_large_key[0] = nullptr;
         return CUDIL_OK;
     }
 
@@ -487,34 +505,31 @@ struct EngineImpl : EngineBase {
             d_msgs = reinterpret_cast<const uint8_t *>(items);
         }
         if (((uintptr_t)d_msgs) & 7u) return CUDIL_ERR_INVALID;
-        int rc = upload_meta(off, mlen, key, n, n_pk, msgs_bytes, true, st);
+        MsgRefs mr{};
+        int rc = upload_meta(mr, off, mlen, key, n, n_pk, msgs_bytes, st);
         if (rc) return rc;
-        if (!g_verify || g_verify_key[0] != d_ret || g_verify_key[1] != d_sig || d_msgs != g_verify_msgs) {
-            rc = capture(st, &g_verify, false, reinterpret_cast<uint8_t *>(d_ret), d_sig, d_msgs);
-            if (rc) return rc;
-            g_verify_key[0] = d_ret;
-            g_verify_key[1] = d_sig;
-            g_verify_msgs = d_msgs;
-        }
-        CUDIL_LAUNCH(KID_FUSED_VERIFY, st, cudaGraphLaunch(g_verify, st));
+        mr.msgs = d_msgs;
+        cudaEvent_t ev = Profiler::get().before(st);
+        CUDIL_LAUNCH(KID_ST_PREHASH, st, k_fused_verify_prehash<MODE><<<prehash_blocks(n), kPrehashBlock, 0, st>>>(pk_cache, pk_pitch, mr, items, q));
+        if (threads == 128)
+            k_fused_verify<MODE, 128><<<verify_grid, 128, verify_smem, st>>>(pk_cache, pk_pitch, mr, d_sig, PM::SIG_BYTES, d_ret, scratch, items, q);
+        else
+            k_fused_verify<MODE, 256><<<verify_grid, 256, verify_smem, st>>>(pk_cache, pk_pitch, mr, d_sig, PM::SIG_BYTES, d_ret, scratch, items, q);
         CUDIL_CK_LAUNCH();
-        Profiler::get().launches.fetch_add(1);  // the graph holds init + verify kernels
+        Profiler::get().after(KID_FUSED_VERIFY, ev, st);
+        CUDIL_CK(cudaMemcpyAsync(h_status, q, sizeof(FusedQueue), cudaMemcpyDeviceToHost, st));
         return CUDIL_OK;
     }
 
-    const uint8_t *g_verify_msgs = nullptr;
-
-    // Target of signing attempts in flight; the graph is re-captured on the next batch.
+    // Signer variant and target of signing attempts in flight, from the next batch on.
     int set_sign_kernel(int v) {
         if (v < 0 || v > kWideVariant) return CUDIL_ERR_INVALID;
         sign_kernel = v;
-        g_sign_key[0] = nullptr;
         return CUDIL_OK;
     }
 
     int set_spec_slots(unsigned v) {
         spec_slots = v ? std::min<unsigned>(v, 2u * (unsigned)threads) : (unsigned)threads;
-        g_sign_key[0] = nullptr;
         return CUDIL_OK;
     }
 
@@ -523,7 +538,6 @@ struct EngineImpl : EngineBase {
         large_min_items = min_items;
         large_kernel = variant;
         large_spec = spec ? std::min<unsigned>(spec, 2u * (unsigned)threads) : (unsigned)threads;
-        g_sign_large_key[0] = nullptr;
         return CUDIL_OK;
     }
 };

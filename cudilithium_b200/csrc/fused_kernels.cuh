@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kBlock) k_cache_pk_t1(const uint8_t *pk, uint8
 // ------------------------------------------------------------------ per-batch prologue
 
 // Messages live in one device buffer at 8-byte aligned offsets.  order[] lists the items longest
-// first so a warp's messages have similar lengths.
+// first so a warp's messages have similar lengths (nullptr: they already are).
 struct MsgRefs {
     const uint8_t *msgs;
     const unsigned long long *offsets;
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kPrehashBlock) k_fused_prehash(const uint8_t *
     using C = Cache<MODE>;
     const unsigned n = q->n;
     for (unsigned r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const unsigned it = mr.order[r];
+        const unsigned it = mr.order ? mr.order[r] : r;
         if (!bc_ok(it < n && mr.key_idx[it] < mr.nkeys, BC_PREHASH_ITEM)) continue;
         const uint8_t *row = cache + (size_t)mr.key_idx[it] * cpitch;
         uint32_t al[25], ah[25];
@@ -434,10 +434,12 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
             // atomic on its nonce counter; otherwise pass p gives one more attempt to the items
             // with at most p in flight, so a full batch spreads its slots over the items.
             const bool one_scan = D >= 2u && D * pend <= cap;
+            unsigned issued = 0;  // this lane's attempts
             auto place = [&](unsigned pos, unsigned i, unsigned nn) {
                 s_item[buf * A + pos] = i;
                 if (nn < arg.nonce_limit) {
                     s_nonce[buf * A + pos] = nn;
+                    ++issued;
                 } else {
                     // every nonce used without acceptance (never for honest keys at the default
                     // limit): the slot becomes a no-op, and the first lane to get here marks the
@@ -497,11 +499,12 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
                     if (filled > cap) filled = cap;
                 }
             }
+            issued = __reduce_add_sync(0xFFFFFFFFu, issued);
             if (lane == 0) {
                 s_ctl[CT_NA0 + buf] = filled;
                 s_ctl[CT_KJOB] = 0;
                 s_ctl[CT_NJOB] = 0;
-                if (filled) atomicAdd(&q->attempts, (unsigned long long)filled);
+                if (issued) atomicAdd(&q->attempts, (unsigned long long)issued);
             }
         }
         __syncthreads();
@@ -837,8 +840,13 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
     // ---------------- main loop (thread 0 accumulates per-phase cycles for the work counters)
     long long t_claim = 0, t_kec = 0, t_ntt = 0, t_start = clock64(), t0;
     unsigned iters = 0;
-    if (tid == 0) s_ctl[CT_PEND] = n_own;
+    // owned items still pending: all of them after k_fused_init, those the staged rounds left otherwise
+    if (tid == 0) s_ctl[CT_PEND] = 0;
     __syncthreads();
+    for (unsigned k = tid; k < n_own; k += THREADS)
+        if (__ldcg(arg.best + b0 + k * grid) == 0xFFFFFFFFu) atomicAdd(&s_ctl[CT_PEND], 1u);
+    __syncthreads();
+    if (s_ctl[CT_PEND] == 0u) return;
     claim(0);
     keccak_phase(0, 0, 0, (int)s_ctl[CT_NA0]);
     __syncthreads();
@@ -886,7 +894,7 @@ __global__ void __launch_bounds__(kPrehashBlock) k_fused_verify_prehash(const ui
     using C = Cache<MODE>;
     const unsigned n = q->n;
     for (unsigned r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const unsigned it = mr.order[r];
+        const unsigned it = mr.order ? mr.order[r] : r;
         if (!bc_ok(it < n && mr.key_idx[it] < mr.nkeys, BC_PREHASH_ITEM)) continue;
         const uint8_t *row = cache + (size_t)mr.key_idx[it] * cpitch;
         uint32_t al[25], ah[25];

@@ -1,0 +1,445 @@
+// Staged signer: the same work queue as k_fused_sign (per-item next nonce, smallest accepted nonce
+// wins), run round by round over the whole GPU instead of block by block.
+//
+// A round is five kernels over the round's attempts, each in the shape its stage needs:
+//   k_st_claim      publishes the previous round's winners, compacts the pending items and gives each its
+//                   next D nonces, D = target / pending clamped to [1, kStagedMaxDepth]
+//   k_st_mask       ExpandMask, one thread per (attempt, j) stream
+//   k_st_w          w = A y, Decompose, w1 packing: one warp per attempt, its two 16-thread groups on
+//                   different polynomials
+//   k_st_challenge  c~ = H(mu || w1) and SampleInBall, one thread per attempt
+//   k_st_reject     rejection checks and hints, one warp per attempt; an accepted attempt lowers its
+//                   item's best nonce
+// The host enqueues as many rounds as the acceptance rate calls for (EngineImpl::staged_rounds) without
+// waiting for any of them; the counts stay on the device, and a round that finds nothing pending returns
+// at once.  k_fused_sign runs last and finishes the items, if any, that the enqueued rounds left.
+//
+// Why rounds over the whole GPU: the persistent kernels bind an item to a block.  A block's rounds then
+// keep costing the latency of their dependent permutations long after most of its items are signed, and
+// one register and shared-memory budget serves every stage.  Here a round's attempts spread over all SMs
+// whatever items they belong to, and every stage runs at its own occupancy.
+#pragma once
+
+#include "fused_kernels.cuh"
+
+namespace cudil {
+
+// Counters of one round, zeroed before the batch.
+struct StagedRound {
+    unsigned npend;     // items given attempts
+    unsigned depth;     // attempts of each
+    unsigned accepted;  // items whose first accepted nonce came in this round
+    unsigned pad;
+};
+
+struct StagedAttempt {
+    unsigned item, nonce;  // nonce 0xFFFFFFFF: none (the item's nonces ran out)
+    unsigned accepted;
+    unsigned pad;
+};
+
+constexpr int kStagedMaxRounds = 40;
+constexpr unsigned kStagedMaxDepth = 64;
+constexpr unsigned kStagedPending = 0xFFFFFFFFu, kStagedNoNonce = 0xFFFFFFFFu;
+
+template <int MODE>
+struct StagedSlot {
+    using PM = P<MODE>;
+    static constexpr int K = PM::K, L = PM::L;
+    static constexpr size_t POLY = N * sizeof(int32_t);
+    static constexpr size_t Y = 0;                                          // packed y (raw ExpandMask output)
+    static constexpr size_t W0 = align256((size_t)L * PM::POLYZ_PACKED);    // [K][4 chunks][16 positions] int4
+    static constexpr size_t W1P = W0 + (size_t)K * POLY;                    // packed w1
+    static constexpr size_t W1B = W1P + align256(PM::W1PACKED_BYTES);       // [K][16 positions][16] w1 bytes
+    static constexpr size_t CM = W1B + (size_t)K * 256;                     // challenge masks
+    static constexpr size_t SIG = CM + 256;                                 // staged signature
+    static constexpr size_t SIZE = SIG + align256(PM::SIG_BYTES);
+    // shared memory of one warp of k_st_w (y_hat and two transposes) and of k_st_reject
+    static constexpr size_t WARP_W = (size_t)L * POLY + 2 * NTT_SMEM_WORDS * 4;
+    static constexpr size_t WARP_R = 2 * NTT_SMEM_WORDS * 4;
+};
+
+struct StagedArgs {
+    const uint8_t *cache;
+    size_t cpitch;
+    const unsigned *key_idx;
+    const uint8_t *items;
+    uint8_t *sig_out;
+    size_t sig_pitch;
+    uint8_t *slots;
+    StagedAttempt *att[2];  // by round parity: a claim writes one while it publishes from the other
+    unsigned *pend[2];
+    StagedRound *rounds;
+    FusedQueue *q;
+    unsigned *best, *locks, *next_nonce, *inflight;
+    unsigned n, cap;     // items, attempt slots
+    unsigned target;     // attempts a round aims at once fewer items than that are pending
+    unsigned nonce_limit;
+    unsigned nkeys;
+};
+
+__device__ __forceinline__ unsigned staged_attempts(const StagedArgs &a, int r) {
+    const unsigned long long v = (unsigned long long)a.rounds[r].npend * a.rounds[r].depth;
+    return v < a.cap ? (unsigned)v : a.cap;
+}
+
+// Round r's claim (claim = false: only the publication of round r - 1).  Positions in the pending list
+// come from an atomic counter, so the list's order varies from run to run; which nonces an item tries, and
+// so its signature, does not depend on it.
+template <int MODE>
+__global__ void __launch_bounds__(256) k_st_claim(StagedArgs a, int r, bool claim) {
+    using PM = P<MODE>;
+    using S = StagedSlot<MODE>;
+    const int lane = threadIdx.x & 31;
+    const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    if (claim) {
+        const unsigned nprev = r ? a.rounds[r - 1].npend : a.n;
+        const unsigned pending = r ? nprev - a.rounds[r - 1].accepted : a.n;
+        unsigned depth = 1;
+        if (pending) {
+            depth = a.target / pending;
+            depth = depth < 1u ? 1u : (depth > kStagedMaxDepth ? kStagedMaxDepth : depth);
+        }
+        if (tid == 0) {
+            a.rounds[r].depth = depth;
+            if (pending) atomicAdd(&a.q->iters, 1u);
+        }
+        const unsigned *prev = a.pend[(r + 1) & 1];
+        unsigned *next = a.pend[r & 1];
+        StagedAttempt *att = a.att[r & 1];
+        for (unsigned k0 = tid - lane; k0 < nprev; k0 += nthreads) {
+            const unsigned k = k0 + lane;
+            unsigned item = 0, nn = 0;
+            bool ok = k < nprev;
+            if (ok) {
+                if (r == 0) {
+                    item = k;
+                    a.best[k] = kStagedPending;
+                    a.locks[k] = 0u;
+                    a.inflight[k] = 0u;
+                } else {
+                    item = prev[k];
+                    ok = bc_ok(item < a.n, BC_SIGN_SLOT) && a.best[item] == kStagedPending;
+                    if (ok) nn = a.next_nonce[item];
+                    if (ok && nn >= a.nonce_limit) {
+                        // every nonce tried, none accepted: the item is finished (error bit 1)
+                        a.best[item] = kNonceExhausted;
+                        atomicOr(&a.q->error, 2u);
+                        ok = false;
+                    }
+                }
+            }
+            const unsigned bal = __ballot_sync(0xFFFFFFFFu, ok);
+            unsigned base = 0;
+            if (lane == 0 && bal) base = atomicAdd(&a.rounds[r].npend, (unsigned)__popc(bal));
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            unsigned issued = 0;
+            if (ok) {
+                const unsigned pos = base + __popc(bal & ((1u << lane) - 1u));
+                next[pos] = item;
+                const unsigned long long s0 = (unsigned long long)pos * depth;
+                // (more items than slots: depth is 1, and the items past the slots wait for the next round)
+                if (s0 + depth <= a.cap) {
+                    for (unsigned d = 0; d < depth; ++d) {
+                        const bool real = nn + d < a.nonce_limit;
+                        att[s0 + d] = StagedAttempt{item, real ? nn + d : kStagedNoNonce, 0u, 0u};
+                        issued += real ? 1u : 0u;
+                    }
+                }
+                a.next_nonce[item] = nn + issued;
+            }
+            issued = __reduce_add_sync(0xFFFFFFFFu, issued);
+            if (lane == 0 && issued) atomicAdd(&a.q->attempts, (unsigned long long)issued);
+        }
+    }
+    if (r == 0) return;
+    const unsigned na = staged_attempts(a, r - 1);
+    const StagedAttempt *att = a.att[(r - 1) & 1];
+    for (unsigned s = tid >> 5; s < na; s += nthreads >> 5) {
+        const StagedAttempt at = att[s];
+        if (!at.accepted || !bc_ok(at.item < a.n, BC_SIGN_SLOT) || a.best[at.item] != at.nonce) continue;
+        publish_signature<PM::SIG_BYTES, 32>(a.sig_out + (size_t)at.item * a.sig_pitch,
+                                             reinterpret_cast<const uint32_t *>(a.slots + (size_t)s * S::SIZE + S::SIG), lane);
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kBlock) k_st_mask(StagedArgs a, int r) {
+    using PM = P<MODE>;
+    using S = StagedSlot<MODE>;
+    constexpr int L = PM::L;
+    const unsigned total = staged_attempts(a, r) * L;
+    const StagedAttempt *att = a.att[r & 1];
+    for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) {
+        const unsigned s = u / L, j = u % L, item = att[s].item, nonce = att[s].nonce;
+        if (nonce == kStagedNoNonce || !bc_ok(item < a.n, BC_SIGN_SLOT)) continue;
+        uint2 rhop[8];
+        ld_lanes(rhop, a.items + (size_t)item * Cache<MODE>::ITEM_BYTES + 64);
+        expand_mask_stream<MODE>(a.slots + (size_t)s * S::SIZE + S::Y + (size_t)j * PM::POLYZ_PACKED, rhop, L * nonce + j);
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kBlock, 4) k_st_w(StagedArgs a, int r) {
+    using PM = P<MODE>;
+    using C = Cache<MODE>;
+    using S = StagedSlot<MODE>;
+    constexpr int K = PM::K, L = PM::L;
+    extern __shared__ __align__(16) uint8_t st_smem[];
+    const int lane = threadIdx.x & 31, half = lane >> 4, warp = threadIdx.x >> 5;
+    int32_t *yh = reinterpret_cast<int32_t *>(st_smem + (size_t)warp * S::WARP_W);
+    Group g;
+    g.t = lane & 15;
+    g.gmask = 0xFFFFu << (lane & 16);
+    g.sm = yh + L * N + half * NTT_SMEM_WORDS;
+    const unsigned na = staged_attempts(a, r), nwarps = gridDim.x * (blockDim.x >> 5);
+    const StagedAttempt *att = a.att[r & 1];
+    for (unsigned s = blockIdx.x * (blockDim.x >> 5) + warp; s < na; s += nwarps) {
+        const unsigned item = att[s].item;
+        if (att[s].nonce == kStagedNoNonce || !bc_ok(item < a.n, BC_SIGN_SLOT)) continue;
+        const unsigned key = a.key_idx[item];
+        if (!bc_ok(key < a.nkeys, BC_SIGN_KEY)) continue;
+        uint8_t *slot = a.slots + (size_t)s * S::SIZE;
+        __syncwarp();  // the previous attempt's y_hat has been read
+#pragma unroll 1
+        for (int j = half; j < L; j += 2) {
+            int32_t x[16];
+            unpack_z_strided<MODE>(x, slot + S::Y + (size_t)j * PM::POLYZ_PACKED, g.t);
+            ntt16s(x, g.sm, g.gmask, g.t);
+            store16_smem(yh + j * N, x, g.t);
+        }
+        __syncwarp();
+        const int32_t *mat = reinterpret_cast<const int32_t *>(a.cache + (size_t)key * a.cpitch + C::SK_MAT);
+#pragma unroll 1
+        for (int i = half; i < K; i += 2) {  // K is even
+            int32_t acc[16];
+            dot16<L, (L + 1) / 2>(acc, yh, g.t, [&](int j) { return mat + ((size_t)i * L + j) * N; });
+            intt16s(acc, g.sm, g.gmask, g.t);
+            int32_t w1[16];
+            int4 *w0 = reinterpret_cast<int4 *>(slot + S::W0 + (size_t)i * S::POLY);
+            uint32_t b[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                int32_t a0[4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) w1[4 * c + m] = decompose<MODE>(a0[m], caddq(reduce32(acc[4 * c + m])));
+                w0[16 * c + g.t] = make_int4(a0[0], a0[1], a0[2], a0[3]);
+                b[c] = (uint32_t)w1[4 * c] | (uint32_t)w1[4 * c + 1] << 8 | (uint32_t)w1[4 * c + 2] << 16 | (uint32_t)w1[4 * c + 3] << 24;
+            }
+            *reinterpret_cast<uint4 *>(slot + S::W1B + (size_t)i * 256 + 16 * g.t) = make_uint4(b[0], b[1], b[2], b[3]);
+            int32_t w1c[16];
+            strided_to_contig(g, w1, w1c);
+            uint32_t v[16];
+#pragma unroll
+            for (int m = 0; m < 16; ++m) v[m] = (uint32_t)w1c[m];
+            pack16_words<PM::W1_BITS>(
+                reinterpret_cast<uint32_t *>(slot + S::W1P + (size_t)i * PM::POLYW1_PACKED + g.t * 2 * PM::W1_BITS), v);
+        }
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kItemBlock) k_st_challenge(StagedArgs a, int r) {
+    using PM = P<MODE>;
+    using S = StagedSlot<MODE>;
+    __shared__ uint32_t s_blk[2 * 17][kItemBlock];
+    __shared__ uint32_t s_mask[16][kItemBlock];
+    const unsigned na = staged_attempts(a, r);
+    const StagedAttempt *att = a.att[r & 1];
+    for (unsigned s = blockIdx.x * kItemBlock + threadIdx.x; s < na; s += gridDim.x * kItemBlock) {
+        const unsigned item = att[s].item;
+        if (att[s].nonce == kStagedNoNonce || !bc_ok(item < a.n, BC_SIGN_SLOT)) continue;
+        uint8_t *slot = a.slots + (size_t)s * S::SIZE;
+        uint32_t al[25], ah[25];
+        TwoPart src{a.items + (size_t)item * Cache<MODE>::ITEM_BYTES, 8, slot + S::W1P, PM::W1PACKED_BYTES};
+        shake_absorb_prefetch<SHAKE256_RATE>(al, ah, src, CRHBYTES + PM::W1PACKED_BYTES);
+        keccak_f1600(al, ah);
+        uint2 ct[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) ct[w] = make_uint2(al[w], ah[w]);
+        uint2 *sg = reinterpret_cast<uint2 *>(slot + S::SIG);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) sg[w] = ct[w];
+        uint32_t *mask = &s_mask[0][threadIdx.x];
+        sample_in_ball<PM::TAU, kItemBlock>(ct, &s_blk[0][threadIdx.x], mask);
+        uint4 *mo = reinterpret_cast<uint4 *>(slot + S::CM);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            mo[k] = make_uint4(mask[(4 * k) * kItemBlock], mask[(4 * k + 1) * kItemBlock], mask[(4 * k + 2) * kItemBlock],
+                               mask[(4 * k + 3) * kItemBlock]);
+    }
+}
+
+// The checks run most selective first, a polynomial pair (2 p + half) at a time, as in k_fused_sign's
+// rejection job: r0 pairs (r0 replaces w0 in the slot, for the hints), z pairs, ct0 pairs with the hints.
+// Both groups of the warp follow the same control flow, and a rejection ends the attempt.
+template <int MODE>
+__global__ void __launch_bounds__(kBlock, 4) k_st_reject(StagedArgs a, int r) {
+    using PM = P<MODE>;
+    using C = Cache<MODE>;
+    using S = StagedSlot<MODE>;
+    constexpr int K = PM::K, L = PM::L, OMEGA = PM::OMEGA;
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    extern __shared__ __align__(16) uint8_t st_smem[];
+    const int lane = threadIdx.x & 31, lane_off = lane & 16, half = lane >> 4, warp = threadIdx.x >> 5;
+    Group g;
+    g.t = lane & 15;
+    g.gmask = 0xFFFFu << lane_off;
+    g.sm = reinterpret_cast<int32_t *>(st_smem + (size_t)warp * S::WARP_R) + half * NTT_SMEM_WORDS;
+    const unsigned na = staged_attempts(a, r), nwarps = gridDim.x * (blockDim.x >> 5);
+    StagedAttempt *att = a.att[r & 1];
+    for (unsigned s = blockIdx.x * (blockDim.x >> 5) + warp; s < na; s += nwarps) {
+        const unsigned item = att[s].item, nonce = att[s].nonce;
+        if (nonce == kStagedNoNonce || !bc_ok(item < a.n, BC_SIGN_SLOT)) continue;
+        const unsigned key = a.key_idx[item];
+        if (!bc_ok(key < a.nkeys, BC_SIGN_KEY)) continue;
+        // a smaller nonce of the item was accepted: this one cannot win (one decision per warp)
+        if (__shfl_sync(FULL, __ldcg(a.best + item) < nonce, 0)) continue;
+        uint8_t *slot = a.slots + (size_t)s * S::SIZE;
+        const uint8_t *row = a.cache + (size_t)key * a.cpitch;
+        int32_t ch[16];
+        {
+            uint32_t masks[16];
+            const uint4 *mi = reinterpret_cast<const uint4 *>(slot + S::CM);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint4 v = mi[k];
+                masks[4 * k] = v.x;
+                masks[4 * k + 1] = v.y;
+                masks[4 * k + 2] = v.z;
+                masks[4 * k + 3] = v.w;
+            }
+            challenge_strided(ch, masks, g.t);  // both groups transform c (same data, same instructions)
+        }
+        ntt16s(ch, g.sm, g.gmask, g.t);
+#pragma unroll
+        for (int m = 0; m < 16; ++m) ch[m] = scale_f(ch[m]);
+        const int32_t *s1 = reinterpret_cast<const int32_t *>(row + C::SK_S1);
+        const int32_t *s2 = reinterpret_cast<const int32_t *>(row + C::SK_S2);
+        const int32_t *t0 = reinterpret_cast<const int32_t *>(row + C::SK_T0);
+        uint8_t *hs = slot + S::SIG + PM::SIG_H;
+        // K is even; L is odd for two parameter sets, so the last z pair may leave the second group without
+        // a polynomial (it transforms zeros and stores nothing)
+        constexpr int PR = K / 2, PZ = (L + 1) / 2, NSTEP = 2 * PR + PZ;
+        auto operand = [&](int step) -> const int32_t * {
+            if (step < PR) return s2 + (size_t)(2 * step + half) * N;
+            if (step < PR + PZ) {
+                const int j = 2 * (step - PR) + half;
+                return s1 + (size_t)(j < L ? j : L - 1) * N;
+            }
+            return t0 + (size_t)(2 * (step - PR - PZ) + half) * N;
+        };
+        bool rejected = false;
+        int n_intt = 0, cnt = 0;
+        int32_t nx[16];
+        load16_contig(nx, operand(0) + 16 * g.t);
+#pragma unroll 1
+        for (int step = 0; step < NSTEP; ++step) {
+            const bool is_r0 = step < PR, is_z = !is_r0 && step < PR + PZ;
+            const int k = 2 * (is_r0 ? step : (is_z ? step - PR : step - PR - PZ)) + half;  // i, or j for z
+            const bool act = !is_z || k < L;
+            int32_t x[16];
+#pragma unroll
+            for (int m = 0; m < 16; ++m) x[m] = act ? montmul(ch[m], nx[m]) : 0;
+            // the next step's key row is in flight during this one's transform
+            if (step + 1 < NSTEP) load16_contig(nx, operand(step + 1) + 16 * g.t);
+            intt16s(x, g.sm, g.gmask, g.t);
+            n_intt += act ? 1 : 0;
+            bool bad = false;
+            if (is_z) {
+                int32_t y[16];
+                unpack_z_strided<MODE>(y, slot + S::Y + (size_t)(act ? k : 0) * PM::POLYZ_PACKED, g.t);
+#pragma unroll
+                for (int m = 0; m < 16; ++m) {
+                    x[m] = reduce32(x[m] + y[m]);
+                    bad |= act && exceeds(x[m], PM::GAMMA1 - PM::BETA);
+                }
+                if (__ballot_sync(FULL, bad)) {
+                    rejected = true;
+                    break;
+                }
+                int32_t zc[16];
+                strided_to_contig(g, x, zc);
+                if (act) {
+                    uint32_t v[16];
+#pragma unroll
+                    for (int m = 0; m < 16; ++m) v[m] = (uint32_t)(PM::GAMMA1 - zc[m]);
+                    pack16_words<PM::Z_BITS>(
+                        reinterpret_cast<uint32_t *>(slot + S::SIG + PM::SIG_Z + (size_t)k * PM::POLYZ_PACKED + g.t * 2 * PM::Z_BITS), v);
+                }
+                continue;
+            }
+            int4 *w0 = reinterpret_cast<int4 *>(slot + S::W0 + (size_t)k * S::POLY);
+            int32_t r0[16];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int4 v = w0[16 * c + g.t];
+                r0[4 * c] = v.x;
+                r0[4 * c + 1] = v.y;
+                r0[4 * c + 2] = v.z;
+                r0[4 * c + 3] = v.w;
+            }
+            if (is_r0) {
+#pragma unroll
+                for (int m = 0; m < 16; ++m) {
+                    r0[m] = reduce32(r0[m] - x[m]);
+                    bad |= exceeds(r0[m], PM::GAMMA2 - PM::BETA);
+                }
+                if (__ballot_sync(FULL, bad)) {
+                    rejected = true;
+                    break;
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) w0[16 * c + g.t] = make_int4(r0[4 * c], r0[4 * c + 1], r0[4 * c + 2], r0[4 * c + 3]);
+                continue;
+            }
+            const uint4 w1v = *reinterpret_cast<const uint4 *>(slot + S::W1B + (size_t)k * 256 + 16 * g.t);
+            const uint32_t w1w[4] = {w1v.x, w1v.y, w1v.z, w1v.w};
+            unsigned hb = 0;  // bit m = hint of coefficient t + 16 m
+#pragma unroll
+            for (int m = 0; m < 16; ++m) {
+                x[m] = reduce32(x[m]);
+                bad |= exceeds(x[m], PM::GAMMA2);
+                hb |= make_hint<MODE>(r0[m] + x[m], (int32_t)((w1w[m >> 2] >> (8 * (m & 3))) & 0xFFu)) << m;
+            }
+            if (__ballot_sync(FULL, bad)) {
+                rejected = true;
+                break;
+            }
+            // hint counts of both polynomials of the pair, then the positions in ascending coefficient
+            // order: poly 2p first, then poly 2p + 1
+            int tot = __popc(hb);
+#pragma unroll
+            for (int o = 8; o >= 1; o >>= 1) tot += __shfl_xor_sync(FULL, tot, o);
+            const int tot0 = __shfl_sync(FULL, tot, 0), tot1 = __shfl_sync(FULL, tot, 16);
+            if (cnt + tot0 + tot1 > OMEGA) {
+                rejected = true;
+                break;
+            }
+            int idx = cnt + (half ? tot0 : 0);
+#pragma unroll
+            for (int m = 0; m < 16; ++m) {
+                const unsigned bit = (hb >> m) & 1u;
+                const unsigned bal = (__ballot_sync(FULL, bit) >> lane_off) & 0xFFFFu;
+                if (bit) hs[idx + __popc(bal & ((1u << g.t) - 1u))] = (uint8_t)(g.t + 16 * m);
+                idx += __popc(bal);
+            }
+            if (g.t == 0) hs[OMEGA + k] = (uint8_t)(cnt + (half ? tot0 + tot1 : tot0));
+            cnt += tot0 + tot1;
+        }
+        n_intt += __shfl_down_sync(FULL, n_intt, 16);  // lane 0: both groups
+        if (lane == 0) atomicAdd(&a.q->intt, (unsigned long long)n_intt);
+        if (rejected) continue;
+        for (int p = cnt + lane; p < OMEGA; p += 32) hs[p] = 0;
+        if (lane == 0) {
+            att[s].accepted = 1u;
+            // the next claim publishes the attempt whose nonce is still the item's smallest
+            if (atomicMin(a.best + item, nonce) == kStagedPending) {
+                atomicAdd(&a.rounds[r].accepted, 1u);
+                atomicAdd(&a.q->done_items, 1u);
+            }
+        }
+    }
+}
+
+}  // namespace cudil

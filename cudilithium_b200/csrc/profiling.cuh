@@ -39,6 +39,12 @@ enum KernelId : int {
     KID_SIG_CHECK,
     KID_SK_CHECK,
     KID_DERIVE_RHOP,
+    KID_ST_PREHASH,
+    KID_ST_CLAIM,
+    KID_ST_MASK,
+    KID_ST_W,
+    KID_ST_CHALLENGE,
+    KID_ST_REJECT,
     KID_COUNT
 };
 
@@ -48,7 +54,8 @@ inline const char *kernel_name(int id) {
         "k_sign_expand_mask", "k_sign_compute_w", "k_sign_challenge", "k_sign_reject", "k_sig_copy",
         "k_verify_prepare", "k_verify_w", "k_verify_final", "k_ntt_mul", "k_alu_peak",
         "k_fused_sign (graph)", "k_fused_verify (graph)", "k_fused_sched", "k_cache_sk", "k_cache_pk",
-        "k_sig_check", "k_sk_check", "k_derive_rhoprime"};
+        "k_sig_check", "k_sk_check", "k_derive_rhoprime",
+        "k_fused_prehash", "k_st_claim", "k_st_mask", "k_st_w", "k_st_challenge", "k_st_reject"};
     return (id >= 0 && id < KID_COUNT) ? names[id] : "?";
 }
 
