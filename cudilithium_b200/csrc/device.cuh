@@ -70,17 +70,19 @@ __device__ __forceinline__ void expand_a_groups(const uint2 (&rho)[4], int i, in
     }
 }
 
-// The same entry, times the inverse transform's factor f (scale_f), written to out[0..255], a group of
-// eight as two 16-byte stores.  Rows start 16-byte aligned (pool rows and key-cache rows are).
+// The same entry, times the inverse transform's factor f (scale_f), written to the polynomial out in the
+// storage order of NTT-domain polynomials (ntt_at4), a group of eight as two 16-byte stores.  Rows start
+// 16-byte aligned (pool rows and key-cache rows are).
 __device__ __forceinline__ void expand_a_row(const uint2 (&rho)[4], int i, int j, int32_t *out) {
     expand_a_groups(
         rho, i, j,
         [&](int c, const uint32_t (&v)[8]) {
-            int4 *o = reinterpret_cast<int4 *>(out + c);
-            o[0] = make_int4(scale_f((int32_t)v[0]), scale_f((int32_t)v[1]), scale_f((int32_t)v[2]), scale_f((int32_t)v[3]));
-            o[1] = make_int4(scale_f((int32_t)v[4]), scale_f((int32_t)v[5]), scale_f((int32_t)v[6]), scale_f((int32_t)v[7]));
+            *reinterpret_cast<int4 *>(out + ntt_at4(c)) =
+                make_int4(scale_f((int32_t)v[0]), scale_f((int32_t)v[1]), scale_f((int32_t)v[2]), scale_f((int32_t)v[3]));
+            *reinterpret_cast<int4 *>(out + ntt_at4(c + 4)) =
+                make_int4(scale_f((int32_t)v[4]), scale_f((int32_t)v[5]), scale_f((int32_t)v[6]), scale_f((int32_t)v[7]));
         },
-        [&](int c, uint32_t v) { out[c] = scale_f((int32_t)v); });
+        [&](int c, uint32_t v) { out[ntt_at4(c & ~3) + (c & 3)] = scale_f((int32_t)v); });
 }
 
 // ExpandMask entry y_j: SHAKE256(rho' || kappa) with kappa = L*nonce + j (src/sign.cu:488-499);

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kBlock) k_cache_sk(const uint8_t *sk, uint8_t 
         dst = C::SK_T0 + (size_t)(p - L - K) * C::POLY;
     }
     ntt16s(x, g.sm, g.gmask, g.t);
-    store16_contig(reinterpret_cast<int32_t *>(row + dst) + 16 * g.t, x);
+    store16_chunks(reinterpret_cast<int32_t *>(row + dst), x, g.t);
 }
 
 // Public rows: tr = H(pk) and rho (thread per key) ...
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kBlock) k_cache_pk_t1(const uint8_t *pk, uint8
         }
     }
     ntt16s(x, g.sm, g.gmask, g.t);
-    store16_contig(reinterpret_cast<int32_t *>(rows + (size_t)it * pitch + C::PK_T1 + (size_t)i * C::POLY) + 16 * g.t, x);
+    store16_chunks(reinterpret_cast<int32_t *>(rows + (size_t)it * pitch + C::PK_T1 + (size_t)i * C::POLY), x, g.t);
 }
 
 // ------------------------------------------------------------------ per-batch prologue
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
             return t0 + (size_t)(2 * (step - PR - PZ) + half) * N;
         };
         int32_t nx[16];
-        load16_contig(nx, operand(0) + 16 * g.t);
+        load16_chunks(nx, operand(0), g.t);
 #pragma unroll 1
         for (int step = 0; step < NSTEP; ++step) {
             const bool is_r0 = step < PR, is_z = !is_r0 && step < PR + PZ;
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
             int32_t x[16];
 #pragma unroll
             for (int m = 0; m < 16; ++m) x[m] = act ? montmul(ch[m], nx[m]) : 0;
-            if (step + 1 < NSTEP) load16_contig(nx, operand(step + 1) + 16 * g.t);
+            if (step + 1 < NSTEP) load16_chunks(nx, operand(step + 1), g.t);
             int32_t *w0 = reinterpret_cast<int32_t *>(slot + C::SL_W0) + (size_t)(is_z ? 0 : k) * N;
             const uint8_t *yp = slot + C::SL_Y + (size_t)(act ? k : 0) * PM::POLYZ_PACKED;
             int32_t pre[16];

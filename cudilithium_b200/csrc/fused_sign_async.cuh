@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512) ? 1 : 512 / THREADS)
             int32_t x[16], r0[16];
             {
                 int32_t sv[16];
-                load16_contig(sv, s2 + (size_t)i * N + 16 * g.t);
+                load16_chunks(sv, s2 + (size_t)i * N, g.t);
 #pragma unroll
                 for (int m = 0; m < 16; ++m) x[m] = montmul(ch[m], sv[m]);
             }
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512) ? 1 : 512 / THREADS)
             int32_t x[16], y[16];
             if (act) {
                 int32_t sv[16];
-                load16_contig(sv, s1 + (size_t)j * N + 16 * g.t);
+                load16_chunks(sv, s1 + (size_t)j * N, g.t);
 #pragma unroll
                 for (int m = 0; m < 16; ++m) x[m] = montmul(ch[m], sv[m]);
                 unpack_z_contig<MODE>(y, slot + C::SL_Y + (size_t)j * PM::POLYZ_PACKED, g.t);  // in flight during the transform
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512) ? 1 : 512 / THREADS)
             int32_t x[16], r0[16];
             {
                 int32_t tv[16];
-                load16_contig(tv, t0 + (size_t)i * N + 16 * g.t);
+                load16_chunks(tv, t0 + (size_t)i * N, g.t);
 #pragma unroll
                 for (int m = 0; m < 16; ++m) x[m] = montmul(ch[m], tv[m]);
             }

@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_st_reject(StagedArgs a, int r) {
         bool rejected = false;
         int n_intt = 0, cnt = 0;
         int32_t nx[16];
-        load16_contig(nx, operand(0) + 16 * g.t);
+        load16_chunks(nx, operand(0), g.t);
 #pragma unroll 1
         for (int step = 0; step < NSTEP; ++step) {
             const bool is_r0 = step < PR, is_z = !is_r0 && step < PR + PZ;
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_st_reject(StagedArgs a, int r) {
 #pragma unroll
             for (int m = 0; m < 16; ++m) x[m] = act ? montmul(ch[m], nx[m]) : 0;
             // the next step's key row is in flight during this one's transform
-            if (step + 1 < NSTEP) load16_contig(nx, operand(step + 1) + 16 * g.t);
+            if (step + 1 < NSTEP) load16_chunks(nx, operand(step + 1), g.t);
             intt16s(x, g.sm, g.gmask, g.t);
             n_intt += act ? 1 : 0;
             bool bad = false;

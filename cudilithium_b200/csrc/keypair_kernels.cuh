@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(kBlock) k_kp_s1(uint8_t *pool, size_t pitch, i
     ntt16s(x, g.sm, g.gmask, g.t);
 #pragma unroll
     for (int m = 0; m < 16; ++m) x[m] = scale_f(x[m]);
+    // natural order: k_kp_t's threads walk it coefficient by coefficient
     store16_contig(reinterpret_cast<int32_t *>(row + LY::KP_S1H) + (size_t)j * N + 16 * g.t, x);
 }
 

@@ -272,7 +272,31 @@ __device__ __forceinline__ void intt16_ool(int32_t (&x)[16], int32_t *sm, unsign
     for (int i = 0; i < 16; ++i) x[i] = c.v[i];
 }
 
-// 64 contiguous bytes (natural-order NTT-domain slice 16t..16t+15) <-> registers.
+// Storage of NTT-domain polynomials (key caches, pool rows): position t's coefficients 16t..16t+15 are four
+// 16-byte chunks, chunk c of the 16 positions contiguous (word 64 c + 4 t), so that a group's 128-bit access
+// covers 256 contiguous bytes.  In natural order the positions' chunks were 64 bytes apart, a four-way
+// bank conflict in every load of A_hat (76% of the L1 data pipe in the staged w kernel).
+__device__ __forceinline__ int ntt_at4(int c) { return ((c & 12) << 4) | ((c >> 2) & ~3); }  // word of coefficient c, c % 4 == 0
+
+__device__ __forceinline__ void load16_chunks(int32_t (&x)[16], const int32_t *poly, int t) {
+    const int4 *q = reinterpret_cast<const int4 *>(poly) + t;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int4 v = q[16 * i];
+        x[4 * i] = v.x;
+        x[4 * i + 1] = v.y;
+        x[4 * i + 2] = v.z;
+        x[4 * i + 3] = v.w;
+    }
+}
+
+__device__ __forceinline__ void store16_chunks(int32_t *poly, const int32_t (&x)[16], int t) {
+    int4 *q = reinterpret_cast<int4 *>(poly) + t;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[16 * i] = make_int4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+}
+
+// 64 contiguous bytes (natural-order slice 16t..16t+15) <-> registers.
 __device__ __forceinline__ void load16_contig(int32_t (&x)[16], const int32_t *p) {
     const int4 *q = reinterpret_cast<const int4 *>(p);
 #pragma unroll
@@ -312,7 +336,7 @@ __device__ __forceinline__ void load16_smem(int32_t (&x)[16], const int32_t *pol
 }
 
 // out[i] = sum_j op(j)[16 t + i] * y_j[16 t + i] mod q (Montgomery-reduced once) over NOPS operand
-// polynomials op(j) in global memory and vectors y_j in shared memory (store16_smem layout, y_j =
+// polynomials op(j) in global memory (load16_chunks layout) and vectors y_j in shared memory (store16_smem layout, y_j =
 // yh + j N).  The products accumulate in 64 bits: |sum| < NOPS * q * 2^27 < 2^53, so |out| < 0.67 q.
 // Eight coefficients at a time, CH operands' loads in flight before the first is consumed.
 template <int NOPS, int CH, typename Op>
@@ -328,9 +352,9 @@ __device__ __forceinline__ void dot16(int32_t (&out)[16], const int32_t *yh, int
 #pragma unroll
             for (int j = 0; j < CH; ++j)
                 if (j0 + j < NOPS) {
-                    const int4 *p = reinterpret_cast<const int4 *>(op(j0 + j) + 16 * t) + 2 * h;
+                    const int4 *p = reinterpret_cast<const int4 *>(op(j0 + j)) + 32 * h + t;
                     a[j][0] = p[0];
-                    a[j][1] = p[1];
+                    a[j][1] = p[16];
                 }
 #pragma unroll
             for (int j = 0; j < CH; ++j)

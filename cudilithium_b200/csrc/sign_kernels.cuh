@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kBlock) k_sign_unpack_ntt(uint8_t *pool, size_
         dst = LY::sg_t0(mlen) + (size_t)(p - L - K) * LY::POLY;
     }
     ntt16s(x, g.sm, g.gmask, g.t);
-    store16_contig(reinterpret_cast<int32_t *>(row + dst) + 16 * g.t, x);
+    store16_chunks(reinterpret_cast<int32_t *>(row + dst), x, g.t);
 }
 
 // ------------------------------------------------------------------ per-attempt stages
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_sign_reject(const uint8_t *sign_p
     uint8_t *hs = trow + LY::TP_SIG + PM::SIG_H;
     int cnt = 0;
     int32_t nx[16];
-    load16_contig(nx, operand(0) + 16 * g.t);
+    load16_chunks(nx, operand(0), g.t);
 #pragma unroll 1
     for (int step = 0; step < NSTEP; ++step) {
         const bool is_r0 = step < PR, is_z = !is_r0 && step < PR + PZ;
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_sign_reject(const uint8_t *sign_p
         int32_t x[16];
 #pragma unroll
         for (int m = 0; m < 16; ++m) x[m] = act ? montmul(ch[m], nx[m]) : 0;
-        if (step + 1 < NSTEP) load16_contig(nx, operand(step + 1) + 16 * g.t);
+        if (step + 1 < NSTEP) load16_chunks(nx, operand(step + 1), g.t);
         intt16s(x, g.sm, g.gmask, g.t);
         bool bad = false;
         if (is_z) {
