@@ -206,14 +206,11 @@ __device__ __forceinline__ void unpack_z_contig(int32_t (&x)[16], const uint8_t 
     }
 }
 
-// c coefficients a[t + 16 i] from the challenge masks (occupied bits, negative bits).
-__device__ __forceinline__ void challenge_strided(int32_t (&x)[16], const uint32_t *masks, int t) {
+// c coefficients a[t + 16 i] from the challenge's 16 words of two-bit fields (sample_in_ball): field t of
+// word i, sign-extended.
+__device__ __forceinline__ void challenge_strided(int32_t (&x)[16], const uint32_t *fld, int t) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const uint32_t occ = masks[i >> 1], neg = masks[8 + (i >> 1)];
-        const int b = t + 16 * (i & 1);
-        x[i] = ((occ >> b) & 1u) ? (((neg >> b) & 1u) ? -1 : 1) : 0;
-    }
+    for (int i = 0; i < 16; ++i) x[i] = (int32_t)(fld[i] << (30 - 2 * t)) >> 30;
 }
 
 }  // namespace cudil

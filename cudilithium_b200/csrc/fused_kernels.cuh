@@ -323,7 +323,7 @@ struct FusedSignSmem {
     static constexpr int G = THREADS / 16;
     static constexpr size_t CTRL = 4 * THREADS * sizeof(unsigned) + 256;
     static constexpr size_t PH_N = (size_t)G * (PM::L * N * 4 + NTT_SMEM_WORDS * 4);
-    static constexpr size_t PH_K = (size_t)THREADS * (34 + 16) * 4;
+    static constexpr size_t PH_K = (size_t)THREADS * SIB_WORDS * 4;
     static constexpr size_t BYTES = CTRL + (PH_N > PH_K ? PH_N : PH_K);
 };
 
@@ -512,8 +512,8 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
 
     // ---------------- Keccak phase: challenge of batch cb (jobs < na_c), ExpandMask of batch nb
     auto keccak_phase = [&](int cb, int na_c, int nb, int na_n) {
-        uint32_t *blkw = reinterpret_cast<uint32_t *>(ph) + tid;
-        uint32_t *mask = reinterpret_cast<uint32_t *>(ph) + 34 * THREADS + tid;
+        uint32_t *sib = reinterpret_cast<uint32_t *>(ph);
+        const uint32_t *mask = sib_result<THREADS>(sib, tid);
         // ExpandMask jobs start at a multiple of 32, so no warp holds both job types (a warp runs
         // divergent branches one after the other: a mixed warp would take 8 + 5 permutations)
         const int cpad = (na_c + 31) & ~31;
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
                     uint2 *sg = reinterpret_cast<uint2 *>(slot + C::SL_SIG);
 #pragma unroll
                     for (int w = 0; w < 4; ++w) sg[w] = ct[w];
-                    sample_in_ball<PM::TAU, THREADS>(ct, blkw, mask);
+                    sample_in_ball<PM::TAU, THREADS>(ct, sib, tid);
                     uint4 *mo = reinterpret_cast<uint4 *>(slot + C::SL_CM);
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
@@ -912,7 +912,7 @@ struct FusedVerifySmem {
     using PM = P<MODE>;
     static constexpr int G = THREADS / 16;
     static constexpr size_t PH_W = (size_t)G * ((PM::L + 1) * N * 4 + NTT_SMEM_WORDS * 4 + 32);
-    static constexpr size_t PH_C = (size_t)THREADS * (34 + 16) * 4;
+    static constexpr size_t PH_C = (size_t)THREADS * SIB_WORDS * 4;
     static constexpr size_t BYTES = 256 + (PH_W > PH_C ? PH_W : PH_C);
 };
 
@@ -968,9 +968,9 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_verify(const u
             uint2 ct[4];
 #pragma unroll
             for (int w = 0; w < 4; ++w) ct[w] = make_uint2(load_lane_bytes(s + 8 * w, 8).x, load_lane_bytes(s + 8 * w, 8).y);
-            uint32_t *blkw = reinterpret_cast<uint32_t *>(ph) + tid;
-            uint32_t *mask = reinterpret_cast<uint32_t *>(ph) + 34 * THREADS + tid;
-            sample_in_ball<PM::TAU, THREADS>(ct, blkw, mask);
+            uint32_t *sib = reinterpret_cast<uint32_t *>(ph);
+            const uint32_t *mask = sib_result<THREADS>(sib, tid);
+            sample_in_ball<PM::TAU, THREADS>(ct, sib, tid);
             uint4 *mo = reinterpret_cast<uint4 *>(slot + C::VS_CM);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)

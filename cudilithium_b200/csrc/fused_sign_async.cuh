@@ -33,9 +33,9 @@ struct AsyncSignSmem {
     using PM = P<MODE>;
     static constexpr int NW = THREADS / 32;
     // per-warp work area: NTT jobs use y_hat (L polynomials) + two transpose areas; Keccak jobs use
-    // the SampleInBall scratch of 32 lanes (34 block words + 16 mask words each, interleaved)
+    // the SampleInBall scratch of 32 lanes
     static constexpr size_t WA_NTT = (size_t)PM::L * N * 4 + 2 * NTT_SMEM_WORDS * 4;
-    static constexpr size_t WA_KEC = (size_t)(34 + 16) * 32 * 4;
+    static constexpr size_t WA_KEC = (size_t)SIB_WORDS * 32 * 4;
     static constexpr size_t WA_CLAIM = (size_t)NS * 4;
     static constexpr size_t WA0 = WA_NTT > WA_KEC ? WA_NTT : WA_KEC;
     static constexpr size_t WA = ((WA0 > WA_CLAIM ? WA0 : WA_CLAIM) + 15) / 16 * 16;
@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512) ? 1 : 512 / THREADS)
 
     // ---------------------------------------------------------------- challenge (lane per slot)
     auto challenge_job = [&](unsigned s, bool act) {
-        uint32_t *blkw = reinterpret_cast<uint32_t *>(wa) + lane;
-        uint32_t *mask = reinterpret_cast<uint32_t *>(wa) + 34 * 32 + lane;
+        uint32_t *sib = reinterpret_cast<uint32_t *>(wa);
+        const uint32_t *mask = sib_result<32>(sib, lane);
         unsigned item = 0, nonce = 0;
         if (act) {
             item = s_item[s];
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512) ? 1 : 512 / THREADS)
             uint2 *sg = reinterpret_cast<uint2 *>(slot + C::SL_SIG);
 #pragma unroll
             for (int w = 0; w < 4; ++w) sg[w] = ct[w];
-            sample_in_ball<PM::TAU, 32>(ct, blkw, mask);
+            sample_in_ball<PM::TAU, 32>(ct, sib, lane);
             uint4 *mo = reinterpret_cast<uint4 *>(slot + C::SL_CM);
 #pragma unroll
             for (int k = 0; k < 4; ++k)

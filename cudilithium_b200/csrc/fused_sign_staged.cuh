@@ -242,8 +242,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kItemBlock) k_st_challenge(StagedArgs a, int r) {
     using PM = P<MODE>;
     using S = StagedSlot<MODE>;
-    __shared__ uint32_t s_blk[2 * 17][kItemBlock];
-    __shared__ uint32_t s_mask[16][kItemBlock];
+    __shared__ uint32_t s_sib[SIB_WORDS * kItemBlock];
     const unsigned na = staged_attempts(a, r);
     const StagedAttempt *att = a.att[r & 1];
     for (unsigned s = blockIdx.x * kItemBlock + threadIdx.x; s < na; s += gridDim.x * kItemBlock) {
@@ -260,8 +259,8 @@ __global__ void __launch_bounds__(kItemBlock) k_st_challenge(StagedArgs a, int r
         uint2 *sg = reinterpret_cast<uint2 *>(slot + S::SIG);
 #pragma unroll
         for (int w = 0; w < 4; ++w) sg[w] = ct[w];
-        uint32_t *mask = &s_mask[0][threadIdx.x];
-        sample_in_ball<PM::TAU, kItemBlock>(ct, &s_blk[0][threadIdx.x], mask);
+        sample_in_ball<PM::TAU, kItemBlock>(ct, s_sib, threadIdx.x);
+        const uint32_t *mask = sib_result<kItemBlock>(s_sib, threadIdx.x);
         uint4 *mo = reinterpret_cast<uint4 *>(slot + S::CM);
 #pragma unroll
         for (int k = 0; k < 4; ++k)

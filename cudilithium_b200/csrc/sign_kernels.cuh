@@ -199,12 +199,29 @@ __global__ void __launch_bounds__(kBlock) k_sign_compute_w(const uint8_t *sign_p
     }
 }
 
-// SampleInBall(c~) (src/sign.cu:767-787), one thread per challenge.  The squeezed block (34
-// words) and the result (two 256-bit masks: non-zero positions, negative positions; 16 words) live
-// in shared memory interleaved across the threads of the block -- word k of this thread at
-// [k * STRIDE] -- so the dynamically indexed accesses of neighbouring threads hit distinct banks.
+// SampleInBall(c~) (src/sign.cu:767-787), one thread per challenge: thread `self` of STRIDE threads that
+// share the scratch, SIB_WORDS words per thread.  The result is 16 words, two bits per coefficient (0, 1 or
+// 3 = -1; coefficient p in bits 2 (p % 16) of word p / 16), word k of a thread at fld[k * STRIDE] so that
+// the dynamically indexed accesses of neighbouring threads hit distinct banks; sib_result gives fld.  The
+// drawn positions are bytes of 17 words (an odd number: no two lanes' same byte in one bank).
+//
+// Two passes.  The first draws the TAU positions from the squeezed block in registers: a byte is stored
+// and the count advanced by its comparison, with no load on the way.  The second moves the coefficients,
+// c[i] = c[b], c[b] = sign, with one dependent read of the result per position (c[i] takes an atomic OR
+// that nothing waits for: coefficient i is 0 until step i).  Drawing from shared memory and moving position
+// by position on separate occupancy and sign masks took about 650 cycles a position: a challenge kernel
+// of one warp per sub-partition (8 permutations, Dilithium2) 54 us, now SIBNOW us.
+constexpr int SIB_POS_WORDS = 17, SIB_WORDS = SIB_POS_WORDS + 16;
+
+template <int STRIDE>
+__device__ __forceinline__ uint32_t *sib_result(uint32_t *scratch, int self) {
+    return scratch + SIB_POS_WORDS * STRIDE + self;
+}
+
 template <int TAU, int STRIDE>
-__device__ __forceinline__ void sample_in_ball(const uint2 (&ct)[4], uint32_t *blkw, uint32_t *mask) {
+__device__ __forceinline__ void sample_in_ball(const uint2 (&ct)[4], uint32_t *scratch, int self) {
+    static_assert(TAU <= 4 * SIB_POS_WORDS, "positions");
+    uint32_t *pos = scratch + SIB_POS_WORDS * self, *fld = sib_result<STRIDE>(scratch, self);
     uint32_t al[25], ah[25];
     keccak_zero(al, ah);
 #pragma unroll
@@ -214,45 +231,49 @@ __device__ __forceinline__ void sample_in_ball(const uint2 (&ct)[4], uint32_t *b
     }
     al[4] = 0x1Fu;
     ah[16] ^= 0x80000000u;
-    keccak_f1600(al, ah);
 #pragma unroll
-    for (int w = 0; w < 17; ++w) {
-        blkw[(2 * w) * STRIDE] = al[w];
-        blkw[(2 * w + 1) * STRIDE] = ah[w];
-    }
-    uint32_t sl = al[0], sh = ah[0];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) mask[k * STRIDE] = 0;
-    int pos = 8;
+    for (int k = 0; k < 16; ++k) fld[k * STRIDE] = 0;
+    uint32_t sl = 0, sh = 0, i = N - TAU;
+    uint8_t *out = reinterpret_cast<uint8_t *>(pos);
+    bool first = true;  // the first block's first lane holds the signs
 #pragma unroll 1
-    for (int i = N - TAU; i < N; ++i) {
-        uint32_t b;
-        do {
-            if (pos >= SHAKE256_RATE) {
-                keccak_f1600(al, ah);
+    while (i < (uint32_t)N) {
+        keccak_f1600(al, ah);
 #pragma unroll
-                for (int w = 0; w < 17; ++w) {
-                    blkw[(2 * w) * STRIDE] = al[w];
-                    blkw[(2 * w + 1) * STRIDE] = ah[w];
+        for (int w = 0; w < 2 * (SHAKE256_RATE / 8); ++w) {
+            if (w < 2 && first) continue;
+            if (i >= (uint32_t)N) break;
+            const uint32_t word = (w & 1) ? ah[w >> 1] : al[w >> 1];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const uint32_t b = (word >> (8 * m)) & 0xFFu;
+                if (b <= i && i < (uint32_t)N) {
+                    *out++ = (uint8_t)b;
+                    ++i;
                 }
-                pos = 0;
             }
-            b = (blkw[(pos >> 2) * STRIDE] >> (8 * (pos & 3))) & 0xFFu;
-            ++pos;
-        } while (b > (uint32_t)i);
-        const uint32_t wb = b >> 5, bb = 1u << (b & 31);
-        const uint32_t wi = (uint32_t)i >> 5, bi = 1u << (i & 31);
-        uint32_t *occ_b = mask + wb * STRIDE, *neg_b = mask + (8 + wb) * STRIDE;
-        uint32_t *occ_i = mask + wi * STRIDE, *neg_i = mask + (8 + wi) * STRIDE;
-        const uint32_t ob = *occ_b & bb, nb = *neg_b & bb;
-        // c[i] = c[b]
-        *occ_i = ob ? (*occ_i | bi) : (*occ_i & ~bi);
-        *neg_i = nb ? (*neg_i | bi) : (*neg_i & ~bi);
-        // c[b] = 1 - 2 * (signs & 1)
-        *occ_b |= bb;
-        *neg_b = (sl & 1u) ? (*neg_b | bb) : (*neg_b & ~bb);
-        sl = (sl >> 1) | (sh << 31);
-        sh >>= 1;
+        }
+        if (first) {
+            sl = al[0];
+            sh = ah[0];
+        }
+        first = false;
+    }
+#pragma unroll 1
+    for (int k0 = 0; k0 < TAU; k0 += 4) {
+        uint32_t pw = pos[k0 >> 2];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            if (k0 + m >= TAU) break;
+            const uint32_t b = pw & 0xFFu, p = (uint32_t)(N - TAU + k0 + m), at = 2u * (b & 15u);
+            pw >>= 8;
+            uint32_t *wb = fld + (b >> 4) * STRIDE;
+            const uint32_t v = *wb, c = (v >> at) & 3u;
+            *wb = (v & ~(3u << at)) | (((sl & 1u) ? 3u : 1u) << at);
+            if (c) atomicOr(fld + (p >> 4) * STRIDE, c << (2u * (p & 15u)));
+            sl = __funnelshift_r(sl, sh, 1);
+            sh >>= 1;
+        }
     }
 }
 
@@ -263,8 +284,7 @@ __global__ void __launch_bounds__(TB) k_sign_challenge(const uint8_t *sign_pool,
                                                        const uint32_t *exec_lut, int nexec, int nitems) {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
-    __shared__ uint32_t s_blk[2 * 17][TB];
-    __shared__ uint32_t s_mask[16][TB];
+    __shared__ uint32_t s_sib[SIB_WORDS * TB];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nexec) return;
     const uint32_t item = exec_lut[e] >> 16;
@@ -280,8 +300,8 @@ __global__ void __launch_bounds__(TB) k_sign_challenge(const uint8_t *sign_pool,
     uint2 *sig_ct = reinterpret_cast<uint2 *>(trow + LY::TP_SIG);
 #pragma unroll
     for (int w = 0; w < 4; ++w) sig_ct[w] = ct[w];
-    uint32_t *mask = &s_mask[0][threadIdx.x];
-    sample_in_ball<PM::TAU, TB>(ct, &s_blk[0][threadIdx.x], mask);
+    sample_in_ball<PM::TAU, TB>(ct, s_sib, threadIdx.x);
+    const uint32_t *mask = sib_result<TB>(s_sib, threadIdx.x);
     uint4 *mo = reinterpret_cast<uint4 *>(trow + LY::TP_CMASK);
 #pragma unroll
     for (int k = 0; k < 4; ++k)

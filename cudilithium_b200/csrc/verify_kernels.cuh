@@ -18,8 +18,7 @@ __global__ void __launch_bounds__(TB) k_verify_prepare(uint8_t *pool, size_t pit
     using PM = P<MODE>;
     using LY = Layout<MODE>;
     constexpr int K = PM::K, OMEGA = PM::OMEGA;
-    __shared__ uint32_t s_blk[2 * 17][TB];
-    __shared__ uint32_t s_mask[16][TB];
+    __shared__ uint32_t s_sib[SIB_WORDS * TB];
     const int it = blockIdx.x * blockDim.x + threadIdx.x;
     if (it >= n) return;
     uint8_t *row = pool + (size_t)it * pitch;
@@ -65,8 +64,8 @@ __global__ void __launch_bounds__(TB) k_verify_prepare(uint8_t *pool, size_t pit
 
     uint2 ct[4];
     ld_lanes(ct, row + LY::VF_SIG);
-    uint32_t *mask = &s_mask[0][threadIdx.x];
-    sample_in_ball<PM::TAU, TB>(ct, &s_blk[0][threadIdx.x], mask);
+    sample_in_ball<PM::TAU, TB>(ct, s_sib, threadIdx.x);
+    const uint32_t *mask = sib_result<TB>(s_sib, threadIdx.x);
     uint4 *mo = reinterpret_cast<uint4 *>(aux);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
