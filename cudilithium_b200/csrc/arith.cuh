@@ -188,11 +188,9 @@ __device__ __forceinline__ int32_t use_hint(int32_t a, unsigned hint) {
     }
 }
 
-// |a| >= bound, computed without branching on the sign (include/poly.cuh:41-50).
+// |a| >= bound (include/poly.cuh:41-50), for |a| < 2^31 - bound: one addition and one unsigned comparison.
 __device__ __forceinline__ bool exceeds(int32_t a, int32_t bound) {
-    int32_t t = a >> 31;
-    t = a - (t & 2 * a);
-    return t >= bound;
+    return (uint32_t)(a + (bound - 1)) > (uint32_t)(2 * bound - 2);
 }
 
 }  // namespace cudil

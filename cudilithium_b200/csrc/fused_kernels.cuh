@@ -4,7 +4,7 @@
 //  * Per-key resident cache (built once per key, reused by every message of that key):
 //      secret rows  [rho | K | tr | pad..256 | A_hat (K*L polys) | s1_hat | s2_hat | t0_hat]
 //      public rows  [rho | tr | pad..256 | A_hat (K*L polys) | t1_hat = NTT(t1 * 2^d)]
-//  * k_fused_prehash  one thread per message, longest messages first: mu = H(tr||m), rho' = H(K||mu)
+//  * k_fused_prehash  one thread (few messages: a pair) per message, longest first: mu, rho' = H(K||mu)
 //  * k_fused_sign     ONE persistent kernel for all signing attempts of a batch.  Block b owns the
 //                     items b, b + grid, ...; every item has a next-nonce counter, so its nonces are
 //                     issued in increasing order, and attempts whose item already has an accepted
@@ -132,27 +132,40 @@ __global__ void __launch_bounds__(kBlock) k_cache_sk(const uint8_t *sk, uint8_t 
     store16_chunks(reinterpret_cast<int32_t *>(row + dst), x, g.t);
 }
 
-// Public rows: tr = H(pk) and rho (thread per key) ...
-template <int MODE>
+// Public rows: tr = H(pk) and rho (thread or thread pair per key) ...
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kBlock) k_cache_pk_tr(const uint8_t *pk, uint8_t *rows, size_t pitch, int n) {
     using PM = P<MODE>;
     using C = Cache<MODE>;
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= n) return;
-    const uint8_t *p = pk + (size_t)it * PM::PK_BYTES;
-    uint8_t *row = rows + (size_t)it * pitch;
-    uint32_t al[25], ah[25];
-    // pk rows of a dense array are only 4-byte aligned when PK_BYTES % 8 != 0: read bytewise
+    using Sp = Shake256<PAIR>;
+    const int it = (blockIdx.x * blockDim.x + threadIdx.x) / Sp::LANES;
+    const bool on = it < n;
+    if (!PAIR && !on) return;
+    const uint8_t *p = pk + (size_t)(on ? it : 0) * PM::PK_BYTES;
+    uint8_t *row = rows + (size_t)(on ? it : 0) * pitch;
+    // pk rows of a dense array may start at any byte
     struct Src {
         const uint8_t *p;
-        __device__ uint2 lane(long long g) const { return load_lane_bytes(p + g * 8, (int)(PM::PK_BYTES - g * 8)); }
-    } src{p};
-    shake_absorb_prefetch<SHAKE256_RATE>(al, ah, src, PM::PK_BYTES);
-    keccak_f1600(al, ah);
-    uint2 *tr = reinterpret_cast<uint2 *>(row + C::PK_TR);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) tr[w] = make_uint2(al[w], ah[w]);
-    for (int b = 0; b < 32; ++b) row[C::PK_RHO + b] = p[b];
+        bool words;  // 4-byte aligned
+        __device__ uint2 lane(long long g) const {
+            if (words && g * 8 + 8 <= PM::PK_BYTES) {
+                const uint32_t *q = reinterpret_cast<const uint32_t *>(p + g * 8);
+                return make_uint2(q[0], q[1]);
+            }
+            return load_lane_bytes(p + g * 8, (int)(PM::PK_BYTES - g * 8));
+        }
+        __device__ uint32_t word(long long g, int h) const {
+            const long long off = g * 8 + 4 * h;
+            if (words && off + 4 <= PM::PK_BYTES) return *reinterpret_cast<const uint32_t *>(p + off);
+            return off < PM::PK_BYTES ? load_lane_bytes(p + off, (int)(PM::PK_BYTES - off)).x : 0u;
+        }
+    } src{p, (reinterpret_cast<uintptr_t>(p) & 3u) == 0u};
+    Sp sp;
+    sp.hash(src, PM::PK_BYTES, on);
+    if (!on) return;
+    sp.template store<4>(row + C::PK_TR);
+    if (!PAIR || sp.half() == 0)
+        for (int b = 0; b < 32; ++b) row[C::PK_RHO + b] = p[b];
 }
 
 // ... and t1_hat = NTT(t1 * 2^d) (group per polynomial).
@@ -203,59 +216,47 @@ struct MsgRefs {
 // spread over all SMs.
 constexpr int kPrehashBlock = 32;
 
-template <int MODE>
+// Items order[first .. first + count).
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kPrehashBlock) k_fused_prehash(const uint8_t *cache, size_t cpitch, MsgRefs mr,
-                                                                 uint8_t *items, const FusedQueue *q) {
+                                                                 uint8_t *items, const FusedQueue *q, unsigned first,
+                                                                 unsigned count) {
     using C = Cache<MODE>;
-    const unsigned n = q->n;
-    for (unsigned r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const unsigned it = mr.order ? mr.order[r] : r;
-        if (!bc_ok(it < n && mr.key_idx[it] < mr.nkeys, BC_PREHASH_ITEM)) continue;
-        const uint8_t *row = cache + (size_t)mr.key_idx[it] * cpitch;
-        uint32_t al[25], ah[25];
-        TwoPart src{row + C::SK_TR, 4, mr.msgs + mr.offsets[it], (long long)mr.mlens[it]};
-        shake_absorb_prefetch<SHAKE256_RATE>(al, ah, src, (long long)SEEDBYTES + mr.mlens[it]);
-        keccak_f1600(al, ah);
-        uint2 mu[8];
-#pragma unroll
-        for (int w = 0; w < 8; ++w) mu[w] = make_uint2(al[w], ah[w]);
-        uint2 *out = reinterpret_cast<uint2 *>(items + (size_t)it * C::ITEM_BYTES);
-#pragma unroll
-        for (int w = 0; w < 8; ++w) out[w] = mu[w];
+    using Sp = Shake256<PAIR>;
+    constexpr unsigned PER = kPrehashBlock / Sp::LANES;  // items of a block
+    for (unsigned r0 = blockIdx.x * PER; r0 < count; r0 += gridDim.x * PER) {
+        const unsigned r = r0 + threadIdx.x / Sp::LANES;
+        bool on = r < count;
+        const unsigned it = on ? (mr.order ? mr.order[first + r] : first + r) : 0u;
+        on = on && bc_ok(it < q->n && mr.key_idx[it] < mr.nkeys, BC_PREHASH_ITEM);
+        if (!PAIR && !on) continue;
+        const uint8_t *row = cache + (on ? (size_t)mr.key_idx[it] * cpitch : 0);
+        const long long ml = on ? (long long)mr.mlens[it] : 0;
+        TwoPart src{row + C::SK_TR, 4, mr.msgs + (on ? mr.offsets[it] : 0), ml};
+        Sp sp;
+        sp.hash(src, SEEDBYTES + ml, on);
+        uint8_t *out = items + (size_t)it * C::ITEM_BYTES;
+        if (on) sp.template store<8>(out);
         if (q->rho_seeded) {
+            if (!on || (PAIR && sp.half())) continue;
             uint32_t seed[8];
 #pragma unroll
             for (int w = 0; w < 8; ++w) seed[w] = q->rho_seed[w];
             uint2 rp[8];
             derive_rhoprime(rp, seed, q->rho_counter + it);
 #pragma unroll
-            for (int w = 0; w < 8; ++w) out[8 + w] = rp[w];
+            for (int w = 0; w < 8; ++w) reinterpret_cast<uint2 *>(out)[8 + w] = rp[w];
             continue;
         }
         if (mr.rhoprime) {
+            if (!on || (PAIR && sp.half())) continue;
             const uint8_t *rp = mr.rhoprime + (size_t)it * CRHBYTES;
 #pragma unroll 1
-            for (int b = 0; b < CRHBYTES; ++b) items[(size_t)it * C::ITEM_BYTES + 64 + b] = rp[b];
+            for (int b = 0; b < CRHBYTES; ++b) out[64 + b] = rp[b];
             continue;
         }
-        uint2 key[4];
-        ld_lanes(key, row + C::SK_KEY);
-        keccak_zero(al, ah);
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            al[w] = key[w].x;
-            ah[w] = key[w].y;
-        }
-#pragma unroll
-        for (int w = 0; w < 8; ++w) {
-            al[4 + w] = mu[w].x;
-            ah[4 + w] = mu[w].y;
-        }
-        al[12] ^= 0x1Fu;
-        ah[16] ^= 0x80000000u;
-        keccak_f1600(al, ah);
-#pragma unroll
-        for (int w = 0; w < 8; ++w) out[8 + w] = make_uint2(al[w], ah[w]);
+        rhoprime_from_mu(sp, row + C::SK_KEY);
+        if (on) sp.template store<8>(out + 64);
     }
 }
 
@@ -888,22 +889,25 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
 // (as k_fused_prehash for signing): one thread per message, longest first, one warp per block, the
 // absorb with the next block's lanes in flight.  A long message therefore costs its own
 // permutations on one thread instead of stalling a verifier block's first phase.
-template <int MODE>
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kPrehashBlock) k_fused_verify_prehash(const uint8_t *cache, size_t cpitch, MsgRefs mr,
                                                                         uint8_t *items, const FusedQueue *q) {
     using C = Cache<MODE>;
+    using Sp = Shake256<PAIR>;
+    constexpr unsigned PER = kPrehashBlock / Sp::LANES;
     const unsigned n = q->n;
-    for (unsigned r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const unsigned it = mr.order ? mr.order[r] : r;
-        if (!bc_ok(it < n && mr.key_idx[it] < mr.nkeys, BC_PREHASH_ITEM)) continue;
-        const uint8_t *row = cache + (size_t)mr.key_idx[it] * cpitch;
-        uint32_t al[25], ah[25];
-        TwoPart src{row + C::PK_TR, 4, mr.msgs + mr.offsets[it], (long long)mr.mlens[it]};
-        shake_absorb_prefetch<SHAKE256_RATE>(al, ah, src, (long long)SEEDBYTES + mr.mlens[it]);
-        keccak_f1600(al, ah);
-        uint2 *out = reinterpret_cast<uint2 *>(items + (size_t)it * C::ITEM_BYTES);
-#pragma unroll
-        for (int w = 0; w < 8; ++w) out[w] = make_uint2(al[w], ah[w]);
+    for (unsigned r0 = blockIdx.x * PER; r0 < n; r0 += gridDim.x * PER) {
+        const unsigned r = r0 + threadIdx.x / Sp::LANES;
+        bool on = r < n;
+        const unsigned it = on ? (mr.order ? mr.order[r] : r) : 0u;
+        on = on && bc_ok(it < n && mr.key_idx[it] < mr.nkeys, BC_PREHASH_ITEM);
+        if (!PAIR && !on) continue;
+        const uint8_t *row = cache + (on ? (size_t)mr.key_idx[it] * cpitch : 0);
+        const long long ml = on ? (long long)mr.mlens[it] : 0;
+        TwoPart src{row + C::PK_TR, 4, mr.msgs + (on ? mr.offsets[it] : 0), ml};
+        Sp sp;
+        sp.hash(src, SEEDBYTES + ml, on);
+        if (on) sp.template store<8>(items + (size_t)it * C::ITEM_BYTES);
     }
 }
 

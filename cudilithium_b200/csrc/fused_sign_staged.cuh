@@ -72,7 +72,10 @@ struct StagedArgs {
     StagedRound *rounds;
     FusedQueue *q;
     unsigned *best, *locks, *next_nonce, *inflight;
-    unsigned n, cap;     // items, attempt slots
+    const unsigned *order;  // longest message first (nullptr: item order)
+    unsigned n;             // items of the batch
+    unsigned first, count;  // this part's items: order[first .. first + count)
+    unsigned cap;           // attempt slots
     unsigned target;     // attempts a round aims at once fewer items than that are pending
     unsigned nonce_limit;
     unsigned nkeys;
@@ -93,8 +96,8 @@ __global__ void __launch_bounds__(256) k_st_claim(StagedArgs a, int r, bool clai
     const int lane = threadIdx.x & 31;
     const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     if (claim) {
-        const unsigned nprev = r ? a.rounds[r - 1].npend : a.n;
-        const unsigned pending = r ? nprev - a.rounds[r - 1].accepted : a.n;
+        const unsigned nprev = r ? a.rounds[r - 1].npend : a.count;
+        const unsigned pending = r ? nprev - a.rounds[r - 1].accepted : a.count;
         unsigned depth = 1;
         if (pending) {
             depth = a.target / pending;
@@ -113,10 +116,13 @@ __global__ void __launch_bounds__(256) k_st_claim(StagedArgs a, int r, bool clai
             bool ok = k < nprev;
             if (ok) {
                 if (r == 0) {
-                    item = k;
-                    a.best[k] = kStagedPending;
-                    a.locks[k] = 0u;
-                    a.inflight[k] = 0u;
+                    item = a.order ? a.order[a.first + k] : a.first + k;
+                    ok = bc_ok(item < a.n, BC_SIGN_SLOT);
+                    if (ok) {
+                        a.best[item] = kStagedPending;
+                        a.locks[item] = 0u;
+                        a.inflight[item] = 0u;
+                    }
                 } else {
                     item = prev[k];
                     ok = bc_ok(item < a.n, BC_SIGN_SLOT) && a.best[item] == kStagedPending;
@@ -180,7 +186,7 @@ __global__ void __launch_bounds__(kBlock) k_st_mask(StagedArgs a, int r) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kBlock, 4) k_st_w(StagedArgs a, int r) {
+__global__ void __launch_bounds__(kBlock, 6) k_st_w(StagedArgs a, int r) {
     using PM = P<MODE>;
     using C = Cache<MODE>;
     using S = StagedSlot<MODE>;
@@ -238,34 +244,29 @@ __global__ void __launch_bounds__(kBlock, 4) k_st_w(StagedArgs a, int r) {
     }
 }
 
-template <int MODE>
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kItemBlock) k_st_challenge(StagedArgs a, int r) {
     using PM = P<MODE>;
     using S = StagedSlot<MODE>;
+    using Sp = Shake256<PAIR>;
+    constexpr unsigned PER = kItemBlock / Sp::LANES;  // attempts of a block
     __shared__ uint32_t s_sib[SIB_WORDS * kItemBlock];
     const unsigned na = staged_attempts(a, r);
     const StagedAttempt *att = a.att[r & 1];
-    for (unsigned s = blockIdx.x * kItemBlock + threadIdx.x; s < na; s += gridDim.x * kItemBlock) {
-        const unsigned item = att[s].item;
-        if (att[s].nonce == kStagedNoNonce || !bc_ok(item < a.n, BC_SIGN_SLOT)) continue;
-        uint8_t *slot = a.slots + (size_t)s * S::SIZE;
-        uint32_t al[25], ah[25];
+    for (unsigned s0 = blockIdx.x * PER; s0 < na; s0 += gridDim.x * PER) {
+        const unsigned s = s0 + threadIdx.x / Sp::LANES;
+        bool on = s < na && att[s].nonce != kStagedNoNonce;
+        const unsigned item = on ? att[s].item : 0u;
+        on = on && bc_ok(item < a.n, BC_SIGN_SLOT);
+        if (!PAIR && !on) continue;
+        uint8_t *slot = a.slots + (size_t)(on ? s : 0u) * S::SIZE;
         TwoPart src{a.items + (size_t)item * Cache<MODE>::ITEM_BYTES, 8, slot + S::W1P, PM::W1PACKED_BYTES};
-        shake_absorb_prefetch<SHAKE256_RATE>(al, ah, src, CRHBYTES + PM::W1PACKED_BYTES);
-        keccak_f1600(al, ah);
-        uint2 ct[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) ct[w] = make_uint2(al[w], ah[w]);
-        uint2 *sg = reinterpret_cast<uint2 *>(slot + S::SIG);
-#pragma unroll
-        for (int w = 0; w < 4; ++w) sg[w] = ct[w];
-        sample_in_ball<PM::TAU, kItemBlock>(ct, s_sib, threadIdx.x);
-        const uint32_t *mask = sib_result<kItemBlock>(s_sib, threadIdx.x);
-        uint4 *mo = reinterpret_cast<uint4 *>(slot + S::CM);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            mo[k] = make_uint4(mask[(4 * k) * kItemBlock], mask[(4 * k + 1) * kItemBlock], mask[(4 * k + 2) * kItemBlock],
-                               mask[(4 * k + 3) * kItemBlock]);
+        Sp sp;
+        sp.hash(src, CRHBYTES + PM::W1PACKED_BYTES, on);
+        if (on) sp.template store<4>(slot + S::SIG);
+        sample_in_ball<PM::TAU, kItemBlock, PAIR>(sp, s_sib, threadIdx.x);
+        if (on && (!PAIR || sp.half() == 0)) sib_store<kItemBlock>(slot + S::CM, s_sib, threadIdx.x);
+        if constexpr (PAIR) __syncwarp();
     }
 }
 
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(kItemBlock) k_st_challenge(StagedArgs a, int r
 // rejection job: r0 pairs (r0 replaces w0 in the slot, for the hints), z pairs, ct0 pairs with the hints.
 // Both groups of the warp follow the same control flow, and a rejection ends the attempt.
 template <int MODE>
-__global__ void __launch_bounds__(kBlock, 4) k_st_reject(StagedArgs a, int r) {
+__global__ void __launch_bounds__(32, 16) k_st_reject(StagedArgs a, int r, unsigned per) {
     using PM = P<MODE>;
     using C = Cache<MODE>;
     using S = StagedSlot<MODE>;
@@ -287,7 +288,29 @@ __global__ void __launch_bounds__(kBlock, 4) k_st_reject(StagedArgs a, int r) {
     g.sm = reinterpret_cast<int32_t *>(st_smem + (size_t)warp * S::WARP_R) + half * NTT_SMEM_WORDS;
     const unsigned na = staged_attempts(a, r), nwarps = gridDim.x * (blockDim.x >> 5);
     StagedAttempt *att = a.att[r & 1];
-    for (unsigned s = blockIdx.x * (blockDim.x >> 5) + warp; s < na; s += nwarps) {
+    // per = 2: a warp takes two attempts, each group transforms one's c, and the lanes exchange them; per =
+    // 1 (rounds with fewer attempts than the GPU has room for warps): both groups transform the same c
+    for (unsigned s0 = (blockIdx.x * (blockDim.x >> 5) + warp) * per; s0 < na; s0 += nwarps * per) {
+        int32_t chg[16];
+        {
+            const unsigned sg = s0 + (per == 2u ? half : 0);
+            uint32_t fld[16];
+            const uint4 *mi = reinterpret_cast<const uint4 *>(a.slots + (size_t)(sg < na ? sg : s0) * S::SIZE + S::CM);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint4 v = mi[k];
+                fld[4 * k] = v.x;
+                fld[4 * k + 1] = v.y;
+                fld[4 * k + 2] = v.z;
+                fld[4 * k + 3] = v.w;
+            }
+            challenge_strided(chg, fld, g.t);
+        }
+        ntt16s(chg, g.sm, g.gmask, g.t);
+#pragma unroll
+        for (int m = 0; m < 16; ++m) chg[m] = scale_f(chg[m]);
+#pragma unroll 1
+        for (unsigned s = s0; s < s0 + per && s < na; ++s) {
         const unsigned item = att[s].item, nonce = att[s].nonce;
         if (nonce == kStagedNoNonce || !bc_ok(item < a.n, BC_SIGN_SLOT)) continue;
         const unsigned key = a.key_idx[item];
@@ -297,22 +320,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_st_reject(StagedArgs a, int r) {
         uint8_t *slot = a.slots + (size_t)s * S::SIZE;
         const uint8_t *row = a.cache + (size_t)key * a.cpitch;
         int32_t ch[16];
-        {
-            uint32_t masks[16];
-            const uint4 *mi = reinterpret_cast<const uint4 *>(slot + S::CM);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint4 v = mi[k];
-                masks[4 * k] = v.x;
-                masks[4 * k + 1] = v.y;
-                masks[4 * k + 2] = v.z;
-                masks[4 * k + 3] = v.w;
-            }
-            challenge_strided(ch, masks, g.t);  // both groups transform c (same data, same instructions)
-        }
-        ntt16s(ch, g.sm, g.gmask, g.t);
-#pragma unroll
-        for (int m = 0; m < 16; ++m) ch[m] = scale_f(ch[m]);
+        for (int m = 0; m < 16; ++m) ch[m] = __shfl_sync(FULL, chg[m], g.t + (s != s0 ? 16 : 0));
         const int32_t *s1 = reinterpret_cast<const int32_t *>(row + C::SK_S1);
         const int32_t *s2 = reinterpret_cast<const int32_t *>(row + C::SK_S2);
         const int32_t *t0 = reinterpret_cast<const int32_t *>(row + C::SK_T0);
@@ -437,6 +446,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_st_reject(StagedArgs a, int r) {
                 atomicAdd(&a.rounds[r].accepted, 1u);
                 atomicAdd(&a.q->done_items, 1u);
             }
+        }
         }
     }
 }

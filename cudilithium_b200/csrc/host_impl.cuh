@@ -42,6 +42,29 @@ inline unsigned blocks_for(size_t threads, int per_block = kBlock) {
     return (unsigned)((threads + per_block - 1) / per_block);
 }
 
+// SMs of the current device.
+inline int current_sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms;
+}
+
+// A launch of a kernel template on <..., PAIR> with LANES threads per item: pairs of threads per hash state
+// where `items` are few (keccak_pairs).
+#define CUDIL_PAIRED_ON(items, sms, ...)                \
+    do {                                                \
+        if (::cudil::keccak_pairs((size_t)(items), sms)) { \
+            constexpr bool PAIR = true;                 \
+            constexpr int LANES = 2;                    \
+            __VA_ARGS__;                                \
+        } else {                                        \
+            constexpr bool PAIR = false;                \
+            constexpr int LANES = 1;                    \
+            __VA_ARGS__;                                \
+        }                                               \
+    } while (0)
+#define CUDIL_PAIRED(items, ...) CUDIL_PAIRED_ON(items, ::cudil::current_sm_count(), __VA_ARGS__)
+
 __global__ void k_ntt_mul(const int32_t *a, const int32_t *b, int32_t *out, long long npolys);
 
 template <int MODE>
@@ -70,7 +93,7 @@ struct Impl {
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_KP_T, st, k_kp_t<MODE><<<blocks_for(n * K, kBlock / L), kBlock, 0, st>>>(pool, pitch, nn));
         CUDIL_CK_LAUNCH();
-        CUDIL_LAUNCH(KID_KP_TR, st, k_kp_tr<MODE><<<blocks_for(n, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, nn));
+        CUDIL_LAUNCH(KID_KP_TR, st, CUDIL_PAIRED(n, k_kp_tr<MODE, PAIR><<<blocks_for(n * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, nn)));
         CUDIL_CK_LAUNCH();
         CUDIL_CK(cudaMemcpy2DAsync(pk, PM::PK_BYTES, pool + LY::KP_PK, pitch, PM::PK_BYTES, n, out_kind, st));
         CUDIL_CK(cudaMemcpy2DAsync(sk, PM::SK_BYTES, pool + LY::KP_SK, pitch, PM::SK_BYTES, n, out_kind, st));
@@ -87,7 +110,7 @@ struct Impl {
         if (mlen) CUDIL_CK(cudaMemcpy2DAsync(pool + LY::SG_MSG, sp, m, m_pitch, mlen, n, in_kind, st));
         CUDIL_CK(cudaMemcpy2DAsync(pool + LY::SG_SK, sp, sk, sk_pitch, PM::SK_BYTES, n, in_kind, st));
         if (rhop) CUDIL_CK(cudaMemcpy2DAsync(pool + LY::SG_RHOP, sp, rhop, rhop_pitch, CRHBYTES, n, in_kind, st));
-        CUDIL_LAUNCH(KID_SIGN_PREHASH, st, k_sign_prehash<MODE><<<blocks_for(n, kItemBlock), kItemBlock, 0, st>>>(pool, sp, mlen, mlens, nn, rhop ? 1 : 0));
+        CUDIL_LAUNCH(KID_SIGN_PREHASH, st, CUDIL_PAIRED(n, k_sign_prehash<MODE, PAIR><<<blocks_for(n * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, sp, mlen, mlens, nn, rhop ? 1 : 0)));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_EXPAND_A, st, k_expand_a<MODE><<<blocks_for(n * K * L), kBlock, 0, st>>>(pool, sp, LY::SG_SK + PM::SK_RHO, LY::sg_mat(mlen), nn));
         CUDIL_CK_LAUNCH();
@@ -103,7 +126,7 @@ struct Impl {
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_SIGN_COMPUTE_W, st, k_sign_compute_w<MODE, AW><<<(unsigned)((nexec + AW - 1) / AW), kBlock, 0, st>>>(pool, sp, mlen, tpool, tp, d_exec, nexec, nitems));
         CUDIL_CK_LAUNCH();
-        CUDIL_LAUNCH(KID_SIGN_CHALLENGE, st, k_sign_challenge<MODE><<<blocks_for((size_t)nexec, kItemBlock), kItemBlock, 0, st>>>(pool, sp, tpool, tp, d_exec, nexec, nitems));
+        CUDIL_LAUNCH(KID_SIGN_CHALLENGE, st, CUDIL_PAIRED(nexec, k_sign_challenge<MODE, PAIR><<<blocks_for((size_t)nexec * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, sp, tpool, tp, d_exec, nexec, nitems)));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_SIGN_REJECT, st, k_sign_reject<MODE><<<blocks_for((size_t)nexec * 32), kBlock, 0, st>>>(pool, sp, mlen, tpool, tp, d_exec, d_done, nexec, nitems));
         CUDIL_CK_LAUNCH();
@@ -205,13 +228,13 @@ struct Impl {
         CUDIL_CK(cudaMemcpy2DAsync(pool + LY::VF_SIG, pitch, sig, sig_pitch, PM::SIG_BYTES, n, in_kind, st));
         if (mlen) CUDIL_CK(cudaMemcpy2DAsync(pool + LY::VF_TRM + SEEDBYTES, pitch, m, m_pitch, mlen, n, in_kind, st));
         CUDIL_CK(cudaMemcpy2DAsync(pool + LY::VF_PK, pitch, pk, pk_pitch, PM::PK_BYTES, n, in_kind, st));
-        CUDIL_LAUNCH(KID_VERIFY_PREPARE, st, k_verify_prepare<MODE><<<blocks_for(n, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, mlen, mlens, nn));
+        CUDIL_LAUNCH(KID_VERIFY_PREPARE, st, CUDIL_PAIRED(n, k_verify_prepare<MODE, PAIR><<<blocks_for(n * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, mlen, mlens, nn)));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_EXPAND_A, st, k_expand_a<MODE><<<blocks_for(n * K * L), kBlock, 0, st>>>(pool, pitch, LY::VF_PK, LY::vf_mat(mlen), nn));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_VERIFY_W, st, k_verify_w<MODE, AV><<<(unsigned)((n + AV - 1) / AV), kBlock, 0, st>>>(pool, pitch, mlen, nn));
         CUDIL_CK_LAUNCH();
-        CUDIL_LAUNCH(KID_VERIFY_FINAL, st, k_verify_final<MODE><<<blocks_for(n, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, mlen, nn));
+        CUDIL_LAUNCH(KID_VERIFY_FINAL, st, CUDIL_PAIRED(n, k_verify_final<MODE, PAIR><<<blocks_for(n * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, mlen, nn)));
         CUDIL_CK_LAUNCH();
         CUDIL_CK(cudaMemcpy2DAsync(ret, sizeof(int), pool + LY::vf_aux(mlen) + 68, pitch, sizeof(int), n, out_kind, st));
         return CUDIL_OK;

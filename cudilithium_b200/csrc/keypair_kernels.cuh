@@ -7,7 +7,7 @@
 //   k_kp_t     one thread per ExpandA entry, products A_ij * s1_hat_j summed into the block's rows of
 //              t_hat in shared memory (no A matrix is stored), then per row invNTT, + s2, Power2Round,
 //              t1/t0 packing
-//   k_kp_tr    one thread per key: tr = SHAKE256(pk, 32)
+//   k_kp_tr    one thread or thread pair per key: tr = SHAKE256(pk, 32)
 #pragma once
 
 #include "sign_kernels.cuh"
@@ -246,20 +246,19 @@ __global__ void __launch_bounds__(kBlock) k_kp_t(uint8_t *pool, size_t pitch, in
     }
 }
 
-template <int MODE>
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kBlock) k_kp_tr(uint8_t *pool, size_t pitch, int n) {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= n) return;
-    uint8_t *row = pool + (size_t)it * pitch;
-    uint32_t al[25], ah[25];
+    using Sp = Shake256<PAIR>;
+    const int it = (blockIdx.x * blockDim.x + threadIdx.x) / Sp::LANES;
+    const bool on = it < n;
+    if (!PAIR && !on) return;
+    uint8_t *row = pool + (size_t)(on ? it : 0) * pitch;
     AlignedBytes pk{row + LY::KP_PK, PM::PK_BYTES};
-    shake_absorb_prefetch<SHAKE256_RATE>(al, ah, pk, PM::PK_BYTES);
-    keccak_f1600(al, ah);
-    uint2 *tr = reinterpret_cast<uint2 *>(row + LY::KP_SK + PM::SK_TR);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) tr[w] = make_uint2(al[w], ah[w]);
+    Sp sp;
+    sp.hash(pk, PM::PK_BYTES, on);
+    if (on) sp.template store<4>(row + LY::KP_SK + PM::SK_TR);
 }
 
 }  // namespace cudil

@@ -21,48 +21,52 @@ constexpr int kBlock = 128;             // threads per block for the SHAKE-strea
 constexpr int kGroupsPerBlock = 8;      // 16-thread groups per 128-thread block
 constexpr int kItemBlock = 32;          // threads per block for thread-per-item kernels
 
+// rho' = SHAKE256(K || mu, 64) into sp's digest, mu being its digest so far (96 bytes, one block).
+template <bool PAIR>
+__device__ __forceinline__ void rhoprime_from_mu(Shake256<PAIR> &sp, const uint8_t *key) {
+    uint32_t bl[12], bh[PAIR ? 1 : 12];
+#pragma unroll
+    for (int w = 0; w < 12; ++w) {
+        if constexpr (PAIR) {
+            bl[w] = w < 4 ? reinterpret_cast<const uint32_t *>(key)[2 * w + sp.half()] : sp.dlo[w < 4 ? 0 : w - 4];
+        } else {
+            const uint2 k = w < 4 ? ld_lane(key + 8 * w) : make_uint2(sp.dlo[w < 4 ? 0 : w - 4], sp.dhi[w < 4 ? 0 : w - 4]);
+            bl[w] = k.x;
+            bh[w] = k.y;
+        }
+    }
+    sp.template one_block<12>(bl, bh);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        sp.dlo[w] = sp.lo[w];
+        if constexpr (!PAIR) sp.dhi[w] = sp.hi[w];
+    }
+}
+
 // ------------------------------------------------------------------ per-item setup
 
+// Fewer items than this fill every sub-partition with one warp of 16 pairs but not with one of 32 states:
+// kernels that hash one message per item then use two threads per state (keccak_f1600_pair).
+inline bool keccak_pairs(size_t items, int sm_count) { return items <= (size_t)sm_count * 4 * 16; }
+
 // rhop_given: rho' was placed in the row by the caller (randomized signing), only mu is computed.
-template <int MODE>
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kBlock) k_sign_prehash(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens,
                                                          int n, int rhop_given) {
     using LY = Layout<MODE>;
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= n) return;
-    uint8_t *row = pool + (size_t)it * pitch;
-    const size_t ml = mlens ? (size_t)mlens[it] : mlen;  // per-item length (<= mlen) when given
-    uint32_t al[25], ah[25];
+    using Sp = Shake256<PAIR>;
+    const int it = (blockIdx.x * blockDim.x + threadIdx.x) / Sp::LANES;
+    const bool on = it < n;
+    if (!PAIR && !on) return;
+    uint8_t *row = pool + (size_t)(on ? it : 0) * pitch;
+    const size_t ml = mlens ? (size_t)mlens[on ? it : 0] : mlen;  // per-item length (<= mlen) when given
     TwoPart src{row + LY::SG_SK + P<MODE>::SK_TR, 4, row + LY::SG_MSG, (long long)ml};
-    shake_absorb_prefetch<SHAKE256_RATE>(al, ah, src, (long long)(SEEDBYTES + ml));
-    keccak_f1600(al, ah);
-    uint2 mu[8];
-#pragma unroll
-    for (int w = 0; w < 8; ++w) mu[w] = make_uint2(al[w], ah[w]);
-    uint2 *mu_out = reinterpret_cast<uint2 *>(row + LY::SG_MU);
-#pragma unroll
-    for (int w = 0; w < 8; ++w) mu_out[w] = mu[w];
+    Sp sp;
+    sp.hash(src, (long long)(SEEDBYTES + ml), on);
+    if (on) sp.template store<8>(row + LY::SG_MU);
     if (rhop_given) return;
-    // rho' = SHAKE256(K || mu, 64): 96 bytes, one block
-    uint2 key[4];
-    ld_lanes(key, row + LY::SG_SK + P<MODE>::SK_KEY);
-    keccak_zero(al, ah);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-        al[w] = key[w].x;
-        ah[w] = key[w].y;
-    }
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-        al[4 + w] = mu[w].x;
-        ah[4 + w] = mu[w].y;
-    }
-    al[12] ^= 0x1Fu;
-    ah[16] ^= 0x80000000u;
-    keccak_f1600(al, ah);
-    uint2 *rp = reinterpret_cast<uint2 *>(row + LY::SG_RHOP);
-#pragma unroll
-    for (int w = 0; w < 8; ++w) rp[w] = make_uint2(al[w], ah[w]);
+    rhoprime_from_mu(sp, row + LY::SG_SK + P<MODE>::SK_KEY);
+    if (on) sp.template store<8>(row + LY::SG_RHOP);
 }
 
 // One thread per ExpandA entry; rho at row+rho_off, A_hat (K*L polys) at row+mat_off.
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(kBlock) k_sign_compute_w(const uint8_t *sign_p
 // c[i] = c[b], c[b] = sign, with one dependent read of the result per position (c[i] takes an atomic OR
 // that nothing waits for: coefficient i is 0 until step i).  Drawing from shared memory and moving position
 // by position on separate occupancy and sign masks took about 650 cycles a position: a challenge kernel
-// of one warp per sub-partition (8 permutations, Dilithium2) 54 us, now SIBNOW us.
+// of one warp per sub-partition (8 permutations, Dilithium2) took 54 us.
 constexpr int SIB_POS_WORDS = 17, SIB_WORDS = SIB_POS_WORDS + 16;
 
 template <int STRIDE>
@@ -218,32 +222,39 @@ __device__ __forceinline__ uint32_t *sib_result(uint32_t *scratch, int self) {
     return scratch + SIB_POS_WORDS * STRIDE + self;
 }
 
-template <int TAU, int STRIDE>
-__device__ __forceinline__ void sample_in_ball(const uint2 (&ct)[4], uint32_t *scratch, int self) {
+template <int TAU, int STRIDE, bool PAIR = false>
+__device__ __forceinline__ void sample_in_ball(Shake256<PAIR> &sp, uint32_t *scratch, int self) {
     static_assert(TAU <= 4 * SIB_POS_WORDS, "positions");
     uint32_t *pos = scratch + SIB_POS_WORDS * self, *fld = sib_result<STRIDE>(scratch, self);
-    uint32_t al[25], ah[25];
-    keccak_zero(al, ah);
+    // the block c~ (the digest's first four lanes), then SHAKE256 of it
+    uint32_t cl[4], ch[PAIR ? 1 : 4];
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-        al[w] = ct[w].x;
-        ah[w] = ct[w].y;
+        cl[w] = sp.dlo[w];
+        if constexpr (!PAIR) ch[w] = sp.dhi[w];
     }
-    al[4] = 0x1Fu;
-    ah[16] ^= 0x80000000u;
+    sp.template one_block<4>(cl, ch);
+    // (pair form: the even thread draws; its odd neighbour hands it the high halves)
+    const bool draws = !PAIR || sp.half() == 0;
+    if (draws) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) fld[k * STRIDE] = 0;
-    uint32_t sl = 0, sh = 0, i = N - TAU;
+        for (int k = 0; k < 16; ++k) fld[k * STRIDE] = 0;
+    }
+    uint32_t sl = 0, sh = 0, i = draws ? N - TAU : N;
     uint8_t *out = reinterpret_cast<uint8_t *>(pos);
     bool first = true;  // the first block's first lane holds the signs
 #pragma unroll 1
-    while (i < (uint32_t)N) {
-        keccak_f1600(al, ah);
+    for (;;) {
 #pragma unroll
         for (int w = 0; w < 2 * (SHAKE256_RATE / 8); ++w) {
-            if (w < 2 && first) continue;
-            if (i >= (uint32_t)N) break;
-            const uint32_t word = (w & 1) ? ah[w >> 1] : al[w >> 1];
+            uint32_t word;
+            if constexpr (PAIR)
+                word = (w & 1) ? __shfl_xor_sync(0xFFFFFFFFu, sp.lo[w >> 1], 1) : sp.lo[w >> 1];
+            else
+                word = (w & 1) ? sp.hi[w >> 1] : sp.lo[w >> 1];
+            if (first && w == 0) sl = word;
+            if (first && w == 1) sh = word;
+            if ((w < 2 && first) || i >= (uint32_t)N) continue;
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 const uint32_t b = (word >> (8 * m)) & 0xFFu;
@@ -253,12 +264,15 @@ __device__ __forceinline__ void sample_in_ball(const uint2 (&ct)[4], uint32_t *s
                 }
             }
         }
-        if (first) {
-            sl = al[0];
-            sh = ah[0];
-        }
         first = false;
+        if constexpr (PAIR) {
+            if (!__any_sync(0xFFFFFFFFu, i < (uint32_t)N)) break;
+        } else {
+            if (i >= (uint32_t)N) break;
+        }
+        sp.permute();
     }
+    if (!draws) return;
 #pragma unroll 1
     for (int k0 = 0; k0 < TAU; k0 += 4) {
         uint32_t pw = pos[k0 >> 2];
@@ -277,35 +291,49 @@ __device__ __forceinline__ void sample_in_ball(const uint2 (&ct)[4], uint32_t *s
     }
 }
 
+// The same from the 32 bytes of c~ in four lanes, one thread per challenge.
+template <int TAU, int STRIDE>
+__device__ __forceinline__ void sample_in_ball(const uint2 (&ct)[4], uint32_t *scratch, int self) {
+    Shake256<false> sp;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        sp.dlo[w] = ct[w].x;
+        sp.dhi[w] = ct[w].y;
+    }
+    sample_in_ball<TAU, STRIDE, false>(sp, scratch, self);
+}
+
+// Copies a challenge's result (16 words) to 64 bytes at p.
+template <int STRIDE>
+__device__ __forceinline__ void sib_store(uint8_t *p, const uint32_t *scratch, int self) {
+    const uint32_t *f = scratch + SIB_POS_WORDS * STRIDE + self;
+    uint4 *o = reinterpret_cast<uint4 *>(p);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        o[k] = make_uint4(f[(4 * k) * STRIDE], f[(4 * k + 1) * STRIDE], f[(4 * k + 2) * STRIDE], f[(4 * k + 3) * STRIDE]);
+}
+
 // Thread-per-item kernels run TB = kItemBlock threads per block so that batches of a few thousand
 // items still spread over every SM.
-template <int MODE, int TB = kItemBlock>
+template <int MODE, bool PAIR, int TB = kItemBlock>
 __global__ void __launch_bounds__(TB) k_sign_challenge(const uint8_t *sign_pool, size_t sp, uint8_t *temp_pool, size_t tp,
                                                        const uint32_t *exec_lut, int nexec, int nitems) {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
+    using Sp = Shake256<PAIR>;
     __shared__ uint32_t s_sib[SIB_WORDS * TB];
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nexec) return;
-    const uint32_t item = exec_lut[e] >> 16;
-    if (!bc_ok(item < (uint32_t)nitems, BC_STAGE_ITEM)) return;
-    uint8_t *trow = temp_pool + (size_t)e * tp;
-    uint32_t al[25], ah[25];
-    TwoPart src{sign_pool + (size_t)item * sp + LY::SG_MU, 8, trow + LY::TP_W1P, PM::W1PACKED_BYTES};
-    shake_absorb<SHAKE256_RATE>(al, ah, src, CRHBYTES + PM::W1PACKED_BYTES);
-    keccak_f1600(al, ah);
-    uint2 ct[4];
-#pragma unroll
-    for (int w = 0; w < 4; ++w) ct[w] = make_uint2(al[w], ah[w]);
-    uint2 *sig_ct = reinterpret_cast<uint2 *>(trow + LY::TP_SIG);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) sig_ct[w] = ct[w];
-    sample_in_ball<PM::TAU, TB>(ct, s_sib, threadIdx.x);
-    const uint32_t *mask = sib_result<TB>(s_sib, threadIdx.x);
-    uint4 *mo = reinterpret_cast<uint4 *>(trow + LY::TP_CMASK);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        mo[k] = make_uint4(mask[(4 * k) * TB], mask[(4 * k + 1) * TB], mask[(4 * k + 2) * TB], mask[(4 * k + 3) * TB]);
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) / Sp::LANES;
+    bool on = e < nexec;
+    const uint32_t item = on ? exec_lut[e] >> 16 : 0u;
+    on = on && bc_ok(item < (uint32_t)nitems, BC_STAGE_ITEM);
+    if (!PAIR && !on) return;
+    uint8_t *trow = temp_pool + (size_t)(on ? e : 0) * tp;
+    TwoPart src{sign_pool + (size_t)(on ? item : 0u) * sp + LY::SG_MU, 8, trow + LY::TP_W1P, PM::W1PACKED_BYTES};
+    Sp sh;
+    sh.hash(src, CRHBYTES + PM::W1PACKED_BYTES, on);
+    if (on) sh.template store<4>(trow + LY::TP_SIG);
+    sample_in_ball<PM::TAU, TB, PAIR>(sh, s_sib, threadIdx.x);
+    if (on && (!PAIR || sh.half() == 0)) sib_store<TB>(trow + LY::TP_CMASK, s_sib, threadIdx.x);
 }
 
 // One warp per attempt: c_hat = NTT(c); r0 = w0 - c*s2, z = y + c*s1 and c*t0 (norm checks);

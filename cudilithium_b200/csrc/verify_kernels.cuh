@@ -12,22 +12,25 @@
 
 namespace cudil {
 
-template <int MODE, int TB = kItemBlock>
+template <int MODE, bool PAIR, int TB = kItemBlock>
 __global__ void __launch_bounds__(TB) k_verify_prepare(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens,
                                                        int n) {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
+    using Sp = Shake256<PAIR>;
     constexpr int K = PM::K, OMEGA = PM::OMEGA;
     __shared__ uint32_t s_sib[SIB_WORDS * TB];
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= n) return;
-    uint8_t *row = pool + (size_t)it * pitch;
+    const int it = (blockIdx.x * blockDim.x + threadIdx.x) / Sp::LANES;
+    const bool on = it < n;
+    if (!PAIR && !on) return;
+    uint8_t *row = pool + (size_t)(on ? it : 0) * pitch;
     uint8_t *aux = row + LY::vf_aux(mlen);
+    Sp sp;
 
     // hint encoding: per-poly counts non-decreasing and <= OMEGA, positions strictly increasing
     // inside each poly, unused slots zero
     int status = 0;
-    {
+    if (on && (!PAIR || sp.half() == 0)) {
         const uint8_t *h = row + LY::VF_SIG + PM::SIG_H;
         int k = 0;
         for (int i = 0; i < K && !status; ++i) {
@@ -43,34 +46,33 @@ __global__ void __launch_bounds__(TB) k_verify_prepare(uint8_t *pool, size_t pit
         if (!status)
             for (int j = k; j < OMEGA; ++j)
                 if (h[j]) status = 1;
+        reinterpret_cast<int *>(aux + 64)[0] = status;
     }
+    __syncwarp();
 
-    uint32_t al[25], ah[25];
     // tr' = SHAKE256(pk, 32) -> row + VF_TRM (m follows it)
     AlignedBytes pk{row + LY::VF_PK, PM::PK_BYTES};
-    shake_absorb_prefetch<SHAKE256_RATE>(al, ah, pk, PM::PK_BYTES);
-    keccak_f1600(al, ah);
-    uint2 *trm = reinterpret_cast<uint2 *>(row + LY::VF_TRM);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) trm[w] = make_uint2(al[w], ah[w]);
+    sp.hash(pk, PM::PK_BYTES, on);
+    if (on) sp.template store<4>(row + LY::VF_TRM);
+    __syncwarp();  // (pair form: each thread wrote its halves)
     // mu = SHAKE256(tr' || m, 64); per-item length (<= mlen) when given
-    const size_t ml = mlens ? (size_t)mlens[it] : mlen;
+    const size_t ml = mlens ? (size_t)mlens[on ? it : 0] : mlen;
     AlignedBytes tm{row + LY::VF_TRM, (long long)(SEEDBYTES + ml)};
-    shake_absorb_prefetch<SHAKE256_RATE>(al, ah, tm, (long long)(SEEDBYTES + ml));
-    keccak_f1600(al, ah);
-    uint2 *mu = reinterpret_cast<uint2 *>(row + LY::vf_mu(mlen));
-#pragma unroll
-    for (int w = 0; w < 8; ++w) mu[w] = make_uint2(al[w], ah[w]);
+    sp.hash(tm, (long long)(SEEDBYTES + ml), on);
+    if (on) sp.template store<8>(row + LY::vf_mu(mlen));
 
-    uint2 ct[4];
-    ld_lanes(ct, row + LY::VF_SIG);
-    sample_in_ball<PM::TAU, TB>(ct, s_sib, threadIdx.x);
-    const uint32_t *mask = sib_result<TB>(s_sib, threadIdx.x);
-    uint4 *mo = reinterpret_cast<uint4 *>(aux);
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-        mo[k] = make_uint4(mask[(4 * k) * TB], mask[(4 * k + 1) * TB], mask[(4 * k + 2) * TB], mask[(4 * k + 3) * TB]);
-    reinterpret_cast<int *>(aux + 64)[0] = status;
+    for (int w = 0; w < 4; ++w) {
+        const uint2 v = ld_lane(row + LY::VF_SIG + 8 * w);
+        if constexpr (PAIR) {
+            sp.dlo[w] = sp.half() ? v.y : v.x;
+        } else {
+            sp.dlo[w] = v.x;
+            sp.dhi[w] = v.y;
+        }
+    }
+    sample_in_ball<PM::TAU, TB, PAIR>(sp, s_sib, threadIdx.x);
+    if (on && (!PAIR || sp.half() == 0)) sib_store<TB>(aux, s_sib, threadIdx.x);
 }
 
 // AV signatures per 128-thread block.  Phase 1 units: (sig, j<L) -> z_hat_j, (sig, L) -> c_hat.
@@ -173,25 +175,30 @@ __global__ void __launch_bounds__(kBlock) k_verify_w(uint8_t *pool, size_t pitch
     }
 }
 
-template <int MODE>
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kBlock) k_verify_final(uint8_t *pool, size_t pitch, size_t mlen, int n) {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= n) return;
-    uint8_t *row = pool + (size_t)it * pitch;
+    using Sp = Shake256<PAIR>;
+    const int it = (blockIdx.x * blockDim.x + threadIdx.x) / Sp::LANES;
+    const bool on = it < n;
+    if (!PAIR && !on) return;
+    uint8_t *row = pool + (size_t)(on ? it : 0) * pitch;
     uint8_t *aux = row + LY::vf_aux(mlen);
-    uint32_t al[25], ah[25];
     AlignedBytes src{row + LY::vf_mu(mlen), CRHBYTES + PM::W1PACKED_BYTES};
-    shake_absorb<SHAKE256_RATE>(al, ah, src, CRHBYTES + PM::W1PACKED_BYTES);
-    keccak_f1600(al, ah);
-    const uint2 *c = reinterpret_cast<const uint2 *>(row + LY::VF_SIG);
+    Sp sp;
+    sp.hash(src, CRHBYTES + PM::W1PACKED_BYTES, on);
     bool eq = true;
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-        const uint2 v = c[w];
-        eq &= (v.x == al[w]) && (v.y == ah[w]);
+        const uint2 v = ld_lane(row + LY::VF_SIG + 8 * w);
+        if constexpr (PAIR)
+            eq &= sp.dlo[w] == (sp.half() ? v.y : v.x);
+        else
+            eq &= (v.x == sp.dlo[w]) && (v.y == sp.dhi[w]);
     }
+    if constexpr (PAIR) eq = __shfl_xor_sync(0xFFFFFFFFu, eq, 1) && eq;
+    if (!on) return;
     const int status = reinterpret_cast<const int *>(aux + 64)[0];
     reinterpret_cast<int *>(aux + 68)[0] = (eq && status == 0) ? 0 : -1;
 }
