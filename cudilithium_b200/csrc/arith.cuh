@@ -108,9 +108,22 @@ __host__ __device__ constexpr bool shoup_matches_montgomery() {
 }
 static_assert(shoup_matches_montgomery(), "shoup table");
 
-// f = mont^2 / 256 (the reference's 41978) and its QINV product.
+// f = mont^2 / 256 (the reference's 41978) and its QINV product; f / mont as a true residue (centred) with
+// its quotient, for shoup_mul.
 constexpr int32_t F_INV = 41978;
 constexpr int32_t F_INV_Q = mul_qinv(41978);
+__host__ __device__ constexpr int32_t f_over_mont() {
+    const int64_t mont = (int64_t)((1ull << 32) % Q);
+    for (int64_t w = 0; w < 256; ++w) {  // f / mont = mont / 256
+        if ((mont + w * Q) % 256 == 0) {
+            const int64_t v = (mont + w * Q) / 256 % Q;
+            return (int32_t)(v > (Q - 1) / 2 ? v - Q : v);
+        }
+    }
+    return 0;
+}
+constexpr int32_t F_TRUE = f_over_mont(), F_TRUE_Q = shoup_quot(f_over_mont());
+static_assert(((int64_t)F_TRUE * (int64_t)((1ull << 32) % Q) - F_INV) % Q == 0, "f / mont");
 
 // ------------------------------------------------------------------ montgomery
 

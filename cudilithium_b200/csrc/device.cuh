@@ -129,6 +129,71 @@ __device__ __forceinline__ void pack16_words(uint32_t *out_words, const uint32_t
     for (int i = 0; i < NW; ++i) out_words[i] = w[i];
 }
 
+// Packs the sixteen values below 2^BITS of every position of a 16-thread group -- byte m of b = coefficient
+// t + 16 m -- in coefficient order: position t writes the words of coefficients 16 t .. 16 t + 15.  The
+// 16 x 16 byte transpose is four exchange steps of two shuffles, where the way through shared memory takes
+// 32 accesses.
+template <int BITS>
+__device__ __forceinline__ void pack_strided_bytes(uint32_t *poly_words, uint32_t (&b)[4], int t, unsigned gmask) {
+    static_assert(BITS == 4 || BITS == 6, "w1 fields");
+    {
+        const bool hi = t & 8;
+        const uint32_t r0 = __shfl_xor_sync(gmask, hi ? b[0] : b[2], 8), r1 = __shfl_xor_sync(gmask, hi ? b[1] : b[3], 8);
+        if (hi) {
+            b[0] = r0;
+            b[1] = r1;
+        } else {
+            b[2] = r0;
+            b[3] = r1;
+        }
+    }
+    {
+        const bool hi = t & 4;
+        const uint32_t r0 = __shfl_xor_sync(gmask, hi ? b[0] : b[1], 4), r1 = __shfl_xor_sync(gmask, hi ? b[2] : b[3], 4);
+        if (hi) {
+            b[0] = r0;
+            b[2] = r1;
+        } else {
+            b[1] = r0;
+            b[3] = r1;
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < 4; p += 2) {  // halfwords of a word pair
+        const bool hi = t & 2;
+        const uint32_t r = __shfl_xor_sync(gmask, __byte_perm(b[p], b[p + 1], hi ? 0x5410 : 0x7632), 2);
+        b[p] = hi ? __byte_perm(r, b[p], 0x7610) : __byte_perm(b[p], r, 0x5410);
+        b[p + 1] = hi ? __byte_perm(r, b[p + 1], 0x7632) : __byte_perm(b[p + 1], r, 0x7610);
+    }
+#pragma unroll
+    for (int p = 0; p < 4; p += 2) {  // bytes of a word pair
+        const bool hi = t & 1;
+        const uint32_t r = __shfl_xor_sync(gmask, __byte_perm(b[p], b[p + 1], hi ? 0x6420 : 0x7531), 1);
+        b[p] = __byte_perm(b[p], r, hi ? 0x3514 : 0x5240);
+        b[p + 1] = __byte_perm(b[p + 1], r, hi ? 0x3716 : 0x7260);
+    }
+    uint32_t z[4];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        if constexpr (BITS == 4) {
+            const uint32_t y = (b[w] | (b[w] >> 4)) & 0x00FF00FFu;
+            z[w] = (y | (y >> 8)) & 0xFFFFu;
+        } else {
+            const uint32_t y = (b[w] & 0x003F003Fu) | ((b[w] & 0x3F003F00u) >> 2);
+            z[w] = (y & 0xFFFu) | ((y >> 4) & 0xFFF000u);
+        }
+    }
+    if constexpr (BITS == 4) {
+        uint2 *o = reinterpret_cast<uint2 *>(poly_words) + t;
+        *o = make_uint2(z[0] | z[1] << 16, z[2] | z[3] << 16);
+    } else {
+        uint32_t *o = poly_words + 3 * t;
+        o[0] = z[0] | z[1] << 24;
+        o[1] = (z[1] >> 8) | z[2] << 16;
+        o[2] = (z[2] >> 16) | z[3] << 8;
+    }
+}
+
 // Group helpers: 16 threads, t = position, gmask = lanes of the group.
 struct Group {
     int t;

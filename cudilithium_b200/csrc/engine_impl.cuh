@@ -2,7 +2,7 @@
 // of a whole signing or verification batch, enqueued without waiting for any of them:
 //   sign    rounds of the staged signer (fused_sign_staged.cuh) after k_fused_prehash, then k_fused_sign
 //           for what they left; or k_fused_init, k_fused_prehash and one persistent signer
-//   verify  k_fused_verify_prehash, k_fused_verify
+//   verify  k_fv_challenge, k_fv_w, k_fv_final (fused_verify.cuh)
 // The batch's metadata -- queue block, message offsets and lengths, key indices, longest-first order -- go
 // up in one copy.  Buffers are kernel arguments, so a call with new buffers costs what a repeated one does.
 #pragma once
@@ -18,6 +18,7 @@
 #include "fused_kernels.cuh"
 #include "fused_sign_async.cuh"
 #include "fused_sign_staged.cuh"
+#include "fused_verify.cuh"
 #include "host_impl.cuh"
 #include "profiling.cuh"
 
@@ -49,7 +50,7 @@ struct EngineBase {
     uint8_t *scratch = nullptr;
     size_t scratch_bytes = 0;
     int sign_grid = 0, verify_grid = 0;
-    size_t sign_smem = 0, verify_smem = 0;
+    size_t sign_smem = 0;
     // signer kernel: 0 = phased k_fused_sign (block-wide Keccak / NTT phases) with the engine's
     // block size; 1..4 = asynchronous k_fused_sign_async with (threads, slots) per block of
     // (256, 64), (512, 128), (640, 160), (768, 192); 5 = phased with one wide block per SM (512
@@ -95,10 +96,10 @@ struct EngineImpl : EngineBase {
         return max_keys * (align256(C::SK_ROW) + align256(C::PK_ROW)) + max_items * (C::ITEM_BYTES + 4 * sizeof(unsigned)) +
                stage_bytes(max_items) + 2 * kStagedMaxRounds * sizeof(StagedRound) + scratch_for(max_items);
     }
-    // attempt slots of the largest signer variant, or the verifier's per-signature slots
+    // attempt slots of the largest signer variant, or the packed w1' of a verification batch
     size_t scratch_for(size_t max_items) const {
         if (max_items == 0) return 0;
-        size_t b = std::max((size_t)sign_grid * 2 * threads * C::SLOT, (size_t)verify_grid * threads * C::VSLOT);
+        size_t b = std::max((size_t)sign_grid * 2 * threads * C::SLOT, max_items * VerifyRow<MODE>::W1);
         static constexpr int slots[kAsyncVariants] = {64, 128, 160, 192};
         for (int v = 0; v < kAsyncVariants; ++v) b = std::max(b, (size_t)async_grid[v] * slots[v] * C::SLOT);
         b = std::max(b, (size_t)wide_grid * 2 * kWideThreads * C::SLOT);
@@ -137,12 +138,10 @@ struct EngineImpl : EngineBase {
     template <int T>
     int configure() {
         sign_smem = FusedSignSmem<MODE, T>::BYTES;
-        verify_smem = FusedVerifySmem<MODE, T>::BYTES;
-        if (cudaFuncSetAttribute(k_fused_sign<MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sign_smem) != cudaSuccess ||
-            cudaFuncSetAttribute(k_fused_verify<MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)verify_smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(k_fused_sign<MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sign_smem) != cudaSuccess)
             return ::cudil::cudil_record_cuda_error(cudaGetLastError(), __FILE__, __LINE__);
         sign_grid = grid_for<T>((const void *)k_fused_sign<MODE, T>, sign_smem, sm_count);
-        verify_grid = grid_for<T>((const void *)k_fused_verify<MODE, T>, verify_smem, sm_count);
+        verify_grid = grid_for<kBlock>((const void *)k_fv_w<MODE>, 4 * VerifyRow<MODE>::WARP, sm_count);
         return (sign_grid > 0 && verify_grid > 0) ? CUDIL_OK : cudil_record_cuda_error(cudaErrorInvalidConfiguration, __FILE__, __LINE__);
     }
 
@@ -603,11 +602,11 @@ struct EngineImpl : EngineBase {
         if (rc) return rc;
         mr.msgs = d_msgs;
         cudaEvent_t ev = Profiler::get().before(st);
-        CUDIL_LAUNCH(KID_ST_PREHASH, st, CUDIL_PAIRED_ON(n, sm_count, k_fused_verify_prehash<MODE, PAIR><<<prehash_blocks(n * LANES), kPrehashBlock, 0, st>>>(pk_cache, pk_pitch, mr, items, q)));
-        if (threads == 128)
-            k_fused_verify<MODE, 128><<<verify_grid, 128, verify_smem, st>>>(pk_cache, pk_pitch, mr, d_sig, PM::SIG_BYTES, d_ret, scratch, items, q);
-        else
-            k_fused_verify<MODE, 256><<<verify_grid, 256, verify_smem, st>>>(pk_cache, pk_pitch, mr, d_sig, PM::SIG_BYTES, d_ret, scratch, items, q);
+        VerifyArgs a{pk_cache, pk_pitch, mr, d_sig, (size_t)PM::SIG_BYTES, items, scratch, best, d_ret, (unsigned)n};
+        CUDIL_LAUNCH(KID_FV_CHALLENGE, st, CUDIL_PAIRED_ON(n, sm_count, k_fv_challenge<MODE, PAIR><<<prehash_blocks(n * LANES), kPrehashBlock, 0, st>>>(a)));
+        const unsigned wb = n <= 8u * (size_t)sm_count ? 1u : 4u;  // warps per block
+        CUDIL_LAUNCH(KID_FV_W, st, k_fv_w<MODE><<<blocks_for(n, wb), 32 * wb, wb * VerifyRow<MODE>::WARP, st>>>(a));
+        CUDIL_LAUNCH(KID_FV_FINAL, st, CUDIL_PAIRED_ON(n, sm_count, k_fv_final<MODE, PAIR><<<blocks_for(n * LANES, kPrehashBlock), kPrehashBlock, 0, st>>>(a)));
         CUDIL_CK_LAUNCH();
         Profiler::get().after(KID_FUSED_VERIFY, ev, st);
         CUDIL_CK(cudaMemcpyAsync(h_status, q, sizeof(FusedQueue), cudaMemcpyDeviceToHost, st));

@@ -18,7 +18,8 @@
 //                     minimum -- the same smallest-accepted-nonce result as deterministic signing
 //                     (src/api.cu:388-411).  k_fused_sign_async (fused_sign_async.cuh) runs the same
 //                     queue without block-wide phases.
-//  * k_fused_verify   persistent verification against public rows (no ExpandA / H(pk) per signature).
+//
+// The staged signer (fused_sign_staged.cuh) and the verifier (fused_verify.cuh) work on the same caches.
 #pragma once
 
 #include "keypair_kernels.cuh"
@@ -54,12 +55,6 @@ struct Cache {
     // w1 as bytes, thread-major (byte 16 t + m = coefficient t + 16 m), for the hint computation
     static constexpr size_t SL_W1B = SL_SIG + align256(PM::SIG_BYTES);
     static constexpr size_t SLOT = SL_W1B + (size_t)K * 256;
-    // per-signature slot of the persistent verifier: mu | w1' | c masks | status
-    static constexpr size_t VS_MU = 0;
-    static constexpr size_t VS_W1 = 64;
-    static constexpr size_t VS_CM = align256(64 + PM::W1PACKED_BYTES);
-    static constexpr size_t VS_STATUS = VS_CM + 64;
-    static constexpr size_t VSLOT = VS_CM + 256;
 };
 
 // Queue / status block shared by the engine kernels (one per engine, device memory).
@@ -880,209 +875,6 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
         atomicAdd(&q->cyc[2], (unsigned long long)t_ntt);
         atomicAdd(&q->cyc[3], (unsigned long long)(clock64() - t_start));
         atomicAdd(&q->iters, iters);
-    }
-}
-
-// ------------------------------------------------------------------ persistent verifier
-
-// mu = H(tr || m) of every signature of a verification batch, ahead of the persistent verifier
-// (as k_fused_prehash for signing): one thread per message, longest first, one warp per block, the
-// absorb with the next block's lanes in flight.  A long message therefore costs its own
-// permutations on one thread instead of stalling a verifier block's first phase.
-template <int MODE, bool PAIR>
-__global__ void __launch_bounds__(kPrehashBlock) k_fused_verify_prehash(const uint8_t *cache, size_t cpitch, MsgRefs mr,
-                                                                        uint8_t *items, const FusedQueue *q) {
-    using C = Cache<MODE>;
-    using Sp = Shake256<PAIR>;
-    constexpr unsigned PER = kPrehashBlock / Sp::LANES;
-    const unsigned n = q->n;
-    for (unsigned r0 = blockIdx.x * PER; r0 < n; r0 += gridDim.x * PER) {
-        const unsigned r = r0 + threadIdx.x / Sp::LANES;
-        bool on = r < n;
-        const unsigned it = on ? (mr.order ? mr.order[r] : r) : 0u;
-        on = on && bc_ok(it < n && mr.key_idx[it] < mr.nkeys, BC_PREHASH_ITEM);
-        if (!PAIR && !on) continue;
-        const uint8_t *row = cache + (on ? (size_t)mr.key_idx[it] * cpitch : 0);
-        const long long ml = on ? (long long)mr.mlens[it] : 0;
-        TwoPart src{row + C::PK_TR, 4, mr.msgs + (on ? mr.offsets[it] : 0), ml};
-        Sp sp;
-        sp.hash(src, SEEDBYTES + ml, on);
-        if (on) sp.template store<8>(items + (size_t)it * C::ITEM_BYTES);
-    }
-}
-
-template <int MODE, int THREADS>
-struct FusedVerifySmem {
-    using PM = P<MODE>;
-    static constexpr int G = THREADS / 16;
-    static constexpr size_t PH_W = (size_t)G * ((PM::L + 1) * N * 4 + NTT_SMEM_WORDS * 4 + 32);
-    static constexpr size_t PH_C = (size_t)THREADS * SIB_WORDS * 4;
-    static constexpr size_t BYTES = 256 + (PH_W > PH_C ? PH_W : PH_C);
-};
-
-template <int MODE, int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_verify(const uint8_t *cache, size_t cpitch, MsgRefs mr,
-                                                          const uint8_t *sig, size_t sig_pitch, int *ret,
-                                                          uint8_t *scratch, const uint8_t *items, FusedQueue *q) {
-    using PM = P<MODE>;
-    using C = Cache<MODE>;
-    constexpr int K = PM::K, L = PM::L, OMEGA = PM::OMEGA, A = THREADS, G = THREADS / 16;
-    extern __shared__ __align__(16) uint8_t fv_smem[];
-    unsigned *s_ctl = reinterpret_cast<unsigned *>(fv_smem);
-    uint8_t *ph = fv_smem + 256;
-    const int tid = threadIdx.x, gi = tid >> 4, lane = tid & 31;
-    const unsigned n = q->n;
-    uint8_t *my_slots = scratch + (size_t)blockIdx.x * A * C::VSLOT;
-    // chunks of at most A signatures, small enough that every block of the grid gets work
-    unsigned chunk = (n + gridDim.x - 1) / gridDim.x;
-    chunk = chunk < 1u ? 1u : (chunk > (unsigned)A ? (unsigned)A : chunk);
-    for (;;) {
-        if (tid == 0) s_ctl[0] = (unsigned)atomicAdd(&q->next_ticket, (unsigned long long)chunk);
-        __syncthreads();
-        const unsigned base = s_ctl[0];
-        if (base >= n) break;
-        const int na = (int)((n - base) < chunk ? (n - base) : chunk);
-
-        // hint encoding checks, mu (from the prehash kernel), c = SampleInBall(c~): thread per signature
-        if (tid < na) {
-            const unsigned it = base + tid;
-            const uint8_t *s = sig + (size_t)it * sig_pitch;
-            uint8_t *slot = my_slots + (size_t)tid * C::VSLOT;
-            int status = bc_ok(mr.key_idx[it] < mr.nkeys, BC_VERIFY_KEY) ? 0 : 4;
-            const uint8_t *h = s + PM::SIG_H;
-            int k = 0;
-            for (int i = 0; i < K && !status; ++i) {
-                const int end = h[OMEGA + i];
-                if (end < k || end > OMEGA) {
-                    status = 1;
-                    break;
-                }
-                for (int j = k + 1; j < end; ++j)
-                    if (h[j] <= h[j - 1]) status = 1;
-                k = end;
-            }
-            if (!status)
-                for (int j = k; j < OMEGA; ++j)
-                    if (h[j]) status = 1;
-            uint2 mu8[8];
-            ld_lanes(mu8, items + (size_t)it * C::ITEM_BYTES);
-            uint2 *mu = reinterpret_cast<uint2 *>(slot + C::VS_MU);
-#pragma unroll
-            for (int w = 0; w < 8; ++w) mu[w] = mu8[w];
-            uint2 ct[4];
-#pragma unroll
-            for (int w = 0; w < 4; ++w) ct[w] = make_uint2(load_lane_bytes(s + 8 * w, 8).x, load_lane_bytes(s + 8 * w, 8).y);
-            uint32_t *sib = reinterpret_cast<uint32_t *>(ph);
-            const uint32_t *mask = sib_result<THREADS>(sib, tid);
-            sample_in_ball<PM::TAU, THREADS>(ct, sib, tid);
-            uint4 *mo = reinterpret_cast<uint4 *>(slot + C::VS_CM);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-                mo[kk] = make_uint4(mask[(4 * kk) * THREADS], mask[(4 * kk + 1) * THREADS], mask[(4 * kk + 2) * THREADS],
-                                    mask[(4 * kk + 3) * THREADS]);
-            reinterpret_cast<int *>(slot + C::VS_STATUS)[0] = status;
-        }
-        __syncthreads();
-
-        // z norm check + NTT(z), NTT(c), w' = A_hat z_hat - c_hat t1_hat, UseHint, pack: group per signature
-        {
-            int32_t *zh = reinterpret_cast<int32_t *>(ph) + (size_t)gi * ((L + 1) * N + NTT_SMEM_WORDS + 8);
-            uint32_t *hbits = reinterpret_cast<uint32_t *>(zh + (L + 1) * N + NTT_SMEM_WORDS);
-            Group g;
-            g.t = tid & 15;
-            g.gmask = 0xFFFFu << (lane & 16);
-            g.sm = zh + (L + 1) * N;
-            for (int a = gi; a < na; a += G) {
-                const unsigned it = base + a;
-                const uint8_t *s = sig + (size_t)it * sig_pitch;
-                const unsigned key = mr.key_idx[it];
-                const uint8_t *row = cache + (size_t)(bc_ok(key < mr.nkeys, BC_VERIFY_KEY) ? key : 0u) * cpitch;
-                uint8_t *slot = my_slots + (size_t)a * C::VSLOT;
-                bool zbad = false;
-#pragma unroll 1
-                for (int j = 0; j < L; ++j) {
-                    int32_t x[16];
-                    unpack_z_strided<MODE>(x, s + PM::SIG_Z + (size_t)j * PM::POLYZ_PACKED, g.t);
-#pragma unroll
-                    for (int m = 0; m < 16; ++m) zbad |= exceeds(x[m], PM::GAMMA1 - PM::BETA);
-                    ntt16s(x, g.sm, g.gmask, g.t);
-                    store16_smem(zh + j * N, x, g.t);
-                }
-                if (group_any(g, zbad) && g.t == 0) reinterpret_cast<int *>(slot + C::VS_STATUS)[0] |= 2;
-                {
-                    uint32_t masks[16];
-                    const uint4 *mi = reinterpret_cast<const uint4 *>(slot + C::VS_CM);
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint4 v = mi[kk];
-                        masks[4 * kk] = v.x;
-                        masks[4 * kk + 1] = v.y;
-                        masks[4 * kk + 2] = v.z;
-                        masks[4 * kk + 3] = v.w;
-                    }
-                    int32_t x[16];
-                    challenge_strided(x, masks, g.t);
-                    ntt16s(x, g.sm, g.gmask, g.t);
-                    // -c_hat with the inverse transform's factor (A_hat carries it already)
-#pragma unroll
-                    for (int m = 0; m < 16; ++m) x[m] = -scale_f(x[m]);
-                    store16_smem(zh + L * N, x, g.t);
-                }
-                __syncwarp(g.gmask);
-                const uint8_t *h = s + PM::SIG_H;
-#pragma unroll 1
-                for (int i = 0; i < K; ++i) {
-                    if (g.t < 8) hbits[g.t] = 0;
-                    __syncwarp(g.gmask);
-                    const int start = (i == 0) ? 0 : h[OMEGA + i - 1];
-                    int end = h[OMEGA + i];
-                    if (end > OMEGA) end = OMEGA;
-                    for (int j = start + g.t; j < end; j += 16) atomicOr(&hbits[h[j] >> 5], 1u << (h[j] & 31));
-                    __syncwarp(g.gmask);
-                    const int32_t *mat = reinterpret_cast<const int32_t *>(row + C::PK_MAT) + (size_t)i * L * N;
-                    // sum_j A_ij z_j - c t1_i: t1_i is operand L, whose shared-memory vector is -c_hat
-                    const int32_t *t1 = reinterpret_cast<const int32_t *>(row + C::PK_T1) + (size_t)i * N;
-                    int32_t acc[16];
-                    dot16<L + 1, (L + 2) / 2>(acc, zh, g.t, [&](int j) { return j < L ? mat + (size_t)j * N : t1; });
-                    intt16s(acc, g.sm, g.gmask, g.t);
-                    int32_t w1[16];
-#pragma unroll
-                    for (int m = 0; m < 16; ++m) {
-                        const int c = g.t + 16 * m;
-                        w1[m] = use_hint<MODE>(caddq(reduce32(acc[m])), (hbits[c >> 5] >> (c & 31)) & 1u);
-                    }
-                    int32_t w1c[16];
-                    strided_to_contig(g, w1, w1c);
-                    uint32_t v[16];
-#pragma unroll
-                    for (int m = 0; m < 16; ++m) v[m] = (uint32_t)w1c[m];
-                    pack16_words<PM::W1_BITS>(
-                        reinterpret_cast<uint32_t *>(slot + C::VS_W1 + (size_t)i * PM::POLYW1_PACKED + g.t * 2 * PM::W1_BITS), v);
-                    __syncwarp(g.gmask);
-                }
-            }
-        }
-        __syncthreads();
-
-        // c~' = H(mu || w1') and compare: thread per signature
-        if (tid < na) {
-            const unsigned it = base + tid;
-            const uint8_t *s = sig + (size_t)it * sig_pitch;
-            uint8_t *slot = my_slots + (size_t)tid * C::VSLOT;
-            uint32_t al[25], ah[25];
-            AlignedBytes src{slot + C::VS_MU, CRHBYTES + PM::W1PACKED_BYTES};
-            shake_absorb<SHAKE256_RATE>(al, ah, src, CRHBYTES + PM::W1PACKED_BYTES);
-            keccak_f1600(al, ah);
-            bool eq = true;
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                const uint2 v = load_lane_bytes(s + 8 * w, 8);
-                eq &= (v.x == al[w]) && (v.y == ah[w]);
-            }
-            const int status = reinterpret_cast<const int *>(slot + C::VS_STATUS)[0];
-            ret[it] = (eq && status == 0) ? 0 : -1;
-        }
-        __syncthreads();
     }
 }
 

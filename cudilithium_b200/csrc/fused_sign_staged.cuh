@@ -221,25 +221,18 @@ __global__ void __launch_bounds__(kBlock, 6) k_st_w(StagedArgs a, int r) {
             int32_t acc[16];
             dot16<L, (L + 1) / 2>(acc, yh, g.t, [&](int j) { return mat + ((size_t)i * L + j) * N; });
             intt16s(acc, g.sm, g.gmask, g.t);
-            int32_t w1[16];
             int4 *w0 = reinterpret_cast<int4 *>(slot + S::W0 + (size_t)i * S::POLY);
             uint32_t b[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                int32_t a0[4];
+                int32_t a0[4], w1[4];
 #pragma unroll
-                for (int m = 0; m < 4; ++m) w1[4 * c + m] = decompose<MODE>(a0[m], caddq(reduce32(acc[4 * c + m])));
+                for (int m = 0; m < 4; ++m) w1[m] = decompose<MODE>(a0[m], caddq(reduce32(acc[4 * c + m])));
                 w0[16 * c + g.t] = make_int4(a0[0], a0[1], a0[2], a0[3]);
-                b[c] = (uint32_t)w1[4 * c] | (uint32_t)w1[4 * c + 1] << 8 | (uint32_t)w1[4 * c + 2] << 16 | (uint32_t)w1[4 * c + 3] << 24;
+                b[c] = (uint32_t)w1[0] | (uint32_t)w1[1] << 8 | (uint32_t)w1[2] << 16 | (uint32_t)w1[3] << 24;
             }
             *reinterpret_cast<uint4 *>(slot + S::W1B + (size_t)i * 256 + 16 * g.t) = make_uint4(b[0], b[1], b[2], b[3]);
-            int32_t w1c[16];
-            strided_to_contig(g, w1, w1c);
-            uint32_t v[16];
-#pragma unroll
-            for (int m = 0; m < 16; ++m) v[m] = (uint32_t)w1c[m];
-            pack16_words<PM::W1_BITS>(
-                reinterpret_cast<uint32_t *>(slot + S::W1P + (size_t)i * PM::POLYW1_PACKED + g.t * 2 * PM::W1_BITS), v);
+            pack_strided_bytes<PM::W1_BITS>(reinterpret_cast<uint32_t *>(slot + S::W1P + (size_t)i * PM::POLYW1_PACKED), b, g.t, g.gmask);
         }
     }
 }

@@ -235,7 +235,7 @@ __device__ __forceinline__ void intt16s(int32_t (&x)[16], int32_t *sm, unsigned 
 // The inverse transform's factor f, put into one operand of the products it will transform -- A_hat
 // when it is sampled, c_hat once per challenge -- instead of into all 256 outputs of every inverse
 // transform (16 multiplications of a thread's ~90 per transform).
-__device__ __forceinline__ int32_t scale_f(int32_t a) { return montmul_pre(a, F_INV, F_INV_Q); }
+__device__ __forceinline__ int32_t scale_f(int32_t a) { return shoup_mul(a, F_TRUE, F_TRUE_Q); }
 
 // Out-of-line forms of the two transforms for large kernels that call them from many places: one
 // copy of each transform instead of one per call site keeps the instruction working set small.
@@ -337,7 +337,7 @@ __device__ __forceinline__ void load16_smem(int32_t (&x)[16], const int32_t *pol
 
 // out[i] = sum_j op(j)[16 t + i] * y_j[16 t + i] mod q (Montgomery-reduced once) over NOPS operand
 // polynomials op(j) in global memory (load16_chunks layout) and vectors y_j in shared memory (store16_smem layout, y_j =
-// yh + j N).  The products accumulate in 64 bits: |sum| < NOPS * q * 2^27 < 2^53, so |out| < 0.67 q.
+// yh + j N).  The products accumulate in 64 bits: |sum| < NOPS * 1.5 q * 2^27 < 2^54, so |out| < 0.8 q.
 // Eight coefficients at a time, CH operands' loads in flight before the first is consumed.
 template <int NOPS, int CH, typename Op>
 __device__ __forceinline__ void dot16(int32_t (&out)[16], const int32_t *yh, int t, Op op) {

@@ -45,6 +45,9 @@ enum KernelId : int {
     KID_ST_W,
     KID_ST_CHALLENGE,
     KID_ST_REJECT,
+    KID_FV_CHALLENGE,
+    KID_FV_W,
+    KID_FV_FINAL,
     KID_COUNT
 };
 
@@ -55,7 +58,8 @@ inline const char *kernel_name(int id) {
         "k_verify_prepare", "k_verify_w", "k_verify_final", "k_ntt_mul", "k_alu_peak",
         "k_fused_sign (graph)", "k_fused_verify (graph)", "k_fused_sched", "k_cache_sk", "k_cache_pk",
         "k_sig_check", "k_sk_check", "k_derive_rhoprime",
-        "k_fused_prehash", "k_st_claim", "k_st_mask", "k_st_w", "k_st_challenge", "k_st_reject"};
+        "k_fused_prehash", "k_st_claim", "k_st_mask", "k_st_w", "k_st_challenge", "k_st_reject",
+        "k_fv_challenge", "k_fv_w", "k_fv_final"};
     return (id >= 0 && id < KID_COUNT) ? names[id] : "?";
 }
 
