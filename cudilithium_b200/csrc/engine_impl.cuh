@@ -49,7 +49,7 @@ struct EngineBase {
     bool stage_pending = false;
     uint8_t *scratch = nullptr;
     size_t scratch_bytes = 0;
-    int sign_grid = 0, verify_grid = 0;
+    int sign_grid = 0, verify_grid = 0, reject_grid = 0;
     size_t sign_smem = 0;
     // signer kernel: 0 = phased k_fused_sign (block-wide Keccak / NTT phases) with the engine's
     // block size; 1..4 = asynchronous k_fused_sign_async with (threads, slots) per block of
@@ -141,8 +141,9 @@ struct EngineImpl : EngineBase {
         if (cudaFuncSetAttribute(k_fused_sign<MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sign_smem) != cudaSuccess)
             return ::cudil::cudil_record_cuda_error(cudaGetLastError(), __FILE__, __LINE__);
         sign_grid = grid_for<T>((const void *)k_fused_sign<MODE, T>, sign_smem, sm_count);
+        reject_grid = grid_for<32>((const void *)k_st_reject<MODE>, 0, sm_count);
         verify_grid = grid_for<kBlock>((const void *)k_fv_w<MODE>, 4 * VerifyRow<MODE>::WARP, sm_count);
-        return (sign_grid > 0 && verify_grid > 0) ? CUDIL_OK : cudil_record_cuda_error(cudaErrorInvalidConfiguration, __FILE__, __LINE__);
+        return (sign_grid > 0 && verify_grid > 0 && reject_grid > 0) ? CUDIL_OK : cudil_record_cuda_error(cudaErrorInvalidConfiguration, __FILE__, __LINE__);
     }
 
     int create(size_t mk, size_t mi, int thr, size_t budget) {
@@ -376,7 +377,6 @@ struct EngineImpl : EngineBase {
         // enough blocks for a pending count four standard deviations above the expected one (kernels
         // stride over what exceeds it)
         const double hi = std::min((double)a.count, t.p + 4.0 * std::sqrt(t.p) + 4.0);
-        const double depth = std::min((double)kStagedMaxDepth, std::max(1.0, std::floor(a.target / std::max(t.p, 1.0))));
         const unsigned slots = (unsigned)std::min((double)a.cap, std::max(hi, std::min((double)a.target, hi * kStagedMaxDepth)));
         if (stage == 0) {
             const unsigned cb = std::max(blocks_for((size_t)hi + 1, 256), std::min(blocks_for(t.prev_slots, 8), 8u * sms));
@@ -390,10 +390,13 @@ struct EngineImpl : EngineBase {
             CUDIL_LAUNCH(KID_ST_CHALLENGE, st,
                          CUDIL_PAIRED_ON(slots, sm_count, k_st_challenge<MODE, PAIR><<<blocks_for((size_t)slots * LANES, kItemBlock), kItemBlock, 0, st>>>(a, t.r)));
         } else {
-            const unsigned per = slots <= 16u * sms ? 1u : 2u;  // attempts per warp
-            CUDIL_LAUNCH(KID_ST_REJECT, st, k_st_reject<MODE><<<blocks_for(slots, per), 32, S::WARP_R, st>>>(a, t.r, per));
+            const unsigned per = slots <= (unsigned)reject_grid ? 1u : 2u;  // attempts per warp
+            CUDIL_LAUNCH(KID_ST_REJECT, st, k_st_reject<MODE><<<blocks_for(slots, per), 32, 0, st>>>(a, t.r, per));
             t.prev_slots = slots;
-            t.p *= std::pow(1.0 - kAccept, depth);
+            if (t.p >= a.target)
+                t.p -= kAccept * (t.p > a.quantum && t.p < 4.0 * a.quantum ? std::floor(t.p / a.quantum) * a.quantum : std::min(t.p, (double)a.cap));
+            else
+                t.p *= std::pow(1.0 - kAccept, std::min((double)kStagedMaxDepth, a.target / std::max(t.p, 1.0)));
             ++t.r;
         }
     }
@@ -466,7 +469,10 @@ struct EngineImpl : EngineBase {
             a.locks = locks;
             a.next_nonce = next_nonce;
             a.inflight = inflight;
+            // two layers of 32 streams on every sub-partition
+            a.quantum = (unsigned)(sm_count * 4 * 32 * 2 / L);
             a.target = (unsigned)std::min<size_t>(std::max(1u, target / parts), cap);
+            if (a.target > a.quantum) a.target = a.target / a.quantum * a.quantum;
             a.nonce_limit = nonce_limit;
             a.nkeys = (unsigned)max_keys;
             part[k].st = k ? side : st;
