@@ -243,6 +243,23 @@ __device__ __forceinline__ void unpack_strided(uint32_t (&v)[16], const uint8_t 
         v[i] = __funnelshift_r(w[(BITS / 2) * i], w[(BITS / 2) * i + second], sh) & ((1u << BITS) - 1u);
 }
 
+// The same for BITS odd and a word-aligned array: sixteen fields are BITS / 2 words and a half, so the even
+// i share one word and shift and the odd i another.
+template <int BITS>
+__device__ __forceinline__ void unpack_strided_odd(uint32_t (&v)[16], const uint8_t *packed, int t) {
+    static_assert(BITS % 2 == 1 && BITS <= 17, "a word and a half every sixteen fields");
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(packed);
+#pragma unroll
+    for (int odd = 0; odd < 2; ++odd) {
+        const unsigned bit = (unsigned)(BITS * (t + 16 * odd)), sh = bit & 31u;
+        const uint32_t *p = w + (bit >> 5);
+        const int second = sh + BITS > 32u ? 1 : 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            v[2 * i + odd] = __funnelshift_r(p[BITS * i], p[BITS * i + second], sh) & ((1u << BITS) - 1u);
+    }
+}
+
 // z coefficients a[t + 16 i] from a packed (gamma1 - z) polynomial.
 template <int MODE>
 __device__ __forceinline__ void unpack_z_strided(int32_t (&x)[16], const uint8_t *packed, int t) {

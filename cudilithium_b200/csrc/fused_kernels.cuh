@@ -105,24 +105,9 @@ __global__ void __launch_bounds__(kBlock) k_cache_sk(const uint8_t *sk, uint8_t 
         return;
     }
     int32_t x[16];
-    size_t dst;
-    if (p < L + K) {
-        const uint8_t *src = s + PM::SK_S1 + (size_t)p * PM::POLYETA_PACKED;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = PM::ETA - (int32_t)get_bits(src, (g.t + 16 * i) * PM::ETA_BITS, PM::ETA_BITS);
-        dst = (p < L) ? C::SK_S1 + (size_t)p * C::POLY : C::SK_S2 + (size_t)(p - L) * C::POLY;
-    } else {
-        const uint8_t *src = s + PM::SK_T0 + (size_t)(p - L - K) * POLYT0_PACKED;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            // last coefficient of the last t0 poly ends exactly at SK_BYTES: read 2 bytes only
-            const int bit = (g.t + 16 * i) * 13, byte = bit >> 3, sh = bit & 7;
-            const uint32_t v = ((uint32_t)src[byte] | ((uint32_t)src[byte + 1] << 8) |
-                                (sh + 13 > 16 ? (uint32_t)src[byte + 2] << 16 : 0u)) >> sh;
-            x[i] = (1 << (D - 1)) - (int32_t)(v & 0x1FFFu);
-        }
-        dst = C::SK_T0 + (size_t)(p - L - K) * C::POLY;
-    }
+    unpack_secret<MODE>(x, s, p, g.t);
+    const size_t dst = p < L ? C::SK_S1 + (size_t)p * C::POLY
+                             : (p < L + K ? C::SK_S2 + (size_t)(p - L) * C::POLY : C::SK_T0 + (size_t)(p - L - K) * C::POLY);
     ntt16s(x, g.sm, g.gmask, g.t);
     store16_chunks(reinterpret_cast<int32_t *>(row + dst), x, g.t);
 }

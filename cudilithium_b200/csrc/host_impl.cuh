@@ -95,6 +95,11 @@ struct Impl {
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_KP_TR, st, CUDIL_PAIRED(n, k_kp_tr<MODE, PAIR><<<blocks_for(n * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, nn)));
         CUDIL_CK_LAUNCH();
+        if (out_kind == cudaMemcpyDeviceToDevice && (((uintptr_t)pk | (uintptr_t)sk) & 3u) == 0u) {
+            CUDIL_LAUNCH(KID_KP_OUT, st, k_kp_out<MODE><<<(unsigned)n, kBlock, 0, st>>>(pool, pitch, pk, sk));
+            CUDIL_CK_LAUNCH();
+            return CUDIL_OK;
+        }
         CUDIL_CK(cudaMemcpy2DAsync(pk, PM::PK_BYTES, pool + LY::KP_PK, pitch, PM::PK_BYTES, n, out_kind, st));
         CUDIL_CK(cudaMemcpy2DAsync(sk, PM::SK_BYTES, pool + LY::KP_SK, pitch, PM::SK_BYTES, n, out_kind, st));
         return CUDIL_OK;
@@ -110,9 +115,10 @@ struct Impl {
         if (mlen) CUDIL_CK(cudaMemcpy2DAsync(pool + LY::SG_MSG, sp, m, m_pitch, mlen, n, in_kind, st));
         CUDIL_CK(cudaMemcpy2DAsync(pool + LY::SG_SK, sp, sk, sk_pitch, PM::SK_BYTES, n, in_kind, st));
         if (rhop) CUDIL_CK(cudaMemcpy2DAsync(pool + LY::SG_RHOP, sp, rhop, rhop_pitch, CRHBYTES, n, in_kind, st));
-        CUDIL_LAUNCH(KID_SIGN_PREHASH, st, CUDIL_PAIRED(n, k_sign_prehash<MODE, PAIR><<<blocks_for(n * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, sp, mlen, mlens, nn, rhop ? 1 : 0)));
-        CUDIL_CK_LAUNCH();
-        CUDIL_LAUNCH(KID_EXPAND_A, st, k_expand_a<MODE><<<blocks_for(n * K * L), kBlock, 0, st>>>(pool, sp, LY::SG_SK + PM::SK_RHO, LY::sg_mat(mlen), nn));
+        CUDIL_LAUNCH(KID_SIGN_PREHASH, st, CUDIL_PAIRED(n, {
+            const unsigned hb = blocks_for(n * LANES, kItemBlock);
+            k_sign_setup<MODE, PAIR><<<hb + blocks_for(n * K * L, kItemBlock), kItemBlock, 0, st>>>(pool, sp, mlen, mlens, nn, rhop ? 1 : 0, hb);
+        }));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_SIGN_UNPACK_NTT, st, k_sign_unpack_ntt<MODE><<<blocks_for(n * (L + 2 * K) * 16), kBlock, 0, st>>>(pool, sp, mlen, nn));
         CUDIL_CK_LAUNCH();
@@ -228,9 +234,10 @@ struct Impl {
         CUDIL_CK(cudaMemcpy2DAsync(pool + LY::VF_SIG, pitch, sig, sig_pitch, PM::SIG_BYTES, n, in_kind, st));
         if (mlen) CUDIL_CK(cudaMemcpy2DAsync(pool + LY::VF_TRM + SEEDBYTES, pitch, m, m_pitch, mlen, n, in_kind, st));
         CUDIL_CK(cudaMemcpy2DAsync(pool + LY::VF_PK, pitch, pk, pk_pitch, PM::PK_BYTES, n, in_kind, st));
-        CUDIL_LAUNCH(KID_VERIFY_PREPARE, st, CUDIL_PAIRED(n, k_verify_prepare<MODE, PAIR><<<blocks_for(n * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, mlen, mlens, nn)));
-        CUDIL_CK_LAUNCH();
-        CUDIL_LAUNCH(KID_EXPAND_A, st, k_expand_a<MODE><<<blocks_for(n * K * L), kBlock, 0, st>>>(pool, pitch, LY::VF_PK, LY::vf_mat(mlen), nn));
+        CUDIL_LAUNCH(KID_VERIFY_PREPARE, st, CUDIL_PAIRED(n, {
+            const unsigned hb = blocks_for(n * LANES, kItemBlock);
+            k_verify_setup<MODE, PAIR><<<hb + blocks_for(n * K * L, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, mlen, mlens, nn, hb);
+        }));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_VERIFY_W, st, k_verify_w<MODE, AV><<<(unsigned)((n + AV - 1) / AV), kBlock, 0, st>>>(pool, pitch, mlen, nn));
         CUDIL_CK_LAUNCH();

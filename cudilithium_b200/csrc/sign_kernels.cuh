@@ -2,8 +2,8 @@
 // that stage needs: SHAKE streams one per thread, polynomial arithmetic one per 16-thread group.
 //
 // Stage list (reference kernel each one replaces):
-//   k_sign_prehash     mu = H(tr||m), rho' = H(K||mu)     notmp_shake_new_kernel, src/api.cu:137-152
-//   k_expand_a         A_hat = ExpandA(rho)               polyvec_matrix_expand_opt_kernel, src/sign.cu:98-163
+//   k_sign_setup       mu = H(tr||m), rho' = H(K||mu)     notmp_shake_new_kernel, src/api.cu:137-152
+//     (its other blocks) A_hat = ExpandA(rho)               polyvec_matrix_expand_opt_kernel, src/sign.cu:98-163
 //   k_sign_unpack_ntt  s1_hat, s2_hat, t0_hat             unpack_fuse_ntt_radix2_opt_kernel, src/sign.cu:306-403
 //   k_sign_expand_mask y = ExpandMask(rho', L*nonce + j)  compute_y_opt_kernel, src/sign.cu:463-526
 //   k_sign_compute_w   w = invNTT(A_hat NTT(y)); w0, w1   compute_w_128t_kernel, src/sign.cu:605-685
@@ -51,11 +51,11 @@ inline bool keccak_pairs(size_t items, int sm_count) { return items <= (size_t)s
 
 // rhop_given: rho' was placed in the row by the caller (randomized signing), only mu is computed.
 template <int MODE, bool PAIR>
-__global__ void __launch_bounds__(kBlock) k_sign_prehash(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens,
-                                                         int n, int rhop_given) {
+__device__ __forceinline__ void sign_prehash(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens, int n, int rhop_given,
+                                             int block) {
     using LY = Layout<MODE>;
     using Sp = Shake256<PAIR>;
-    const int it = (blockIdx.x * blockDim.x + threadIdx.x) / Sp::LANES;
+    const int it = (block * (int)blockDim.x + (int)threadIdx.x) / Sp::LANES;
     const bool on = it < n;
     if (!PAIR && !on) return;
     uint8_t *row = pool + (size_t)(on ? it : 0) * pitch;
@@ -71,9 +71,9 @@ __global__ void __launch_bounds__(kBlock) k_sign_prehash(uint8_t *pool, size_t p
 
 // One thread per ExpandA entry; rho at row+rho_off, A_hat (K*L polys) at row+mat_off.
 template <int MODE>
-__global__ void __launch_bounds__(kBlock) k_expand_a(uint8_t *pool, size_t pitch, size_t rho_off, size_t mat_off, int n) {
+__device__ __forceinline__ void expand_a_entry(uint8_t *pool, size_t pitch, size_t rho_off, size_t mat_off, int n, int block) {
     constexpr int K = Params<MODE>::K, L = Params<MODE>::L, KL = K * L;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = block * (int)blockDim.x + (int)threadIdx.x;
     if (s >= n * KL) return;
     const int it = s / KL, ij = s % KL;
     uint8_t *row = pool + (size_t)it * pitch;
@@ -81,6 +81,19 @@ __global__ void __launch_bounds__(kBlock) k_expand_a(uint8_t *pool, size_t pitch
     ld_lanes(rho, row + rho_off);
     int32_t *out = reinterpret_cast<int32_t *>(row + mat_off) + (size_t)ij * N;
     expand_a_row(rho, ij / L, ij % L, out);
+}
+
+// Blocks [0, hash_blocks) hash the messages, the others run ExpandA: neither needs the other, and the hash
+// chains of a small batch would leave most of the GPU idle in a launch of their own.  (1024 Dilithium3 items:
+// prehash and ExpandA 21 + 73 us apart; verification's prepare and ExpandA 96 + 73 us.)
+template <int MODE, bool PAIR>
+__global__ void __launch_bounds__(kItemBlock) k_sign_setup(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens, int n,
+                                                           int rhop_given, unsigned hash_blocks) {
+    using LY = Layout<MODE>;
+    if (blockIdx.x < hash_blocks)
+        sign_prehash<MODE, PAIR>(pool, pitch, mlen, mlens, n, rhop_given, (int)blockIdx.x);
+    else
+        expand_a_entry<MODE>(pool, pitch, LY::SG_SK + P<MODE>::SK_RHO, LY::sg_mat(mlen), n, (int)(blockIdx.x - hash_blocks));
 }
 
 // The same with rho read from the packed keys (key i at keys + i * key_bytes, rho = its first 32
@@ -104,6 +117,39 @@ __global__ void __launch_bounds__(kBlock) k_expand_a_keys(const uint8_t *keys, s
     expand_a_row(rho, ij / L, ij % L, out);
 }
 
+// Coefficients a[t + 16 i] of secret polynomial p of a packed key: s1 (p < L), s2 (p < L + K), then t0.
+template <int MODE>
+__device__ __forceinline__ void unpack_secret(int32_t (&x)[16], const uint8_t *sk, int p, int t) {
+    using PM = P<MODE>;
+    constexpr int K = PM::K, L = PM::L;
+    const bool eta = p < L + K;
+    const uint8_t *src = sk + (eta ? PM::SK_S1 + (size_t)p * PM::POLYETA_PACKED : PM::SK_T0 + (size_t)(p - L - K) * POLYT0_PACKED);
+    const int32_t top = eta ? PM::ETA : 1 << (D - 1);
+    uint32_t v[16];
+    if ((reinterpret_cast<uintptr_t>(sk) & 3u) == 0u) {
+        if (!eta) {
+            unpack_strided_odd<13>(v, src, t);
+        } else if constexpr (PM::ETA_BITS == 3) {
+            unpack_strided_odd<3>(v, src, t);
+        } else {
+            unpack_strided<4>(v, src, t);
+        }
+    } else {
+        // packed keys at any byte: three byte loads, two where the field ends with the key's last byte
+        const int bits = eta ? PM::ETA_BITS : 13;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int bit = (t + 16 * i) * bits, byte = bit >> 3, sh = bit & 7;
+            uint32_t w = src[byte];
+            if (sh + bits > 8) w |= (uint32_t)src[byte + 1] << 8;
+            if (sh + bits > 16) w |= (uint32_t)src[byte + 2] << 16;
+            v[i] = (w >> sh) & ((1u << bits) - 1u);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = top - (int32_t)v[i];
+}
+
 // One 16-thread group per secret polynomial: unpack (eta / 13-bit) and forward NTT.
 template <int MODE>
 __global__ void __launch_bounds__(kBlock) k_sign_unpack_ntt(uint8_t *pool, size_t pitch, size_t mlen, int n) {
@@ -116,20 +162,10 @@ __global__ void __launch_bounds__(kBlock) k_sign_unpack_ntt(uint8_t *pool, size_
     if (it >= n) return;
     Group g = make_group(sm, threadIdx.x >> 4);
     uint8_t *row = pool + (size_t)it * pitch;
-    const uint8_t *sk = row + LY::SG_SK;
     int32_t x[16];
-    size_t dst;
-    if (p < L + K) {
-        const uint8_t *src = sk + PM::SK_S1 + (size_t)p * PM::POLYETA_PACKED;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = PM::ETA - (int32_t)get_bits(src, (g.t + 16 * i) * PM::ETA_BITS, PM::ETA_BITS);
-        dst = (p < L) ? LY::sg_s1(mlen) + (size_t)p * LY::POLY : LY::sg_s2(mlen) + (size_t)(p - L) * LY::POLY;
-    } else {
-        const uint8_t *src = sk + PM::SK_T0 + (size_t)(p - L - K) * POLYT0_PACKED;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = (1 << (D - 1)) - (int32_t)get_bits(src, (g.t + 16 * i) * 13, 13);
-        dst = LY::sg_t0(mlen) + (size_t)(p - L - K) * LY::POLY;
-    }
+    unpack_secret<MODE>(x, row + LY::SG_SK, p, g.t);
+    const size_t dst = p < L ? LY::sg_s1(mlen) + (size_t)p * LY::POLY
+                             : (p < L + K ? LY::sg_s2(mlen) + (size_t)(p - L) * LY::POLY : LY::sg_t0(mlen) + (size_t)(p - L - K) * LY::POLY);
     ntt16s(x, g.sm, g.gmask, g.t);
     store16_chunks(reinterpret_cast<int32_t *>(row + dst), x, g.t);
 }
@@ -490,7 +526,9 @@ __global__ void k_sig_copy(uint8_t *sign_pool, size_t sp, const uint8_t *temp_po
     if (!bc_ok(e.exec_idx < nexec && e.sign_idx < nitems, BC_COPY_ENTRY)) return;
     const uint8_t *src = temp_pool + e.exec_idx * tp + Layout<MODE>::TP_SIG;
     uint8_t *dst = sign_pool + e.sign_idx * sp + Layout<MODE>::SG_SIG;
-    for (int i = threadIdx.x; i < P<MODE>::SIG_BYTES; i += blockDim.x) dst[i] = src[i];
+    // (both start at a multiple of 16 bytes and their areas are whole 256-byte units)
+    for (int i = threadIdx.x; i < (P<MODE>::SIG_BYTES + 15) / 16; i += blockDim.x)
+        reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
 }
 
 }  // namespace cudil

@@ -1,8 +1,8 @@
 // Batched verification kernels (reference: gpu_verify, src/verify.cu:28-325, one warp per
 // signature).  Split by stage shape:
-//   k_verify_prepare  one thread per signature: hint-encoding checks (src/verify.cu:51-93),
+//   k_verify_setup    one thread or pair per signature: hint-encoding checks (src/verify.cu:51-93),
 //                     tr' = H(pk), mu = H(tr'||m), c = SampleInBall(c~)
-//   k_expand_a        one thread per ExpandA entry (shared with signing)
+//                     and, in blocks of its own, one thread per ExpandA entry
 //   k_verify_w        16-thread groups: z norm check + NTT(z), NTT(c), A z - c t1 2^d, invNTT,
 //                     UseHint, pack w1'
 //   k_verify_final    one thread per signature: c~' = H(mu||w1') and compare
@@ -12,15 +12,14 @@
 
 namespace cudil {
 
-template <int MODE, bool PAIR, int TB = kItemBlock>
-__global__ void __launch_bounds__(TB) k_verify_prepare(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens,
-                                                       int n) {
+template <int MODE, bool PAIR, int TB>
+__device__ __forceinline__ void verify_prepare(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens, int n, int block,
+                                               uint32_t *s_sib) {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
     using Sp = Shake256<PAIR>;
     constexpr int K = PM::K, OMEGA = PM::OMEGA;
-    __shared__ uint32_t s_sib[SIB_WORDS * TB];
-    const int it = (blockIdx.x * blockDim.x + threadIdx.x) / Sp::LANES;
+    const int it = (block * TB + (int)threadIdx.x) / Sp::LANES;
     const bool on = it < n;
     if (!PAIR && !on) return;
     uint8_t *row = pool + (size_t)(on ? it : 0) * pitch;
@@ -75,6 +74,18 @@ __global__ void __launch_bounds__(TB) k_verify_prepare(uint8_t *pool, size_t pit
     if (on && (!PAIR || sp.half() == 0)) sib_store<TB>(aux, s_sib, threadIdx.x);
 }
 
+// Blocks [0, prep_blocks) prepare the signatures, the others run ExpandA (as k_sign_setup).
+template <int MODE, bool PAIR>
+__global__ void __launch_bounds__(kItemBlock) k_verify_setup(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens, int n,
+                                                             unsigned prep_blocks) {
+    using LY = Layout<MODE>;
+    __shared__ uint32_t s_sib[SIB_WORDS * kItemBlock];
+    if (blockIdx.x < prep_blocks)
+        verify_prepare<MODE, PAIR, kItemBlock>(pool, pitch, mlen, mlens, n, (int)blockIdx.x, s_sib);
+    else
+        expand_a_entry<MODE>(pool, pitch, LY::VF_PK, LY::vf_mat(mlen), n, (int)(blockIdx.x - prep_blocks));
+}
+
 // AV signatures per 128-thread block.  Phase 1 units: (sig, j<L) -> z_hat_j, (sig, L) -> c_hat.
 // Phase 2 units: (sig, i<K) -> w1'_i packed.
 template <int MODE, int AV>
@@ -91,7 +102,7 @@ __global__ void __launch_bounds__(kBlock) k_verify_w(uint8_t *pool, size_t pitch
 
     for (int q = threadIdx.x; q < AV * K * 8; q += blockDim.x) (&s_hint[0][0][0])[q] = 0;
     __syncthreads();
-    // hint bitmaps (positions are validated by k_verify_prepare; a bad encoding only needs to not
+    // hint bitmaps (positions are validated by k_verify_setup; a bad encoding only needs to not
     // index out of range here, which byte positions < 256 guarantee)
     for (int q = threadIdx.x; q < AV * K; q += blockDim.x) {
         const int a = q / K, i = q % K, it = i0 + a;
