@@ -20,6 +20,22 @@ __device__ __forceinline__ void ld_lanes(uint2 (&v)[NL], const uint8_t *p) {
     for (int i = 0; i < NL; ++i) v[i] = ld_lane(p + 8 * i);
 }
 
+// The eight 23-bit little-endian candidates of three lanes of an ExpandA block.
+__device__ __forceinline__ void expand_a_candidates(uint32_t (&c)[8], const uint32_t (&al)[25], const uint32_t (&ah)[25], int g) {
+    const uint32_t w0 = al[3 * g], w1 = ah[3 * g], w2 = al[3 * g + 1];
+    const uint32_t w3 = ah[3 * g + 1], w4 = al[3 * g + 2], w5 = ah[3 * g + 2];
+    c[0] = w0;
+    c[1] = __funnelshift_r(w0, w1, 24);
+    c[2] = __funnelshift_r(w1, w2, 16);
+    c[3] = w2 >> 8;
+    c[4] = w3;
+    c[5] = __funnelshift_r(w3, w4, 24);
+    c[6] = __funnelshift_r(w4, w5, 16);
+    c[7] = w5 >> 8;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) c[m] &= 0x7FFFFFu;
+}
+
 // ExpandA entry A[i][j] (NTT domain): SHAKE128(rho || j || i), 23-bit little-endian candidates
 // accepted below q (src/sign.cu:98-163, src/keypair.cu:139-190; the stream is extended until 256
 // coefficients are accepted, as benches/bench_rej_sampling.cu:571-593 does).  Eight candidates that are
@@ -37,23 +53,11 @@ __device__ __forceinline__ void expand_a_groups(const uint2 (&rho)[4], int i, in
         // 21 lanes = 7 groups of 3 lanes = 7 x 8 candidates of 3 bytes.
 #pragma unroll
         for (int g = 0; g < 7; ++g) {
-            const uint32_t w0 = al[3 * g], w1 = ah[3 * g], w2 = al[3 * g + 1];
-            const uint32_t w3 = ah[3 * g + 1], w4 = al[3 * g + 2], w5 = ah[3 * g + 2];
             uint32_t c[8];
-            c[0] = w0;
-            c[1] = __funnelshift_r(w0, w1, 24);
-            c[2] = __funnelshift_r(w1, w2, 16);
-            c[3] = w2 >> 8;
-            c[4] = w3;
-            c[5] = __funnelshift_r(w3, w4, 24);
-            c[6] = __funnelshift_r(w4, w5, 16);
-            c[7] = w5 >> 8;
+            expand_a_candidates(c, al, ah, g);
             bool all = true;
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                c[m] &= 0x7FFFFFu;
-                all &= c[m] < (uint32_t)Q;
-            }
+            for (int m = 0; m < 8; ++m) all &= c[m] < (uint32_t)Q;
             if (all && (ctr & 3) == 0 && ctr + 8 <= N) {
                 emit8(ctr, c);
                 ctr += 8;

@@ -164,15 +164,19 @@ __global__ void __launch_bounds__(kBlock) k_kp_s1(uint8_t *pool, size_t pitch, i
 }
 
 // A block takes kBlock / L consecutive rows (key, i) of t_hat, one thread per entry A_ij of them, and
-// sums the products in shared memory.  Coefficient c of a row sits at c + c / 16 and rows are 273 words
-// apart: the lanes of a warp -- the same j of different rows -- then add to the same coefficient in
-// different banks, and a group's reads of its contiguous slices do not collide either.
+// sums the products in shared memory.  Rows are 257 words apart: the lanes of a warp -- the same j of
+// different rows -- then add to the same coefficient in different banks.
+//
+// Every candidate goes the same way: eight acceptances give eight offsets, then the loads of s1_hat, the
+// products and the predicated additions follow without a branch.  (A wide path for aligned groups beside a
+// path for the others was executed twice by nearly every warp: a lane that has rejected a candidate, one in
+// five by the end of its stream, is no longer aligned.)
 //
 // Bound: the ALU pipe (K L 5 permutations a key).  10 000 Dilithium2 key pairs, this stage: sums by
 // shared-memory atomics with a row's L entries in neighbouring lanes (L-way collisions) 316 us; entries
-// kept in shared memory and summed by the groups (128 KiB per 128 threads, too few warps) 372 us; this
-// layout 322 us (ALU pipe 76% busy while active).  Whole call: global atomics 658 us, now 537 us.
-constexpr int KP_ROW = 273;
+// kept in shared memory and summed by the groups (128 KiB per 128 threads, too few warps) 372 us; wide and
+// narrow paths 321 us; this form 283 us (186 us of permutations at the ALU rate).
+constexpr int KP_ROW = N + 1;
 
 template <int MODE>
 __global__ void __launch_bounds__(kBlock) k_kp_t(uint8_t *pool, size_t pitch, int n) {
@@ -194,21 +198,47 @@ __global__ void __launch_bounds__(kBlock) k_kp_t(uint8_t *pool, size_t pitch, in
             ld_lanes(rho, row + LY::KP_PK);
             const int32_t *sh = reinterpret_cast<const int32_t *>(row + LY::KP_S1H) + (size_t)j * N;
             int32_t *ac = acc + r * KP_ROW;
-            expand_a_groups(
-                rho, i, j,
-                [&](int c, const uint32_t (&v)[8]) {
-                    const int4 s0 = *reinterpret_cast<const int4 *>(sh + c), s1 = *reinterpret_cast<const int4 *>(sh + c + 4);
-                    int32_t *a0 = ac + c + (c >> 4), *a1 = ac + c + 4 + ((c + 4) >> 4);
-                    atomicAdd(a0, montmul((int32_t)v[0], s0.x));
-                    atomicAdd(a0 + 1, montmul((int32_t)v[1], s0.y));
-                    atomicAdd(a0 + 2, montmul((int32_t)v[2], s0.z));
-                    atomicAdd(a0 + 3, montmul((int32_t)v[3], s0.w));
-                    atomicAdd(a1, montmul((int32_t)v[4], s1.x));
-                    atomicAdd(a1 + 1, montmul((int32_t)v[5], s1.y));
-                    atomicAdd(a1 + 2, montmul((int32_t)v[6], s1.z));
-                    atomicAdd(a1 + 3, montmul((int32_t)v[7], s1.w));
-                },
-                [&](int c, uint32_t v) { atomicAdd(ac + c + (c >> 4), montmul((int32_t)v, sh[c])); });
+            uint32_t al[25], ah[25];
+            shake_absorb_seed_nonce<SHAKE128_RATE, 4>(al, ah, rho, (uint32_t)((i << 8) | j));
+            int ctr = 0;
+            // four blocks give at most 224 coefficients: no candidate is one too many
+#pragma unroll 1
+            for (int blk = 0; blk < 4; ++blk) {
+                keccak_f1600(al, ah);
+#pragma unroll
+                for (int gq = 0; gq < 7; ++gq) {
+                    uint32_t c[8];
+                    int32_t sv[8];
+                    int at[8], o = ctr;
+                    expand_a_candidates(c, al, ah, gq);
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) {
+                        at[m] = o;
+                        o += c[m] < (uint32_t)Q ? 1 : 0;
+                    }
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) sv[m] = sh[at[m]];
+#pragma unroll
+                    for (int m = 0; m < 8; ++m)
+                        if (c[m] < (uint32_t)Q) atomicAdd(ac + at[m], montmul((int32_t)c[m], sv[m]));
+                    ctr = o;
+                }
+            }
+#pragma unroll 1
+            while (ctr < N) {
+                keccak_f1600(al, ah);
+#pragma unroll
+                for (int gq = 0; gq < 7; ++gq) {
+                    uint32_t c[8];
+                    expand_a_candidates(c, al, ah, gq);
+#pragma unroll
+                    for (int m = 0; m < 8; ++m)
+                        if (c[m] < (uint32_t)Q && ctr < N) {
+                            atomicAdd(ac + ctr, montmul((int32_t)c[m], sh[ctr]));
+                            ++ctr;
+                        }
+                }
+            }
         }
     }
     __syncthreads();
@@ -222,8 +252,12 @@ __global__ void __launch_bounds__(kBlock) k_kp_t(uint8_t *pool, size_t pitch, in
         const int it = (int)(gr / K), i = (int)(gr % K);
         uint8_t *row = pool + (size_t)it * pitch;
         int32_t x[16];
+        {
+            int32_t y[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) x[m] = reduce32(acc[r * KP_ROW + 17 * g.t + m]);
+            for (int m = 0; m < 16; ++m) y[m] = reduce32(acc[r * KP_ROW + g.t + 16 * m]);
+            strided_to_contig(g, y, x);
+        }
         intt16s(x, g.sm, g.gmask, g.t);
         const uint8_t *s2 = row + LY::KP_SK + PM::SK_S2 + (size_t)i * PM::POLYETA_PACKED;
         int32_t t1[16], t0[16];
