@@ -71,7 +71,8 @@ __device__ __forceinline__ void sign_prehash(uint8_t *pool, size_t pitch, size_t
 
 // One thread per ExpandA entry; rho at row+rho_off, A_hat (K*L polys) at row+mat_off.
 template <int MODE>
-__device__ __forceinline__ void expand_a_entry(uint8_t *pool, size_t pitch, size_t rho_off, size_t mat_off, int n, int block) {
+__device__ __forceinline__ void expand_a_entry(uint8_t *pool, size_t pitch, size_t rho_off, size_t mat_off, int n, int block,
+                                               uint32_t *stage) {
     constexpr int K = Params<MODE>::K, L = Params<MODE>::L, KL = K * L;
     const int s = block * (int)blockDim.x + (int)threadIdx.x;
     if (s >= n * KL) return;
@@ -80,7 +81,7 @@ __device__ __forceinline__ void expand_a_entry(uint8_t *pool, size_t pitch, size
     uint2 rho[4];
     ld_lanes(rho, row + rho_off);
     int32_t *out = reinterpret_cast<int32_t *>(row + mat_off) + (size_t)ij * N;
-    expand_a_row(rho, ij / L, ij % L, out);
+    expand_a_row(rho, ij / L, ij % L, out, stage + threadIdx.x * EA_STAGE);
 }
 
 // Blocks [0, hash_blocks) hash the messages, the others run ExpandA: neither needs the other, and the hash
@@ -90,10 +91,11 @@ template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kItemBlock) k_sign_setup(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens, int n,
                                                            int rhop_given, unsigned hash_blocks) {
     using LY = Layout<MODE>;
+    __shared__ __align__(16) uint32_t s_stage[kItemBlock * EA_STAGE];
     if (blockIdx.x < hash_blocks)
         sign_prehash<MODE, PAIR>(pool, pitch, mlen, mlens, n, rhop_given, (int)blockIdx.x);
     else
-        expand_a_entry<MODE>(pool, pitch, LY::SG_SK + P<MODE>::SK_RHO, LY::sg_mat(mlen), n, (int)(blockIdx.x - hash_blocks));
+        expand_a_entry<MODE>(pool, pitch, LY::SG_SK + P<MODE>::SK_RHO, LY::sg_mat(mlen), n, (int)(blockIdx.x - hash_blocks), s_stage);
 }
 
 // The same with rho read from the packed keys (key i at keys + i * key_bytes, rho = its first 32
@@ -102,6 +104,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kBlock) k_expand_a_keys(const uint8_t *keys, size_t key_bytes, uint8_t *rows, size_t pitch,
                                                           size_t mat_off, int n) {
     constexpr int K = Params<MODE>::K, L = Params<MODE>::L, KL = K * L;
+    __shared__ __align__(16) uint32_t s_stage[kBlock * EA_STAGE];
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n * KL) return;
     const int it = s / KL, ij = s % KL;
@@ -114,7 +117,7 @@ __global__ void __launch_bounds__(kBlock) k_expand_a_keys(const uint8_t *keys, s
         for (int w = 0; w < 4; ++w) rho[w] = load_lane_bytes(key + 8 * w, 8);
     }
     int32_t *out = reinterpret_cast<int32_t *>(rows + (size_t)it * pitch + mat_off) + (size_t)ij * N;
-    expand_a_row(rho, ij / L, ij % L, out);
+    expand_a_row(rho, ij / L, ij % L, out, s_stage + threadIdx.x * EA_STAGE);
 }
 
 // Coefficients a[t + 16 i] of secret polynomial p of a packed key: s1 (p < L), s2 (p < L + K), then t0.

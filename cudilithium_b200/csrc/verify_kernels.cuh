@@ -79,11 +79,12 @@ template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kItemBlock) k_verify_setup(uint8_t *pool, size_t pitch, size_t mlen, const uint32_t *mlens, int n,
                                                              unsigned prep_blocks) {
     using LY = Layout<MODE>;
-    __shared__ uint32_t s_sib[SIB_WORDS * kItemBlock];
+    // SampleInBall scratch or ExpandA rows
+    __shared__ __align__(16) uint32_t s_words[kItemBlock * (EA_STAGE > SIB_WORDS ? EA_STAGE : SIB_WORDS)];
     if (blockIdx.x < prep_blocks)
-        verify_prepare<MODE, PAIR, kItemBlock>(pool, pitch, mlen, mlens, n, (int)blockIdx.x, s_sib);
+        verify_prepare<MODE, PAIR, kItemBlock>(pool, pitch, mlen, mlens, n, (int)blockIdx.x, s_words);
     else
-        expand_a_entry<MODE>(pool, pitch, LY::VF_PK, LY::vf_mat(mlen), n, (int)(blockIdx.x - prep_blocks));
+        expand_a_entry<MODE>(pool, pitch, LY::VF_PK, LY::vf_mat(mlen), n, (int)(blockIdx.x - prep_blocks), s_words);
 }
 
 // AV signatures per 128-thread block.  Phase 1 units: (sig, j<L) -> z_hat_j, (sig, L) -> c_hat.
