@@ -37,10 +37,10 @@ struct EngineBase {
     unsigned nonce_limit = kNonceLimit, lock_spins = kLockSpinLimit, idle_polls = kAsyncIdleLimit;
     size_t last_n = 0;  // items of the last signing batch
     // a batch's metadata (device, the queue block first) and its pinned staging:
-    // [FusedQueue, padded | off | key | mlen | order], each array as long as the batch
+    // [FusedQueue | staged rounds | off | key | mlen | order], each array as long as the batch
     uint8_t *d_meta = nullptr, *h_stage = nullptr;
     FusedQueue *q = nullptr;  // = d_meta
-    StagedRound *rounds = nullptr;
+    StagedRound *rounds = nullptr;  // in d_meta
     FusedQueue *h_status = nullptr; // D2H copy of the queue after a batch
     cudaEvent_t stage_ev = nullptr; // recorded after a batch's metadata upload from h_stage
     // key-cache builds run their independent kernels on a side stream too (fork / join events)
@@ -79,7 +79,10 @@ struct EngineImpl : EngineBase {
     using C = Cache<MODE>;
 
     static constexpr int L = PM::L;
-    static constexpr size_t kStageHead = (sizeof(FusedQueue) + 63) / 64 * 64;
+    // the queue block and the (zeroed) counters of both parts' staged rounds
+    static constexpr size_t kQueueBytes = (sizeof(FusedQueue) + 63) / 64 * 64;
+    static constexpr size_t kStageHead = kQueueBytes + 2 * kStagedMaxRounds * sizeof(StagedRound);
+    static_assert(kStageHead % 64 == 0, "alignment of the arrays behind it");
     static size_t stage_bytes(size_t max_items) {
         return kStageHead + max_items * (3 * sizeof(unsigned) + sizeof(unsigned long long));
     }
@@ -94,7 +97,7 @@ struct EngineImpl : EngineBase {
     // Device bytes the engine needs (the admission budget checks this before allocating).
     size_t required_bytes(size_t max_keys, size_t max_items) const {
         return max_keys * (align256(C::SK_ROW) + align256(C::PK_ROW)) + max_items * (C::ITEM_BYTES + 4 * sizeof(unsigned)) +
-               stage_bytes(max_items) + 2 * kStagedMaxRounds * sizeof(StagedRound) + scratch_for(max_items);
+               stage_bytes(max_items) + scratch_for(max_items);
     }
     // attempt slots of the largest signer variant, or the packed w1' of a verification batch
     size_t scratch_for(size_t max_items) const {
@@ -173,8 +176,7 @@ struct EngineImpl : EngineBase {
                     cudaMalloc(&next_nonce, mi * sizeof(unsigned)) != cudaSuccess ||
                     cudaMalloc(&inflight, mi * sizeof(unsigned)) != cudaSuccess ||
                     cudaMalloc(&scratch, scratch_bytes) != cudaSuccess)) ||
-            cudaMalloc(&d_meta, stage_bytes(mi)) != cudaSuccess ||
-            cudaMalloc(&rounds, 2 * kStagedMaxRounds * sizeof(StagedRound)) != cudaSuccess || cudaMallocHost(&h_stage, stage_bytes(mi)) != cudaSuccess ||
+            cudaMalloc(&d_meta, stage_bytes(mi)) != cudaSuccess || cudaMallocHost(&h_stage, stage_bytes(mi)) != cudaSuccess ||
             cudaMallocHost(&h_status, sizeof(FusedQueue)) != cudaSuccess)
             return ::cudil::cudil_record_cuda_error(cudaGetLastError(), __FILE__, __LINE__);
         std::memset(h_status, 0, sizeof(FusedQueue));
@@ -183,6 +185,7 @@ struct EngineImpl : EngineBase {
         CUDIL_CK(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming));
         CUDIL_CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
         q = reinterpret_cast<FusedQueue *>(d_meta);
+        rounds = reinterpret_cast<StagedRound *>(d_meta + kQueueBytes);
         CUDIL_CK(cudaMemset(q, 0, sizeof(FusedQueue)));
         return CUDIL_OK;
     }
@@ -198,7 +201,6 @@ struct EngineImpl : EngineBase {
         cudaFree(next_nonce);
         cudaFree(inflight);
         cudaFree(d_meta);
-        cudaFree(rounds);
         cudaFree(scratch);
         if (h_stage) cudaFreeHost(h_stage);
         if (h_status) cudaFreeHost(h_status);
@@ -293,7 +295,7 @@ struct EngineImpl : EngineBase {
         // batch is prepared)
         if (stage_pending) CUDIL_CK(cudaEventSynchronize(stage_ev));
         FusedQueue *hq = reinterpret_cast<FusedQueue *>(h_stage);
-        std::memset(hq, 0, sizeof(FusedQueue));
+        std::memset(h_stage, 0, kStageHead);
         hq->n = (unsigned)n;
         if (rho_seed) {
             hq->rho_seeded = 1u;
@@ -381,8 +383,8 @@ struct EngineImpl : EngineBase {
         if (stage == 0) {
             const unsigned cb = std::max(blocks_for((size_t)hi + 1, 256), std::min(blocks_for(t.prev_slots, 8), 8u * sms));
             CUDIL_LAUNCH(KID_ST_CLAIM, st, k_st_claim<MODE><<<cb, 256, 0, st>>>(a, t.r, true));
-            const unsigned mb = (size_t)slots * L <= (size_t)sm_count * 128 ? 32u : (unsigned)kBlock;
-            CUDIL_LAUNCH(KID_ST_MASK, st, k_st_mask<MODE><<<blocks_for((size_t)slots * L, mb), mb, 0, st>>>(a, t.r));
+            const unsigned mb = (size_t)slots * L <= (size_t)sms * 128 ? 32u : (unsigned)kBlock;
+            CUDIL_LAUNCH(KID_ST_MASK, st, CUDIL_PAIRED_ON((size_t)slots * L, sm_count, k_st_mask<MODE, PAIR><<<blocks_for((size_t)slots * L * LANES, mb), mb, 0, st>>>(a, t.r)));
         } else if (stage == 1) {
             const unsigned wb = slots <= 8u * sms ? 1u : 4u;  // warps per block
             CUDIL_LAUNCH(KID_ST_W, st, k_st_w<MODE><<<blocks_for(slots, wb), 32 * wb, wb * S::WARP_W, st>>>(a, t.r));
@@ -481,7 +483,6 @@ struct EngineImpl : EngineBase {
             part[k].r = 0;
             first += a.count;
         }
-        CUDIL_CK(cudaMemsetAsync(rounds, 0, 2 * kStagedMaxRounds * sizeof(StagedRound), st));
         if (parts == 2) {
             CUDIL_CK(cudaEventRecord(fork_ev, st));
             CUDIL_CK(cudaStreamWaitEvent(side, fork_ev, 0));

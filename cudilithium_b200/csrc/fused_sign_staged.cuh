@@ -4,7 +4,7 @@
 // A round is five kernels over the round's attempts, each in the shape its stage needs:
 //   k_st_claim      publishes the previous round's winners, compacts the pending items and gives each its
 //                   next D nonces, D = target / pending, at most kStagedMaxDepth
-//   k_st_mask       ExpandMask, one thread per (attempt, j) stream
+//   k_st_mask       ExpandMask, one thread (few streams: a pair) per (attempt, j) stream
 //   k_st_w          w = A y, Decompose, w1 packing: one warp per attempt, its two 16-thread groups on
 //                   different polynomials
 //   k_st_challenge  c~ = H(mu || w1) and SampleInBall, one thread per attempt
@@ -24,7 +24,7 @@
 
 namespace cudil {
 
-// Counters of one round, zeroed before the batch.
+// Counters of one round; they go up zeroed with the batch's metadata.
 struct StagedRound {
     unsigned npend;     // pending items listed
     unsigned depth;     // attempts of each; the first `extra` listed have one more
@@ -214,30 +214,53 @@ __device__ __forceinline__ void unpack_y(int32_t (&x)[16], const uint8_t *poly, 
     }
 }
 
-template <int MODE>
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kBlock) k_st_mask(StagedArgs a, int r) {
     using PM = P<MODE>;
     using S = StagedSlot<MODE>;
-    constexpr int L = PM::L;
-    const unsigned total = staged_attempts(a, r) * L;
+    constexpr int L = PM::L, YW = PM::Z_BITS / 2, RL = SHAKE256_RATE / 8, LANES = PAIR ? 2 : 1;
+    const unsigned total = staged_attempts(a, r) * L, per = blockDim.x / LANES;
     const StagedAttempt *att = a.att[r & 1];
-    for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) {
-        const unsigned s = u / L, j = u % L, item = att[s].item, nonce = att[s].nonce;
-        if (nonce == kStagedNoNonce || !bc_ok(item < a.n, BC_SIGN_SLOT)) continue;
-        uint2 rhop[8];
-        ld_lanes(rhop, a.items + (size_t)item * Cache<MODE>::ITEM_BYTES + 64);
-        uint32_t al[25], ah[25];
-        shake_absorb_seed_nonce<SHAKE256_RATE, 8>(al, ah, rhop, (L * nonce + j) & 0xFFFFu);
+    // (the whole block strides together: in pair form every lane of a warp takes part in the shuffles)
+    for (unsigned u0 = blockIdx.x * per; u0 < total; u0 += gridDim.x * per) {
+        const unsigned u = u0 + threadIdx.x / LANES;
+        bool on = u < total;
+        const unsigned s = on ? u / L : 0u, j = u % L, item = on ? att[s].item : 0u, nonce = on ? att[s].nonce : kStagedNoNonce;
+        on = nonce != kStagedNoNonce && bc_ok(item < a.n, BC_SIGN_SLOT);
+        if (!PAIR && !on) continue;
+        const uint8_t *rhop = a.items + (size_t)(on ? item : 0u) * Cache<MODE>::ITEM_BYTES + 64;
         uint32_t *o = reinterpret_cast<uint32_t *>(a.slots + (size_t)s * S::SIZE + S::Y + (size_t)j * PM::POLYZ_PACKED);
-        // (unrolled: the words' places are constants)
-        constexpr int YW = PM::Z_BITS / 2, RL = SHAKE256_RATE / 8;
+        const uint32_t kappa = (L * nonce + j) & 0xFFFFu;
+        // SHAKE256(rho' || kappa): the words' places are constants, so the blocks are unrolled
+        if constexpr (PAIR) {
+            const int half = threadIdx.x & 1;
+            uint32_t st[25];
 #pragma unroll
-        for (int blk = 0; blk < PM::MASK_BLOCKS; ++blk) {
-            keccak_f1600(al, ah);
+            for (int w = 0; w < 25; ++w) st[w] = w < 8 ? reinterpret_cast<const uint32_t *>(rhop)[2 * w + half] : 0u;
+            st[8] = half ? 0u : (kappa | (0x1Fu << 16));
+            st[RL - 1] ^= half ? 0x80000000u : 0u;
 #pragma unroll
-            for (int w = 0; w < 2 * RL; ++w) {
-                const int g = 2 * RL * blk + w;
-                if (g < 16 * YW) o[y_word<MODE>(g / YW, g % YW)] = (w & 1) ? ah[w >> 1] : al[w >> 1];
+            for (int blk = 0; blk < PM::MASK_BLOCKS; ++blk) {
+                keccak_f1600_pair(st, half);
+#pragma unroll
+                for (int w = 0; w < RL; ++w) {
+                    const int g = 2 * (RL * blk + w);  // the pair's words g and g + 1
+                    if (g < 16 * YW && on) o[half ? y_word<MODE>((g + 1) / YW, (g + 1) % YW) : y_word<MODE>(g / YW, g % YW)] = st[w];
+                }
+            }
+        } else {
+            uint2 rp[8];
+            ld_lanes(rp, rhop);
+            uint32_t al[25], ah[25];
+            shake_absorb_seed_nonce<SHAKE256_RATE, 8>(al, ah, rp, kappa);
+#pragma unroll
+            for (int blk = 0; blk < PM::MASK_BLOCKS; ++blk) {
+                keccak_f1600(al, ah);
+#pragma unroll
+                for (int w = 0; w < 2 * RL; ++w) {
+                    const int g = 2 * RL * blk + w;
+                    if (g < 16 * YW) o[y_word<MODE>(g / YW, g % YW)] = (w & 1) ? ah[w >> 1] : al[w >> 1];
+                }
             }
         }
     }

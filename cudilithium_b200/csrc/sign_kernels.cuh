@@ -375,19 +375,19 @@ __global__ void __launch_bounds__(TB) k_sign_challenge(const uint8_t *sign_pool,
     if (on && (!PAIR || sh.half() == 0)) sib_store<TB>(trow + LY::TP_CMASK, s_sib, threadIdx.x);
 }
 
-// One warp per attempt: c_hat = NTT(c); r0 = w0 - c*s2, z = y + c*s1 and c*t0 (norm checks);
+// One warp (a block of its own: attempts end after different numbers of steps) per attempt: c_hat = NTT(c); r0 = w0 - c*s2, z = y + c*s1 and c*t0 (norm checks);
 // MakeHint (at most OMEGA, positions in ascending order).  The two 16-thread groups of the warp
 // take the attempt's polynomials in pairs (poly 2p + half), so they follow the same control flow
 // and a rejection ends the attempt for the whole warp.  On acceptance the temp row holds the
 // complete signature and done[e] = 1 (src/sign.cu:1010-1195).
 template <int MODE>
-__global__ void __launch_bounds__(kBlock, 4) k_sign_reject(const uint8_t *sign_pool, size_t sp, size_t mlen, uint8_t *temp_pool,
+__global__ void __launch_bounds__(32, 16) k_sign_reject(const uint8_t *sign_pool, size_t sp, size_t mlen, uint8_t *temp_pool,
                                                         size_t tp, const uint32_t *exec_lut, uint8_t *done, int nexec,
                                                         int nitems) {
     using PM = P<MODE>;
     using LY = Layout<MODE>;
     constexpr int K = PM::K, L = PM::L, OMEGA = PM::OMEGA;
-    __shared__ int32_t sm[kGroupsPerBlock * NTT_SMEM_WORDS];
+    __shared__ int32_t sm[2 * NTT_SMEM_WORDS];
     const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (e >= nexec) return;  // (the same for the whole warp)
     Group g = make_group(sm, threadIdx.x >> 4);
