@@ -4,7 +4,7 @@
 Headline workload: Dilithium2 batched signing of 10000 32-byte messages, one key per message (the
 reference's bench_dilithium batch, benches/bench_dilithium.cu:277-296), keys from the reference's
 seed scheme SHAKE128(le64(2i+1)).  A step = the fused engine building the batch's key caches and
-signing the batch in one graph launch (then verifying it against freshly built public-key caches).
+signing the batch in one call (then verifying it against freshly built public-key caches).
 
   value         Dilithium2 signatures/s of the fused engine, inputs resident in HBM
   plain         the same batch through the plain stage-by-stage path (cudil_sign_dev /
@@ -14,7 +14,7 @@ signing the batch in one graph launch (then verifying it against freshly built p
                 signatures written by the signer into pinned host memory; all copies inside the
                 timed region (the one-batch-at-a-time figure is reported beside it)
   verify_per_s  verifications/s of the same step (fused engine, public-key caches built per step)
-  roofline      the persistent signing kernel: algorithmic 32-bit ALU operations (work model below,
+  roofline      the signing batch: algorithmic 32-bit ALU operations (work model below,
                 attempts counted on the device) over its CUDA-event duration, against the measured
                 LOP3/SHF issue peak of this GPU
   configs       configs 1-4 of the workload list (batch-1024 latency, NTT microbench vs HBM peak,
@@ -52,10 +52,6 @@ OPS_PERM = 24 * 190
 OPS_NTT_FWD = 1024 * 6          # 1024 butterflies: 3 IMAD + 3 IADD
 OPS_NTT_INV = 1024 * 6 + 256 * 4  # + the final multiplication by f
 OPS_PW = 5                        # one Montgomery pointwise product
-# k_fused_sign<2,256> (engine sign-kernel variant 0, the tuned Dilithium2 signer), batch 10000:
-# 0.771482 GB read + 0.418236 GB written per launch (ncu)
-FUSED_SIGN_TRAFFIC_BYTES = 0.771482e9 + 0.418236e9
-FUSED_SIGN_TRAFFIC_VARIANT = 0
 
 
 def log(*a):
@@ -448,7 +444,7 @@ def run_gpu(args) -> dict | None:
     plain_verify_rate = world * B * args.steps / (plain_verify_ms / 1e3)
 
     # ---- fused engine: per step the key caches are built for this batch's keys (each key signs
-    # once here, so the cache build is part of the per-signature work) and one graph launch signs
+    # once here, so the cache build is part of the per-signature work) and one call signs
     es = Engine(mode, max_keys=B, max_items=B, threads=args.engine_threads)
     ev = Engine(mode, max_keys=B, max_items=B, threads=args.engine_threads)
     if args.spec_slots:
@@ -619,7 +615,7 @@ def run_gpu(args) -> dict | None:
         pe[j].sign(p_out[j], pm_m, offs, lens, keys, stream=p_st[j])
         free_ev[j].record(p_st[j])
 
-    for k in range(2):  # warm-up: captures both engines' graphs
+    for k in range(2):  # warm-up
         stream_step(k)
     barrier()
     for k in range(2):
@@ -655,22 +651,20 @@ def run_gpu(args) -> dict | None:
     stats = _lib.kernel_stats()
     att1, intt1 = es.last_work()
     alg_att, alg_intt = algorithmic_attempts(es.last_nonces(B), att1, intt1)
-    g_ms = stats.get("k_fused_sign (graph)", (0.0, 1))[0]
+    g_ms = stats.get("sign batch (engine)", (0.0, 1))[0]
     # algorithmic work: the attempts deterministic signing needs (not the speculative ones issued)
     sign_ops = sign_attempt_ops(pm, alg_att, alg_intt) + B * sign_prehash_ops(MLEN)
     c_ms = cb0.elapsed_time(cb1)
     achieved = sign_ops / (g_ms / 1e3) / 1e9 if g_ms else None
-    total_ms = g_ms + c_ms  # the step: cache build span + signing graph
+    total_ms = g_ms + c_ms  # the step: cache build span + signing batch
     roofline = {
         "bound": "int32-alu",
-        "kernel": f"persistent signer, engine sign-kernel variant {es.sign_kernel} "
-                  f"({es.info()['sign_blocks']} blocks; graph with init + prehash)",
+        "kernel": f"signing batch, engine sign-kernel variant {es.sign_kernel} (0: prehash, rounds of claim, "
+                  f"ExpandMask, w, challenge and rejection kernels, then the persistent kernel on what they leave)",
         "achieved": achieved, "peak": peak_ops / 1e9, "unit": "Gop/s",
         "frac": achieved / (peak_ops / 1e9) if achieved else None,
-        # DRAM bytes per launch of the same signer launch (batch 10000, one key per message) from
-        # one ncu capture: dram__bytes_read.sum + dram__bytes_write.sum
-        "traffic": FUSED_SIGN_TRAFFIC_BYTES if (B == 10000 and mode == 2 and es.sign_kernel == FUSED_SIGN_TRAFFIC_VARIANT) else None,
-        "traffic_source": "ncu --set full capture of k_fused_sign<2,256>, bench.py --workload fused-sign --batch 10000",
+        "traffic": None,
+        "traffic_source": "not one kernel: the rounds' kernels are captured one by one (profiles/)",
         "ms_per_launch": g_ms, "launches": 1, "share_of_step": g_ms / total_ms if total_ms else None,
         "attempts_algorithmic": alg_att, "attempts_issued": att1, "speculation_overhead": att1 / alg_att,
         "reject_intt_issued": intt1, "signer_phases": es.last_phases(),
@@ -689,8 +683,8 @@ def run_gpu(args) -> dict | None:
         "ms_per_step": pipe_ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": "int32", "data": "synthetic: keys from the reference seed scheme, uniform random 32-byte messages",
         "config": headline_config(mode, B, world),
-        "path": "fused engine: per step the batch's key caches are built and the batch is signed in one graph "
-                "launch (persistent signer); consecutive steps alternate between two engines on two streams "
+        "path": "fused engine: per step the batch's key caches are built and the batch is signed in one "
+                "call (staged rounds); consecutive steps alternate between two engines on two streams "
                 "(EnginePipeline), one timed region over all steps",
         "one_batch_at_a_time": {"value": value_single, "ms_per_step": fs_ms / args.steps, "verify_per_s": verify_single,
                                 "note": "the same steps on one engine and one stream, each step timed on its own"},
@@ -1159,7 +1153,7 @@ def run_profile_case(args) -> dict:
     spp = torch.cuda.current_stream().cuda_stream
     if args.workload == "d3-sign":
         # the Dilithium3 long-message signing workload (16384 messages over 1024 keys, log-uniform
-        # 32 B .. 64 KiB): one warm-up and one measured graph launch of the fused engine, checked
+        # 32 B .. 64 KiB): one warm-up and one measured batch of the fused engine, checked
         # against the plain path
         nk, nm = 1024, 16384
         d3 = cd.Dilithium(3)

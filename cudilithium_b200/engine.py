@@ -1,4 +1,4 @@
-"""Fused engine: per-key resident caches + one persistent, graph-launched kernel per batch.
+"""Fused engine: per-key resident caches, a whole signing or verification batch enqueued per call.
 
 Python host side of the ``cudil_engine_*`` C ABI (include/cudilithium.h).  An ``Engine`` wraps one
 engine of one parameter set on the current CUDA device; an ``EnginePipeline`` runs a stream of
@@ -68,7 +68,7 @@ class Engine:
         return lib.cudil_engine_device_bytes(self.h)
 
     def set_sign_kernel(self, variant: int):
-        """0 phased persistent signer; 1..4 asynchronous with (threads, slots) per block of
+        """0 staged rounds over the whole GPU; 1..4 asynchronous persistent with (threads, slots) per block of
         (256, 64), (512, 128), (640, 160), (768, 192); 5 phased with one wide block per SM (512
         threads, 384 for Dilithium5); see cudil_engine_set_sign_kernel."""
         check(lib.cudil_engine_set_sign_kernel(self.h, variant), "set_sign_kernel")
@@ -174,7 +174,8 @@ class Engine:
         return a.value, i.value
 
     def last_phases(self) -> dict:
-        """Signer phase profile of the last batch (block-summed SM cycles and iterations)."""
+        """Signer profile of the last batch: rounds of the staged signer (iterations), block-summed SM cycles
+        and iterations of the phased one."""
         cyc = (ctypes.c_ulonglong * 4)()
         it = ctypes.c_uint32()
         lib.cudil_engine_last_phases(self.h, cyc, ctypes.byref(it))
@@ -207,10 +208,9 @@ class EnginePipeline:
     """Runs a stream of batches over ``depth`` engines, each on its own CUDA stream, batch k on
     engine k mod depth (signing or verification).
 
-    The persistent kernels' blocks finish apart: over the last part of a launch more and more SMs
-    have no block left.  With one engine on one stream the next batch's key-cache build and prehash
-    wait for the whole launch; with an engine per stream they start on the SMs freed at its end,
-    and so do the first blocks of the next kernel.  Batches are independent (each engine keeps its
+    A batch's late signing rounds leave most of the GPU idle.  With one engine on one stream the next
+    batch's key-cache build and prehash wait for them; with an engine per stream they run beside
+    them, and so do the next batch's first rounds.  Batches are independent (each engine keeps its
     own caches, queue and scratch), so every batch's results are the same as run alone.  The same
     works from C with one ``cudil_engine`` per stream.
 

@@ -198,9 +198,9 @@ int cudil_ntt_mul(const int32_t *d_a, const int32_t *d_b, int32_t *d_out, size_t
  * One engine serves one parameter set on the current device.  It keeps, per key, the expanded
  * matrix A_hat and the NTT-domain key material resident in device memory (secret keys: A_hat,
  * s1_hat, s2_hat, t0_hat, rho, K, tr; public keys: A_hat, NTT(t1 * 2^d), tr) and runs a whole
- * signing batch as one CUDA-graph launch around ONE persistent kernel whose device-side ticket
- * queue hands every rejected attempt's slot the next (message, nonce) attempt.  Results are
- * identical to cudil_sign / cudil_verify (deterministic signing: smallest accepted nonce).
+ * signing batch without waiting for the device in between: rounds of stage kernels over all pending
+ * attempts (or one persistent kernel, cudil_engine_set_sign_kernel) whose counts stay on the
+ * device.  Results are identical to cudil_sign / cudil_verify (deterministic signing: smallest accepted nonce).
  *
  * create:  allocates everything up front (max_keys cache rows of each kind, max_items messages per
  *          batch, scratch for one persistent grid); CUDIL_ERR_BUDGET if that exceeds
@@ -209,8 +209,8 @@ int cudil_ntt_mul(const int32_t *d_a, const int32_t *d_b, int32_t *d_out, size_t
  *          aligned offset (offsets[i] + mlens[i] <= msgs_bytes, checked before any launch);
  *          offsets / mlens / key_idx are HOST arrays of n entries (uploaded before the launch);
  *          signatures are dense (sig_bytes each).  The signature output of sign may be device
- *          memory or pinned host memory: in host memory each signature is written over PCIe as
- *          soon as it is found, so the download overlaps the signing (pageable host memory:
+ *          memory or pinned host memory: in host memory a round's signatures are written over
+ *          PCIe when the round ends, so the download overlaps the rest (pageable host memory:
  *          CUDIL_ERR_INVALID).  Asynchronous on `stream`; one batch in flight
  *          per engine (calls on one engine must be ordered on one stream).
  * last_status: attempts and error flags of the last completed batch (valid after sync);
@@ -275,23 +275,26 @@ int cudil_engine_last_nonces(cudil_engine *e, unsigned *out, size_t n, void *str
  * rejection checks (for throughput accounting). */
 int cudil_engine_last_work(const cudil_engine *e, unsigned long long *attempts, unsigned long long *reject_intt);
 /* Signer tuning: per-block target of signing attempts in flight (1 .. 2 * threads_per_block).
- * Every block owns a share of the batch's items; while it has many pending items each has at most
+ * The staged signer (kernel 0) counts four blocks per SM: a round aims at 4 * SMs * target attempts,
+ * rounded to whole layers of ExpandMask streams, at most 64 per item.  In the persistent kernels every
+ * block owns a share of the batch's items; while it has many pending items each has at most
  * two attempts in flight, and as they run out the remaining ones get up to target / pending
  * consecutive nonces in flight (at most 64).  0 = default (threads_per_block).  Takes effect
  * from the next batch. */
 int cudil_engine_set_spec_slots(cudil_engine *e, unsigned spec_slots);
-/* Signer kernel: 0 (default) = phased persistent kernel (block-wide Keccak / NTT phases,
- * threads_per_block threads); 1..4 = asynchronous persistent kernel -- warps take ready jobs from a
+/* Signer kernel: 0 (default) = staged rounds over the whole GPU, finished by the phased persistent
+ * kernel (block-wide Keccak / NTT phases, threads_per_block threads) on what they leave; that kernel
+ * alone where lock_spins is set below its default, and variant 5 where a batch has more items than the
+ * scratch has attempt slots; 1..4 = asynchronous persistent kernel -- warps take ready jobs from a
  * per-block attempt-slot state machine without block barriers, the speculation target capped at
  * the slot count -- with (threads, slots) per block of (256, 64), (512, 128), (640, 160) and
  * (768, 192); 5 = the phased kernel with one wide block per SM (512 threads; 384 for Dilithium5).
  * Results are identical for every variant. */
 int cudil_engine_set_sign_kernel(cudil_engine *e, int variant);
 /* Large batches: a signing batch of at least min_items items runs signer kernel `variant` with
- * speculation target `spec_slots` (0 = threads_per_block) through a graph of its own; smaller
- * batches keep the kernel and target set above.  min_items = 0 turns the large-batch choice off.
- * Default: min_items = 224 items per SM, variant 5 (the wide phased kernel), target 128, which is
- * the fastest signer at 64 Ki items for every parameter set.  Results are identical either way. */
+ * speculation target `spec_slots` (0 = threads_per_block); smaller batches keep the kernel and
+ * target set above.  min_items = 0 (the default) turns the large-batch choice off: the staged signer
+ * is the fastest at every size.  Results are identical either way. */
 int cudil_engine_set_large_batch(cudil_engine *e, size_t min_items, int variant, unsigned spec_slots);
 /* Job profile of the last batch of the asynchronous signer, summed over warps: SM cycles spent in
  * rejection / w / challenge / ExpandMask jobs, claims and idle polls (out[0..5]) and their counts
