@@ -609,7 +609,7 @@ struct EngineImpl : EngineBase {
         if (rc) return rc;
         mr.msgs = d_msgs;
         cudaEvent_t ev = Profiler::get().before(st);
-        VerifyArgs a{pk_cache, pk_pitch, mr, d_sig, (size_t)PM::SIG_BYTES, items, scratch, best, d_ret, (unsigned)n};
+        VerifyArgs a{pk_cache, pk_pitch, mr, d_sig, (size_t)PM::SIG_BYTES, items, scratch, locks, d_ret, (unsigned)n};  // (best[] keeps the last signing batch's nonces)
         CUDIL_LAUNCH(KID_FV_CHALLENGE, st, CUDIL_PAIRED_ON(n, sm_count, k_fv_challenge<MODE, PAIR><<<prehash_blocks(n * LANES), kPrehashBlock, 0, st>>>(a)));
         const unsigned wb = n <= 8u * (size_t)sm_count ? 1u : 4u;  // warps per block
         CUDIL_LAUNCH(KID_FV_W, st, k_fv_w<MODE><<<blocks_for(n, wb), 32 * wb, wb * VerifyRow<MODE>::WARP, st>>>(a));

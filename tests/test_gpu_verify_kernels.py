@@ -50,3 +50,30 @@ def test_verify_matches_oracle(cuda_ok, oracle, mode, n):
     assert np.array_equal(d_ret.cpu().numpy(), want)
     if n > 7:
         assert (want == 0).any() and (want == -1).any()
+
+
+def test_verify_keeps_the_last_signing_nonces(cuda_ok, oracle):
+    """last_nonces reports the last signing batch also after a verification on the same engine."""
+    import torch
+
+    from cudilithium_b200.engine import Engine, pack_messages
+    n = 50
+    pk, sk = oracle.keypair_batch(2, 3, rand_index=8)
+    m = np.random.default_rng(1).integers(0, 256, (n, 20), dtype=np.uint8)
+    idx = (np.arange(n) % 3).astype(np.uint32)
+    want, att = oracle.sign_batch(2, m, sk[idx], return_attempts=True)
+    d_msgs, offs, lens = pack_messages(m)
+    eng = Engine(2, max_keys=3, max_items=n)
+    eng.set_secret_keys(torch.from_numpy(sk.reshape(-1)).cuda())
+    eng.set_public_keys(torch.from_numpy(pk.reshape(-1)).cuda())
+    sig = torch.zeros(n * eng.params.sig_bytes, dtype=torch.uint8, device="cuda")
+    ret = torch.full((n,), 5, dtype=torch.int32, device="cuda")
+    eng.sign(sig, d_msgs, offs, lens, idx)
+    eng.verify(ret, sig, d_msgs, offs, lens, idx)
+    torch.cuda.synchronize()
+    assert np.array_equal(sig.cpu().numpy().reshape(n, -1), want) and not ret.cpu().numpy().any()
+    assert np.array_equal(eng.last_nonces(n).astype(np.int64) + 1, np.asarray(att, np.int64))
+    eng.sign(sig, d_msgs, offs, lens, idx)  # and the next signing batch is unaffected
+    torch.cuda.synchronize()
+    assert np.array_equal(sig.cpu().numpy().reshape(n, -1), want)
+    eng.close()
