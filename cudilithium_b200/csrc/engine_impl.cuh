@@ -379,7 +379,9 @@ struct EngineImpl : EngineBase {
         // enough blocks for a pending count four standard deviations above the expected one (kernels
         // stride over what exceeds it)
         const double hi = std::min((double)a.count, t.p + 4.0 * std::sqrt(t.p) + 4.0);
-        const unsigned slots = (unsigned)std::min((double)a.cap, std::max(hi, std::min((double)a.target, hi * kStagedMaxDepth)));
+        // (attempts at most: whole quanta where the claim rounds down to them)
+        const double most = hi > a.quantum && hi < 4.0 * a.quantum ? std::floor(hi / a.quantum) * a.quantum : hi;
+        const unsigned slots = (unsigned)std::min((double)a.cap, std::max(most, std::min((double)a.target, hi * kStagedMaxDepth)));
         if (stage == 0) {
             const unsigned cb = std::max(blocks_for((size_t)hi + 1, 256), std::min(blocks_for(t.prev_slots, 8), 8u * sms));
             CUDIL_LAUNCH(KID_ST_CLAIM, st, k_st_claim<MODE><<<cb, 256, 0, st>>>(a, t.r, true));
