@@ -824,10 +824,12 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_fused_sign(FusedSign
     // owned items still pending: all of them after k_fused_init, those the staged rounds left otherwise
     if (tid == 0) s_ctl[CT_PEND] = 0;
     __syncthreads();
-    for (unsigned k = tid; k < n_own; k += THREADS)
-        if (__ldcg(arg.best + b0 + k * grid) == 0xFFFFFFFFu) atomicAdd(&s_ctl[CT_PEND], 1u);
-    __syncthreads();
-    if (s_ctl[CT_PEND] == 0u) return;
+    unsigned mine = 0;
+    for (unsigned k = tid; k < n_own; k += THREADS) mine += __ldcg(arg.best + b0 + k * grid) == 0xFFFFFFFFu ? 1u : 0u;
+    if (mine) atomicAdd(&s_ctl[CT_PEND], mine);
+    // The block leaves as a whole: every thread gets the barrier's own result.  (The count itself may already
+    // have been lowered when a late warp reads it: the claim that follows marks items that are out of nonces.)
+    if (!__syncthreads_or(mine != 0u)) return;
     claim(0);
     keccak_phase(0, 0, 0, (int)s_ctl[CT_NA0]);
     __syncthreads();
