@@ -37,10 +37,9 @@ struct EngineBase {
     unsigned nonce_limit = kNonceLimit, lock_spins = kLockSpinLimit, idle_polls = kAsyncIdleLimit;
     size_t last_n = 0;  // items of the last signing batch
     // a batch's metadata (device, the queue block first) and its pinned staging:
-    // [FusedQueue | staged rounds | off | key | mlen | order], each array as long as the batch
+    // [FusedQueue | off | key | mlen | order], each array as long as the batch
     uint8_t *d_meta = nullptr, *h_stage = nullptr;
     FusedQueue *q = nullptr;  // = d_meta
-    StagedRound *rounds = nullptr;  // in d_meta
     FusedQueue *h_status = nullptr; // D2H copy of the queue after a batch
     cudaEvent_t stage_ev = nullptr; // recorded after a batch's metadata upload from h_stage
     // key-cache builds run their independent kernels on a side stream too (fork / join events)
@@ -79,10 +78,8 @@ struct EngineImpl : EngineBase {
     using C = Cache<MODE>;
 
     static constexpr int L = PM::L;
-    // the queue block and the (zeroed) counters of both parts' staged rounds
-    static constexpr size_t kQueueBytes = (sizeof(FusedQueue) + 63) / 64 * 64;
-    static constexpr size_t kStageHead = kQueueBytes + 2 * kStagedMaxRounds * sizeof(StagedRound);
-    static_assert(kStageHead % 64 == 0, "alignment of the arrays behind it");
+    // the queue block, padded for the arrays behind it
+    static constexpr size_t kStageHead = (sizeof(FusedQueue) + 63) / 64 * 64;
     static size_t stage_bytes(size_t max_items) {
         return kStageHead + max_items * (3 * sizeof(unsigned) + sizeof(unsigned long long));
     }
@@ -99,10 +96,10 @@ struct EngineImpl : EngineBase {
         return max_keys * (align256(C::SK_ROW) + align256(C::PK_ROW)) + max_items * (C::ITEM_BYTES + 4 * sizeof(unsigned)) +
                stage_bytes(max_items) + scratch_for(max_items);
     }
-    // attempt slots of the largest signer variant, or the packed w1' of a verification batch
+    // attempt slots of the largest signer variant, or the packed w1' of a verification turn
     size_t scratch_for(size_t max_items) const {
         if (max_items == 0) return 0;
-        size_t b = std::max((size_t)sign_grid * 2 * threads * C::SLOT, max_items * VerifyRow<MODE>::W1);
+        size_t b = std::max((size_t)sign_grid * 2 * threads * C::SLOT, std::min(max_items, kVerifyTurn) * VerifyRow<MODE>::W1);
         static constexpr int slots[kAsyncVariants] = {64, 128, 160, 192};
         for (int v = 0; v < kAsyncVariants; ++v) b = std::max(b, (size_t)async_grid[v] * slots[v] * C::SLOT);
         b = std::max(b, (size_t)wide_grid * 2 * kWideThreads * C::SLOT);
@@ -185,7 +182,6 @@ struct EngineImpl : EngineBase {
         CUDIL_CK(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming));
         CUDIL_CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
         q = reinterpret_cast<FusedQueue *>(d_meta);
-        rounds = reinterpret_cast<StagedRound *>(d_meta + kQueueBytes);
         CUDIL_CK(cudaMemset(q, 0, sizeof(FusedQueue)));
         return CUDIL_OK;
     }
@@ -349,9 +345,12 @@ struct EngineImpl : EngineBase {
             k_fused_sign<MODE, 256><<<sign_grid, 256, sign_smem, st>>>(a);
     }
 
-    // Attempt slots the scratch holds beside the staged signer's lists.
+    // Where the staged signer's attempt slots start in the scratch: behind two lists of pending items and the
+    // round counters of both parts.
+    size_t staged_lists() const { return 2 * align256(max_items * sizeof(unsigned)) + align256(2 * kStagedRoundBytes); }
+    // Attempt slots the scratch holds behind them.
     size_t staged_cap() const {
-        const size_t lists = 2 * align256(max_items * sizeof(unsigned));
+        const size_t lists = staged_lists();
         if (scratch_bytes <= lists) return 0;
         return (scratch_bytes - lists) / (StagedSlot<MODE>::SIZE + 2 * sizeof(StagedAttempt));
     }
@@ -444,7 +443,8 @@ struct EngineImpl : EngineBase {
         const int parts = split ? 2 : 1;
         const size_t cap = std::min<size_t>(staged_cap(), 0x7FFFFFFFu) / parts;
         unsigned *pend = reinterpret_cast<unsigned *>(scratch);
-        uint8_t *slots = scratch + 2 * align256(max_items * sizeof(unsigned));
+        StagedRound *rounds = reinterpret_cast<StagedRound *>(scratch + 2 * align256(max_items * sizeof(unsigned)));
+        uint8_t *slots = scratch + staged_lists();
         StagedAttempt *att = reinterpret_cast<StagedAttempt *>(slots + cap * parts * S::SIZE);
         unsigned first = 0;
         StagedPart part[2];
@@ -492,7 +492,7 @@ struct EngineImpl : EngineBase {
         for (int k = 0; k < parts; ++k) {
             const StagedArgs &a = part[k].a;
             CUDIL_LAUNCH(KID_ST_PREHASH, part[k].st,
-                         CUDIL_PAIRED_ON(a.count, sm_count, k_fused_prehash<MODE, PAIR><<<prehash_blocks(a.count * LANES), kPrehashBlock, 0, part[k].st>>>(sk_cache, sk_pitch, mr, items, q, a.first, a.count)));
+                         CUDIL_PAIRED_ON(a.count, sm_count, k_fused_prehash<MODE, PAIR><<<prehash_blocks(a.count * LANES), kPrehashBlock, 0, part[k].st>>>(sk_cache, sk_pitch, mr, items, q, a.first, a.count, reinterpret_cast<uint4 *>(a.rounds), (unsigned)(kStagedRoundBytes / sizeof(uint4)))));
         }
         for (bool more = true; more;) {
             more = false;
@@ -566,7 +566,7 @@ struct EngineImpl : EngineBase {
             if (rc) return rc;
         } else {
             k_fused_init<<<std::max(1, sm_count * 2), 256, 0, st>>>(q, best, locks, next_nonce, inflight);
-            CUDIL_LAUNCH(KID_ST_PREHASH, st, CUDIL_PAIRED_ON(n, sm_count, k_fused_prehash<MODE, PAIR><<<prehash_blocks(n * LANES), kPrehashBlock, 0, st>>>(sk_cache, sk_pitch, mr, items, q, 0u, (unsigned)n)));
+            CUDIL_LAUNCH(KID_ST_PREHASH, st, CUDIL_PAIRED_ON(n, sm_count, k_fused_prehash<MODE, PAIR><<<prehash_blocks(n * LANES), kPrehashBlock, 0, st>>>(sk_cache, sk_pitch, mr, items, q, 0u, (unsigned)n, nullptr, 0u)));
         }
         launch_persistent(a, variant, st);
         CUDIL_CK_LAUNCH();
@@ -611,11 +611,16 @@ struct EngineImpl : EngineBase {
         if (rc) return rc;
         mr.msgs = d_msgs;
         cudaEvent_t ev = Profiler::get().before(st);
-        VerifyArgs a{pk_cache, pk_pitch, mr, d_sig, (size_t)PM::SIG_BYTES, items, scratch, locks, d_ret, (unsigned)n};  // (best[] keeps the last signing batch's nonces)
+        VerifyArgs a{pk_cache, pk_pitch, mr, d_sig, (size_t)PM::SIG_BYTES, items, scratch, locks, d_ret, (unsigned)n, 0u, 0u};  // (best[] keeps the last signing batch's nonces)
         CUDIL_LAUNCH(KID_FV_CHALLENGE, st, CUDIL_PAIRED_ON(n, sm_count, k_fv_challenge<MODE, PAIR><<<prehash_blocks(n * LANES), kPrehashBlock, 0, st>>>(a)));
-        const unsigned wb = n <= 8u * (size_t)sm_count ? 1u : 4u;  // warps per block
-        CUDIL_LAUNCH(KID_FV_W, st, k_fv_w<MODE><<<blocks_for(n, wb), 32 * wb, wb * VerifyRow<MODE>::WARP, st>>>(a));
-        CUDIL_LAUNCH(KID_FV_FINAL, st, CUDIL_PAIRED_ON(n, sm_count, k_fv_final<MODE, PAIR><<<blocks_for(n * LANES, kPrehashBlock), kPrehashBlock, 0, st>>>(a)));
+        for (size_t first = 0; first < n; first += kVerifyTurn) {
+            const size_t count = std::min(n - first, kVerifyTurn);
+            a.first = (unsigned)first;
+            a.count = (unsigned)count;
+            const unsigned wb = count <= 8u * (size_t)sm_count ? 1u : 4u;  // warps per block
+            CUDIL_LAUNCH(KID_FV_W, st, k_fv_w<MODE><<<blocks_for(count, wb), 32 * wb, wb * VerifyRow<MODE>::WARP, st>>>(a));
+            CUDIL_LAUNCH(KID_FV_FINAL, st, CUDIL_PAIRED_ON(count, sm_count, k_fv_final<MODE, PAIR><<<blocks_for(count * LANES, kPrehashBlock), kPrehashBlock, 0, st>>>(a)));
+        }
         CUDIL_CK_LAUNCH();
         Profiler::get().after(KID_FUSED_VERIFY, ev, st);
         CUDIL_CK(cudaMemcpyAsync(h_status, q, sizeof(FusedQueue), cudaMemcpyDeviceToHost, st));

@@ -196,14 +196,17 @@ struct MsgRefs {
 // spread over all SMs.
 constexpr int kPrehashBlock = 32;
 
-// Items order[first .. first + count).
+// Items order[first .. first + count).  Also clears the nclear 16-byte units at `clear` (the staged signer's
+// round counters) for the kernels that follow.
 template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kPrehashBlock) k_fused_prehash(const uint8_t *cache, size_t cpitch, MsgRefs mr,
                                                                  uint8_t *items, const FusedQueue *q, unsigned first,
-                                                                 unsigned count) {
+                                                                 unsigned count, uint4 *clear, unsigned nclear) {
     using C = Cache<MODE>;
     using Sp = Shake256<PAIR>;
     constexpr unsigned PER = kPrehashBlock / Sp::LANES;  // items of a block
+    if (blockIdx.x == 0)
+        for (unsigned k = threadIdx.x; k < nclear; k += kPrehashBlock) clear[k] = make_uint4(0u, 0u, 0u, 0u);
     for (unsigned r0 = blockIdx.x * PER; r0 < count; r0 += gridDim.x * PER) {
         const unsigned r = r0 + threadIdx.x / Sp::LANES;
         bool on = r < count;

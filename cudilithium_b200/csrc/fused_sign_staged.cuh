@@ -24,7 +24,7 @@
 
 namespace cudil {
 
-// Counters of one round; they go up zeroed with the batch's metadata.
+// Counters of one round; the prehash kernel clears them.
 struct StagedRound {
     unsigned npend;     // pending items listed
     unsigned depth;     // attempts of each; the first `extra` listed have one more
@@ -41,6 +41,7 @@ struct StagedAttempt {
 };
 
 constexpr int kStagedMaxRounds = 40;
+constexpr size_t kStagedRoundBytes = kStagedMaxRounds * sizeof(StagedRound);  // of one part
 constexpr unsigned kStagedMaxDepth = 64;
 constexpr unsigned kStagedPending = 0xFFFFFFFFu, kStagedNoNonce = 0xFFFFFFFFu;
 

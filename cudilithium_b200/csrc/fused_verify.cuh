@@ -35,8 +35,15 @@ struct VerifyArgs {
     uint8_t *w1;       // VerifyRow::W1 bytes per signature
     unsigned *status;  // 0 = no check failed
     int *ret;
-    unsigned n;  // signatures
+    unsigned n;             // signatures
+    unsigned first, count;  // those of one launch of k_fv_w and k_fv_final, first's w1 at the scratch's start
 };
+
+// Signatures whose packed w1' the scratch holds at a time (200 MB for Dilithium2, 270 MB for the others); a
+// larger batch runs k_fv_w and k_fv_final in turns.  The bound keeps an engine's memory per item from
+// growing by the size of a w1' (768 or 1024 bytes to the 164 an item takes); turns of this size are hundreds
+// of waves of blocks, so their ends cost nothing.
+constexpr size_t kVerifyTurn = size_t(1) << 18;
 
 // Word w (0..7) of the 32 bytes of c~ at s, which may start at any byte.
 __device__ __forceinline__ uint32_t ctilde_word(const uint8_t *s, int w) {
@@ -96,7 +103,8 @@ __global__ void __launch_bounds__(kBlock, MODE == 5 ? 5 : 6) k_fv_w(VerifyArgs a
     g.sm = zh + (L + 1) * N + half * NTT_SMEM_WORDS;
     uint32_t *hbits = reinterpret_cast<uint32_t *>(zh + (L + 1) * N + 2 * NTT_SMEM_WORDS) + 8 * half;
     const unsigned nwarps = gridDim.x * (blockDim.x >> 5);
-    for (unsigned it = blockIdx.x * (blockDim.x >> 5) + warp; it < a.n; it += nwarps) {
+    for (unsigned u = blockIdx.x * (blockDim.x >> 5) + warp; u < a.count; u += nwarps) {
+        const unsigned it = a.first + u;
         const unsigned key = a.mr.key_idx[it];
         const bool key_ok = bc_ok(key < a.mr.nkeys, BC_VERIFY_KEY);
         const uint8_t *row = a.cache + (size_t)(key_ok ? key : 0u) * a.cpitch;
@@ -151,7 +159,7 @@ __global__ void __launch_bounds__(kBlock, MODE == 5 ? 5 : 6) k_fv_w(VerifyArgs a
         if (lane == 0) a.status[it] = bad ? 1u : 0u;
         if (bad) continue;  // rejected whatever the hash says
         const int32_t *mat = reinterpret_cast<const int32_t *>(row + C::PK_MAT), *t1 = reinterpret_cast<const int32_t *>(row + C::PK_T1);
-        uint8_t *w1out = a.w1 + (size_t)it * V::W1;
+        uint8_t *w1out = a.w1 + (size_t)u * V::W1;
 #pragma unroll 1
         for (int i = half; i < K; i += 2) {  // K is even
             // the poly's hint bitmap (positions were checked above)
@@ -188,13 +196,13 @@ __global__ void __launch_bounds__(kPrehashBlock) k_fv_final(VerifyArgs a) {
     using V = VerifyRow<MODE>;
     using Sp = Shake256<PAIR>;
     constexpr unsigned PER = kPrehashBlock / Sp::LANES;
-    for (unsigned u0 = blockIdx.x * PER; u0 < a.n; u0 += gridDim.x * PER) {
+    for (unsigned u0 = blockIdx.x * PER; u0 < a.count; u0 += gridDim.x * PER) {
         const unsigned u = u0 + threadIdx.x / Sp::LANES;
-        const bool on = u < a.n;
+        const bool on = u < a.count;
         if (!PAIR && !on) continue;
-        const unsigned it = on ? u : 0u;
+        const unsigned it = a.first + (on ? u : 0u);
         const uint8_t *s = a.sig + (size_t)it * a.sig_pitch;
-        TwoPart src{a.items + (size_t)it * C::ITEM_BYTES, 8, a.w1 + (size_t)it * V::W1, PM::W1PACKED_BYTES};
+        TwoPart src{a.items + (size_t)it * C::ITEM_BYTES, 8, a.w1 + (size_t)(it - a.first) * V::W1, PM::W1PACKED_BYTES};
         Sp sp;
         sp.hash(src, CRHBYTES + PM::W1PACKED_BYTES, on);
         bool eq = true;
