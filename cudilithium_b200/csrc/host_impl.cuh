@@ -49,6 +49,21 @@ inline int current_sm_count() {
     return sms;
 }
 
+// Whether a kernel of the current device may write at p, an output pointer of a device call: only the
+// device's own memory (*own).  Pinned host memory, managed memory and another GPU's memory are left to
+// the copy functions, which reach what a kernel may not.  Pageable host memory is refused, except where the
+// device can access it.
+inline int check_device_output(const void *p, bool *own) {
+    cudaPointerAttributes a{};
+    int dev = 0, pageable = 0;
+    CUDIL_CK(cudaGetDevice(&dev));
+    CUDIL_CK(cudaPointerGetAttributes(&a, p));
+    *own = a.type == cudaMemoryTypeDevice && a.device == dev;
+    if (a.type != cudaMemoryTypeUnregistered) return CUDIL_OK;
+    CUDIL_CK(cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev));
+    return pageable ? CUDIL_OK : CUDIL_ERR_INVALID;
+}
+
 // A launch of a kernel template on <..., PAIR> with LANES threads per item: pairs of threads per hash state
 // where `items` are few (keccak_pairs).
 #define CUDIL_PAIRED_ON(items, sms, ...)                \
@@ -83,6 +98,12 @@ struct Impl {
         if (n == 0) return CUDIL_OK;
         if (!pk || !sk || !pool || pitch < LY::ref_keypair_row() || misaligned(pool, pitch) || n > (size_t)INT_MAX / 64)
             return CUDIL_ERR_INVALID;
+        bool pk_own = false, sk_own = false;
+        if (out_kind == cudaMemcpyDeviceToDevice) {
+            int rc = check_device_output(pk, &pk_own);
+            if (!rc) rc = check_device_output(sk, &sk_own);
+            if (rc) return rc;
+        }
         const int nn = (int)n;
         if (seeds) CUDIL_CK(cudaMemcpy2DAsync(pool + LY::KP_SK + PM::SK_TR, pitch, seeds, SEEDBYTES, SEEDBYTES, n, in_kind, st));
         CUDIL_LAUNCH(KID_KP_SEED, st, k_kp_seed<MODE><<<blocks_for(n, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, nn, (unsigned long long)rand_index, seeds ? 1 : 0));
@@ -95,7 +116,7 @@ struct Impl {
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_KP_TR, st, CUDIL_PAIRED(n, k_kp_tr<MODE, PAIR><<<blocks_for(n * LANES, kItemBlock), kItemBlock, 0, st>>>(pool, pitch, nn)));
         CUDIL_CK_LAUNCH();
-        if (out_kind == cudaMemcpyDeviceToDevice && (((uintptr_t)pk | (uintptr_t)sk) & 3u) == 0u) {
+        if (pk_own && sk_own && (((uintptr_t)pk | (uintptr_t)sk) & 3u) == 0u) {
             CUDIL_LAUNCH(KID_KP_OUT, st, k_kp_out<MODE><<<(unsigned)n, kBlock, 0, st>>>(pool, pitch, pk, sk));
             CUDIL_CK_LAUNCH();
             return CUDIL_OK;
