@@ -281,6 +281,14 @@ struct EngineImpl : EngineBase {
         return CUDIL_OK;
     }
 
+    // A batch's metadata goes up from the engine's staging buffer, which the next call rewrites: a batch in a
+    // captured graph would read some later call's lengths and key indices at its replay.
+    static int refuse_capture(cudaStream_t st) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        CUDIL_CK(cudaStreamIsCapturing(st, &cs));
+        return cs == cudaStreamCaptureStatusNone ? CUDIL_OK : CUDIL_ERR_INVALID;
+    }
+
     // ------------------------------------------------------------ metadata upload
     // Checks the batch's metadata and queues its upload; m gets the device arrays (and the caller's
     // buffers).  An order that is the identity -- every batch of equal lengths -- does not travel.
@@ -542,7 +550,8 @@ struct EngineImpl : EngineBase {
             out = static_cast<uint8_t *>(pa.devicePointer);
         }
         MsgRefs mr{};
-        int rc = upload_meta(mr, off, mlen, key, n, n_sk, msgs_bytes, st, rho_seed, rho_counter);
+        int rc = refuse_capture(st);
+        if (!rc) rc = upload_meta(mr, off, mlen, key, n, n_sk, msgs_bytes, st, rho_seed, rho_counter);
         if (rc) return rc;
         mr.msgs = d_msgs;
         mr.rhoprime = d_rhop;
@@ -607,7 +616,8 @@ struct EngineImpl : EngineBase {
         }
         if (((uintptr_t)d_msgs) & 7u) return CUDIL_ERR_INVALID;
         MsgRefs mr{};
-        int rc = upload_meta(mr, off, mlen, key, n, n_pk, msgs_bytes, st);
+        int rc = refuse_capture(st);
+        if (!rc) rc = upload_meta(mr, off, mlen, key, n, n_pk, msgs_bytes, st);
         if (rc) return rc;
         mr.msgs = d_msgs;
         cudaEvent_t ev = Profiler::get().before(st);

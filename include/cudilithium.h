@@ -212,7 +212,8 @@ int cudil_ntt_mul(const int32_t *d_a, const int32_t *d_b, int32_t *d_out, size_t
  *          memory or pinned host memory: in host memory a round's signatures are written over
  *          PCIe when the round ends, so the download overlaps the rest (pageable host memory:
  *          CUDIL_ERR_INVALID).  Asynchronous on `stream`; one batch in flight
- *          per engine (calls on one engine must be ordered on one stream).
+ *          per engine (calls on one engine must be ordered on one stream).  A stream that is being
+ *          captured is refused (CUDIL_ERR_INVALID, nothing queued).
  * last_status: attempts and error flags of the last completed batch (valid after sync);
  *          returns CUDIL_ERR_TIMEOUT if a device-side loop hit its bound (cudil_engine_set_limits).
  *          Error bits: 1 = a per-item publication-lock wait gave up (that attempt's signature is
