@@ -10,8 +10,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <numeric>
-#include <vector>
+#include <new>
 
 #include <cuda_runtime.h>
 
@@ -20,6 +19,7 @@
 #include "fused_sign_staged.cuh"
 #include "fused_verify.cuh"
 #include "host_impl.cuh"
+#include "length_order.cuh"
 #include "profiling.cuh"
 
 namespace cudil {
@@ -39,6 +39,7 @@ struct EngineBase {
     // a batch's metadata (device, the queue block first) and its pinned staging:
     // [FusedQueue | off | key | mlen | order], each array as long as the batch
     uint8_t *d_meta = nullptr, *h_stage = nullptr;
+    unsigned *h_order = nullptr;    // second array of the ordering by length
     FusedQueue *q = nullptr;  // = d_meta
     FusedQueue *h_status = nullptr; // D2H copy of the queue after a batch
     cudaEvent_t stage_ev = nullptr; // recorded after a batch's metadata upload from h_stage
@@ -176,6 +177,7 @@ struct EngineImpl : EngineBase {
             cudaMalloc(&d_meta, stage_bytes(mi)) != cudaSuccess || cudaMallocHost(&h_stage, stage_bytes(mi)) != cudaSuccess ||
             cudaMallocHost(&h_status, sizeof(FusedQueue)) != cudaSuccess)
             return ::cudil::cudil_record_cuda_error(cudaGetLastError(), __FILE__, __LINE__);
+        if (mi && !(h_order = new (std::nothrow) unsigned[mi])) return CUDIL_ERR_INVALID;
         std::memset(h_status, 0, sizeof(FusedQueue));
         CUDIL_CK(cudaEventCreateWithFlags(&stage_ev, cudaEventDisableTiming));
         CUDIL_CK(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
@@ -198,6 +200,7 @@ struct EngineImpl : EngineBase {
         cudaFree(inflight);
         cudaFree(d_meta);
         cudaFree(scratch);
+        delete[] h_order;
         if (h_stage) cudaFreeHost(h_stage);
         if (h_status) cudaFreeHost(h_status);
         if (stage_ev) cudaEventDestroy(stage_ev);
@@ -319,8 +322,7 @@ struct EngineImpl : EngineBase {
         }
         size_t bytes = kStageHead + n * (sizeof(unsigned long long) + 2 * sizeof(unsigned));
         if (!descending) {
-            std::iota(ho, ho + n, 0u);
-            std::stable_sort(ho, ho + n, [&](unsigned a, unsigned b) { return hm[a] > hm[b]; });
+            order_longest_first(ho, h_order, hm, n);
             bytes += n * sizeof(unsigned);
         }
         CUDIL_CK(cudaMemcpyAsync(d_meta, h_stage, bytes, cudaMemcpyHostToDevice, st));
