@@ -67,8 +67,8 @@ static_assert(kTwiddles.zeta[255] == 1976782, "zeta table");
 // congruent to b * w mod q and lies in (-q/2, 3q/2) for any 32-bit b -- one high multiply and two
 // low multiply-adds instead of montmul's two high multiplies, one low multiply and a subtraction.
 // The transforms built on it give the reference's residues (not its representatives), so they
-// serve every path whose outputs are reduced before use; key generation and the NTT microbench,
-// whose outputs are compared representative for representative, keep the Montgomery transforms.
+// serve every path whose outputs are reduced before use; the NTT product, whose outputs are compared
+// representative for representative, keeps the Montgomery transforms.
 __host__ __device__ constexpr int32_t shoup_quot(int32_t w) {
     const int64_t num = (int64_t)w * (int64_t)(1ll << 32);
     int64_t qq = num / Q;

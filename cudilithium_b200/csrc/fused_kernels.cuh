@@ -59,7 +59,6 @@ struct Cache {
 
 // Queue / status block shared by the engine kernels (one per engine, device memory).
 struct FusedQueue {
-    unsigned long long next_ticket;
     unsigned int done_items;
     // bit 0: a bounded publication-lock wait gave up; bit 1: an item reached its nonce limit (with no
     // accepted nonce its signature row is not written); bit 2: an asynchronous signer block gave up
@@ -243,19 +242,17 @@ __global__ void __launch_bounds__(kPrehashBlock) k_fused_prehash(const uint8_t *
     }
 }
 
-// Resets the queue and, for signing, the per-item winner state of q->n items (n set by the host
-// copy; best == nullptr: queue only).
+// Resets the queue and the per-item winner state of q->n items (n set by the host copy).
 static __global__ void k_fused_init(FusedQueue *q, unsigned *best, unsigned *locks, unsigned *next_nonce,
                                     unsigned *inflight) {
     const unsigned n = q->n;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; best && i < n; i += gridDim.x * blockDim.x) {
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         best[i] = 0xFFFFFFFFu;
         locks[i] = 0u;
-        if (next_nonce) next_nonce[i] = 0u;
-        if (inflight) inflight[i] = 0u;
+        next_nonce[i] = 0u;
+        inflight[i] = 0u;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        q->next_ticket = 0;
         q->done_items = 0;
         q->error = 0;
         q->attempts = 0;

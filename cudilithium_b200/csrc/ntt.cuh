@@ -4,23 +4,24 @@
 // Arithmetic: the same Cooley-Tukey (forward) and Gentleman-Sande (inverse) butterfly network
 // as the reference (src/ntt.cu:58-207, include/ntt.cuh:74-306), whose inverse ends with a Montgomery
 // multiplication of every coefficient by f = 41978 (src/ntt.cu:201-205).  Two forms:
-//   ntt16 / intt16   every butterfly is a +/- montmul(zeta, b) with the reference's Montgomery
+//   ntt16_tw<false> / intt16_tw<false>
+//                    every butterfly is a +/- montmul(zeta, b) with the reference's Montgomery
 //                    zetas, so outputs are bit-identical to the reference's radix-8 kernels and to
-//                    the CPU oracle (key generation, the NTT microbench);
+//                    the CPU oracle (the NTT product);
 //   ntt16s / intt16s the butterflies multiply by the true zetas with precomputed quotients
-//                    (shoup_mul): the same residues mod q in other representatives, for the
-//                    signing and verification paths, which reduce every output before use and
+//                    (shoup_mul): the same residues mod q in other representatives, for key
+//                    generation, signing and verification, which reduce every output before use and
 //                    carry f in an operand of the products (scale_f).
 //
 // Layout (radix-16, one shared-memory transpose per transform instead of two):
 //   forward: in  x[i] = a[t + 16 i]  -> levels len 128..16 in registers
 //            transpose through shared memory (17-word padded rows, conflict-free)
 //            levels len 8..1 in registers -> out x[i] = a_hat[16 t + i]
-//   inverse: in  x[i] = a_hat[16 t + i] -> levels len 1..8, transpose, len 16..128, * f
+//   inverse: in  x[i] = a_hat[16 t + i] -> levels len 1..8, transpose, len 16..128
 //            -> out x[i] = a[t + 16 i]
-// so NTT -> pointwise -> invNTT needs no extra exchange, NTT-domain data is stored in natural
-// order with 64 contiguous bytes per thread (128-bit accesses) and time-domain data with 16
-// consecutive words per i across the group (coalesced).
+// so NTT -> pointwise -> invNTT needs no extra exchange.  NTT-domain polynomials are stored by 16-byte
+// chunks (ntt_at4 below), except s1_hat of key generation, whose reader walks it coefficient by
+// coefficient; time-domain data has 16 consecutive words per i across the group (coalesced).
 #pragma once
 
 #include <cstdint>
@@ -160,13 +161,6 @@ __device__ __forceinline__ void ntt16_tw(int32_t (&x)[16], int32_t *sm, unsigned
 }
 
 // Forward NTT; sm = this group's NTT_SMEM_WORDS-word region, gmask = this group's lanes.
-template <bool S>
-__device__ __forceinline__ void ntt16_t(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) {
-    int2 tw[16];
-    load_tw16(tw, (S ? g_group_tw_s : g_group_tw).fwd, t);
-    ntt16_tw<S>(x, sm, gmask, t, tw);
-}
-
 // Inverse NTT including the final multiplication by f (invntt_tomont), register-local twiddles
 // already loaded (tw = the group position's pairs of GroupTwiddles::inv).  FIN = false leaves the
 // final multiplication out: for inputs that carry the factor already.  Then |x| <= q at the input
@@ -215,22 +209,20 @@ __device__ __forceinline__ void intt16_tw(int32_t (&x)[16], int32_t *sm, unsigne
     }
 }
 
-template <bool S, bool FIN = true>
-__device__ __forceinline__ void intt16_t(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) {
+// Precomputed-quotient transforms: the same residues, cheaper butterflies (key generation, signing,
+// verification and the engine's key caches -- every consumer reduces the outputs before use).  The inverse has
+// no final multiplication: its callers' products carry the factor f (scale_f below).
+__device__ __forceinline__ void ntt16s(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) {
     int2 tw[16];
-    load_tw16(tw, (S ? g_group_tw_s : g_group_tw).inv, t);
-    intt16_tw<S, FIN>(x, sm, gmask, t, tw);
+    load_tw16(tw, g_group_tw_s.fwd, t);
+    ntt16_tw<true>(x, sm, gmask, t, tw);
 }
 
-// Montgomery transforms: the reference's exact output representatives (key generation, the NTT
-// microbench).
-__device__ __forceinline__ void ntt16(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { ntt16_t<false>(x, sm, gmask, t); }
-__device__ __forceinline__ void intt16(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { intt16_t<false>(x, sm, gmask, t); }
-// Precomputed-quotient transforms: the same residues, cheaper butterflies (signing, verification,
-// the engine's key caches -- every consumer reduces the outputs before use).  The inverse has no final
-// multiplication: its callers' products carry the factor f (scale_f below).
-__device__ __forceinline__ void ntt16s(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { ntt16_t<true>(x, sm, gmask, t); }
-__device__ __forceinline__ void intt16s(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) { intt16_t<true, false>(x, sm, gmask, t); }
+__device__ __forceinline__ void intt16s(int32_t (&x)[16], int32_t *sm, unsigned gmask, int t) {
+    int2 tw[16];
+    load_tw16(tw, g_group_tw_s.inv, t);
+    intt16_tw<true, false>(x, sm, gmask, t, tw);
+}
 
 // The inverse transform's factor f, put into one operand of the products it will transform -- A_hat
 // when it is sampled, c_hat once per challenge -- instead of into all 256 outputs of every inverse

@@ -33,7 +33,6 @@ enum KernelId : int {
     KID_ALU_PEAK,
     KID_FUSED_SIGN,
     KID_FUSED_VERIFY,
-    KID_FUSED_SCHED,
     KID_CACHE_SK,
     KID_CACHE_PK,
     KID_SIG_CHECK,
@@ -57,7 +56,7 @@ inline const char *kernel_name(int id) {
         "k_kp_seed", "k_kp_s", "k_kp_s1", "k_kp_t", "k_kp_tr", "k_sign_setup", "k_expand_a", "k_sign_unpack_ntt",
         "k_sign_expand_mask", "k_sign_compute_w", "k_sign_challenge", "k_sign_reject", "k_sig_copy",
         "k_verify_setup", "k_verify_w", "k_verify_final", "k_ntt_mul", "k_alu_peak",
-        "sign batch (engine)", "verify batch (engine)", "k_fused_sched", "k_cache_sk", "k_cache_pk",
+        "sign batch (engine)", "verify batch (engine)", "k_cache_sk", "k_cache_pk",
         "k_sig_check", "k_sk_check", "k_derive_rhoprime",
         "k_fused_prehash", "k_st_claim", "k_st_mask", "k_st_w", "k_st_challenge", "k_st_reject",
         "k_fv_challenge", "k_fv_w", "k_fv_final", "k_kp_out"};
