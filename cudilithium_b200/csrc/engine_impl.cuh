@@ -51,8 +51,8 @@ struct EngineBase {
     size_t scratch_bytes = 0;
     int sign_grid = 0, verify_grid = 0, reject_grid = 0;
     size_t sign_smem = 0;
-    // signer kernel: 0 = phased k_fused_sign (block-wide Keccak / NTT phases) with the engine's
-    // block size; 1..4 = asynchronous k_fused_sign_async with (threads, slots) per block of
+    // signer kernel: 0 = staged rounds, finished by the phased k_fused_sign (block-wide Keccak / NTT
+    // phases, the engine's block size) on what they leave; 1..4 = asynchronous k_fused_sign_async with (threads, slots) per block of
     // (256, 64), (512, 128), (640, 160), (768, 192); 5 = phased with one wide block per SM (512
     // threads, 384 for Dilithium5, whose wider phase buffers allow no more)
     int sign_kernel = 0;
@@ -425,9 +425,10 @@ struct EngineImpl : EngineBase {
     // each), and nothing is signed before.  In two parts the shorter messages are signed on a second stream
     // while the longest are still being hashed.  The split is the eighth of the batch that ends soonest by
     // this model: hashing as above, signing 0.3 ms (rounds' latency) and kSignUs per item.
-    // 16 384 Dilithium3 messages of 32 B..64 KiB: 5.78 ms whole, 4.50 ms in two parts.  Batches of
-    // equal lengths stay whole: two halves on two streams gained 5% alone and lost 4% where batches already
-    // run on two engines' streams.
+    // 16 384 Dilithium3 messages of 32 B..64 KiB: 5.78 ms whole, 4.50 ms in two parts.  A batch without an
+    // order array stays whole.  That is every batch of equal lengths -- two halves on two streams gained 5%
+    // alone and lost 4% where batches already run on two engines' streams -- and also a mixed one that arrives
+    // longest first, which the two parts would serve too.
     size_t staged_split(const MsgRefs &mr, const unsigned *mlen, size_t n) const {
         if (!mr.order) return 0;
         constexpr double kSignUs = MODE == 2 ? 0.10 : (MODE == 3 ? 0.18 : 0.25), kRoundsUs = 300.0, kBlockUs = 3.5;

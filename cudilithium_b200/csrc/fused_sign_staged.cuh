@@ -10,7 +10,7 @@
 //   k_st_challenge  c~ = H(mu || w1) and SampleInBall, one thread per attempt
 //   k_st_reject     rejection checks and hints, one warp per attempt; an accepted attempt lowers its
 //                   item's best nonce
-// The host enqueues as many rounds as the acceptance rate calls for (EngineImpl::staged_rounds) without
+// The host enqueues as many rounds as the acceptance rate calls for (EngineImpl::sign_staged) without
 // waiting for any of them; the counts stay on the device, and a round that finds nothing pending returns
 // at once.  k_fused_sign runs last and finishes the items, if any, that the enqueued rounds left.
 //
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(256) k_st_claim(StagedArgs a, int r, bool clai
 
 // The staged signer keeps a packed y polynomial (ExpandMask's output, gamma1 - y in Z_BITS-bit fields) in the
 // order its readers load it.  Sixteen fields are YW = Z_BITS / 2 words; word k of each sixteen, for four
-// consecutive sixteens, makes a 16-byte chunk, and the chunks of four sixteens follow one another: word 
+// consecutive sixteens, makes a 16-byte chunk, and the chunks of four sixteens follow one another: word
 // YW i + k of the stream is at y_word(i, k).  Position t's fields t + 16 i sit in words k and k + 1 of every
 // sixteen, k = Z_BITS t / 32: eight 128-bit loads read a position's sixteen fields instead of 32 word loads.
 template <int MODE>
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kItemBlock) k_st_challenge(StagedArgs a, int r
 // rejection job: r0 pairs (r0 replaces w0 in the slot, for the hints), z pairs, ct0 pairs with the hints.
 // Both groups of the warp follow the same control flow, and a rejection ends the attempt.
 //
-// A one-warp block takes `per` attempts (one to eleven steps each).  per = 2: each group transforms one
+// A one-warp block takes `per` attempts (up to NSTEP = 6, 9 or 12 steps each).  per = 2: each group transforms one
 // attempt's c, once for both groups; per = 1, in rounds with fewer attempts than resident warps: both groups
 // transform the same c.  c_hat waits in shared memory, which leaves the registers to hold a step's w0 in
 // flight across its transform.  Resident blocks that draw tickets measured slower in rounds of one or two

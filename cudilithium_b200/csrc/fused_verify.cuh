@@ -9,8 +9,8 @@
 // One persistent kernel did the three before, a block's 30 to 200 signatures at a time: its hashing phases
 // kept a few of the block's warps busy, and a signature's polynomials went one after the other through one
 // group.  65 536 Dilithium5 signatures over 256 resident keys: 1.37 ms, 1.00 ms in these kernels; 10 000
-// Dilithium2 signatures with as many fresh keys 537 us (key
-// caches included), 459 us; 33 Dilithium3 signatures 118 us, 102 us.
+// Dilithium2 signatures with as many fresh keys 537 us (key caches included), 459 us; 33 Dilithium3
+// signatures 118 us, 99 us.
 #pragma once
 
 #include "fused_kernels.cuh"

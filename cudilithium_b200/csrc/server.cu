@@ -97,8 +97,7 @@ struct Slot {
 
     size_t device_bytes = 0;
 
-    // record = false: a warm-up batch (graph capture, first-touch of buffers) whose results are
-    // dropped.
+    // record = false: a warm-up batch (first touch of buffers) whose results are dropped.
     int run_batch(bool record = true) {
         const cudil_params &p = tr->prm[mode_index(mode)];
         const size_t n = batch.size();
