@@ -539,8 +539,8 @@ def run_gpu(args) -> dict | None:
     # ---- e2e: host buffers in, host signatures out, through the engine API.  The messages and
     # the secret keys go up on a copy stream, the keys in --e2e-chunks chunks; each chunk's cache
     # rows are built on the compute stream behind its own copy (update_secret_keys), so the copies
-    # of later chunks overlap the builds of earlier ones.  The signer writes every signature straight
-    # into the pinned host output as soon as it is found (PCIe writes during the kernel), so the
+    # of later chunks overlap the builds of earlier ones.  The signer writes a round's signatures
+    # straight into the pinned host output when the round ends (PCIe writes by a kernel), so the
     # download overlaps the signing.  The timed region spans all copies, builds and the signing.
     h_m = pinned(B * MLEN)
     h_m.numpy()[:] = m_host.reshape(-1)
