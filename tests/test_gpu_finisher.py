@@ -149,3 +149,25 @@ def test_phased_kernel_signs_whole_batches(cuda_ok, oracle, mode, threads):
         assert np.array_equal(rows, want) and np.array_equal(eng.last_nonces(n) + 1, att)
         assert eng.last_phases()["total"] > 0
     eng.close()
+
+
+def test_bounds_checked_build_finds_nothing(cuda_ok):
+    """The tests above in the bounds-checked build: the same results and a clean error word."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    root = Path(__file__).resolve().parents[1]
+    lib = root / "cudilithium_b200" / "libcudilithium_b200_bc.so"
+    if not lib.exists():
+        subprocess.run([sys.executable, str(root / "cudilithium_b200" / "build.py"), "--bounds-check"], check=True)
+    run = ("import ctypes, sys, pytest\n"
+           f"rc = pytest.main(['-x', '-q', '-p', 'no:cacheprovider', '-k', 'not bounds_checked', {str(Path(__file__))!r}])\n"
+           "from cudilithium_b200._lib import LIB_PATH, lib\n"
+           "err = ctypes.c_uint32(0xFFFFFFFF)\n"
+           "assert lib.cudil_bounds_check_status(ctypes.byref(err), 1) == 0\n"
+           "print('tests', int(rc), LIB_PATH.name, 'error word', err.value)\n")
+    r = subprocess.run([sys.executable, "-c", run], cwd=root, env=dict(os.environ, CUDIL_LIB=str(lib)), capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
+    assert r.stdout.strip().splitlines()[-1] == f"tests 0 {lib.name} error word 0", r.stdout[-2000:]
