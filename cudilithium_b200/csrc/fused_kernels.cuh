@@ -317,26 +317,43 @@ constexpr unsigned kLockSpinLimit = 1u << 22;  // x ~64 ns sleeps
 // number of words): the row's aligned words are put together from two staged ones, and only the bytes before the
 // first and after the last of them are stored singly.  Word stores matter when the output is pinned host memory
 // written over PCIe: 20 000 Dilithium3 signatures 44.5 ms with such rows stored byte by byte, 5.1 ms this
-// way.  Eight words per thread are loaded before they are stored.
+// way.  Eight words per thread are in flight before any is stored.
 template <int BYTES, int NT>
 __device__ __forceinline__ void publish_signature(uint8_t *dst, const uint32_t *src, int t) {
     const unsigned head = (0u - (unsigned)(reinterpret_cast<uintptr_t>(dst))) & 3u;  // bytes before the first aligned word
     const int nfull = (BYTES - (int)head) / 4, tail = (BYTES - (int)head) % 4;
     uint32_t *d = reinterpret_cast<uint32_t *>(dst + head);
-    // aligned word w holds the signature's bytes head + 4 w ..: the end of staged word w, the start of w + 1
+    if (head == 0u) {  // (loads of its own: 0.7% of 65 536 Dilithium2 signatures)
 #pragma unroll 1
-    for (int w0 = 0; w0 < nfull; w0 += 8 * NT) {
-        uint32_t lo[8], hi[8];
+        for (int w0 = 0; w0 < nfull; w0 += 8 * NT) {
+            uint32_t v[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int w = w0 + t + NT * k;
-            lo[k] = w < nfull ? src[w] : 0u;
-            hi[k] = head && w < nfull ? src[w + 1] : 0u;
+            for (int k = 0; k < 8; ++k) {
+                const int w = w0 + t + NT * k;
+                v[k] = w < nfull ? src[w] : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int w = w0 + t + NT * k;
+                if (w < nfull) d[w] = v[k];
+            }
         }
+    } else {
+        // aligned word w holds the signature's bytes head + 4 w ..: the end of staged word w, the start of w + 1
+#pragma unroll 1
+        for (int w0 = 0; w0 < nfull; w0 += 4 * NT) {
+            uint32_t lo[4], hi[4];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int w = w0 + t + NT * k;
-            if (w < nfull) d[w] = __funnelshift_r(lo[k], hi[k], 8u * head);
+            for (int k = 0; k < 4; ++k) {
+                const int w = w0 + t + NT * k;
+                lo[k] = w < nfull ? src[w] : 0u;
+                hi[k] = w < nfull ? src[w + 1] : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int w = w0 + t + NT * k;
+                if (w < nfull) d[w] = __funnelshift_r(lo[k], hi[k], 8u * head);
+            }
         }
     }
     const uint8_t *sb = reinterpret_cast<const uint8_t *>(src);
