@@ -136,6 +136,21 @@ struct EngineImpl : EngineBase {
         return rc;
     }
 
+    // The kernels of a key-cache build run side by side, on one SM too, so they ask for the same split of its
+    // memory between L1 and shared memory.  An SM changes the split only while it is idle: with the driver's
+    // choice, which follows each kernel's own shared memory, ExpandA and the transforms waited for one another:
+    // secret rows of 1024 Dilithium2 keys 151 us, 75 us with one split; public rows of 2048 keys 182 and 96 us.
+    // Three quarters of the memory hold the 24 ExpandA warps that the registers allow; with all of it
+    // verification of 10 000 signatures with fresh keys takes 451 instead of 447 us.
+    static constexpr int kCacheSplit = 75;  // percent
+    int configure_caches() {
+        const void *fns[] = {(const void *)k_cache_sk<MODE>, (const void *)k_expand_a_keys<MODE>, (const void *)k_cache_pk_t1<MODE>,
+                             (const void *)k_cache_pk_tr<MODE, false>, (const void *)k_cache_pk_tr<MODE, true>};
+        for (const void *fn : fns)
+            CUDIL_CK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, kCacheSplit));
+        return CUDIL_OK;
+    }
+
     template <int T>
     int configure() {
         sign_smem = FusedSignSmem<MODE, T>::BYTES;
@@ -161,6 +176,8 @@ struct EngineImpl : EngineBase {
         rc = configure_async();
         if (rc) return rc;
         rc = configure_wide();
+        if (rc) return rc;
+        rc = configure_caches();
         if (rc) return rc;
         device_bytes = required_bytes(mk, mi);
         if (budget && device_bytes > budget) return CUDIL_ERR_BUDGET;
@@ -244,22 +261,32 @@ struct EngineImpl : EngineBase {
         return rc;
     }
 
-    // The unpack / transform of s1, s2, t0 (side stream) and ExpandA (caller's stream, rho read from
-    // the packed keys) are independent and run concurrently; the caller's stream waits for both.
+    // The unpack / transform of s1, s2, t0 and ExpandA (rho read from the packed keys) are independent: the
+    // transforms go to the side stream, beside ExpandA, and the caller's stream waits for both.  Between 4 and 48
+    // of the transforms' blocks per SM the two follow one another instead.  Side by side ExpandA's few warps
+    // then start behind the transforms, and unevenly: 1024 Dilithium2 keys 75 us, one after the other 54, 4096
+    // keys 166 and 144.  Below that the transforms leave the SMs free (repeated builds of 100 keys 37 against
+    // 41 us), above it ExpandA is long enough to even out (6000 keys 199 against 205).
     int build_sk_rows(const uint8_t *d_sk, size_t first, size_t nkeys, cudaStream_t st) {
         const int nn = (int)nkeys;
         uint8_t *rows = sk_cache + first * sk_pitch;
-        CUDIL_CK(cudaEventRecord(fork_ev, st));
-        CUDIL_CK(cudaStreamWaitEvent(side, fork_ev, 0));
-        CUDIL_LAUNCH(KID_CACHE_SK, side,
-                     k_cache_sk<MODE><<<blocks_for(nkeys * (PM::L + 2 * PM::K + 1) * 16), kBlock, 0, side>>>(d_sk, rows, sk_pitch, nn));
+        const unsigned blocks = blocks_for(nkeys * (PM::L + 2 * PM::K + 1) * 16);
+        const bool beside = blocks <= 4u * (unsigned)sm_count || blocks > 48u * (unsigned)sm_count;
+        cudaStream_t ts = beside ? side : st;
+        if (beside) {
+            CUDIL_CK(cudaEventRecord(fork_ev, st));
+            CUDIL_CK(cudaStreamWaitEvent(side, fork_ev, 0));
+        }
+        CUDIL_LAUNCH(KID_CACHE_SK, ts, k_cache_sk<MODE><<<blocks, kBlock, 0, ts>>>(d_sk, rows, sk_pitch, nn));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_EXPAND_A, st,
-                     k_expand_a_keys<MODE><<<blocks_for(nkeys * PM::K * PM::L), kBlock, 0, st>>>(d_sk, PM::SK_BYTES, rows, sk_pitch,
+                     k_expand_a_keys<MODE><<<blocks_for(nkeys * PM::K * PM::L, kItemBlock), kItemBlock, 0, st>>>(d_sk, PM::SK_BYTES, rows, sk_pitch,
                                                                                              C::SK_MAT, nn));
         CUDIL_CK_LAUNCH();
-        CUDIL_CK(cudaEventRecord(join_ev, side));
-        CUDIL_CK(cudaStreamWaitEvent(st, join_ev, 0));
+        if (beside) {
+            CUDIL_CK(cudaEventRecord(join_ev, side));
+            CUDIL_CK(cudaStreamWaitEvent(st, join_ev, 0));
+        }
         return CUDIL_OK;
     }
 
@@ -275,7 +302,7 @@ struct EngineImpl : EngineBase {
                      k_cache_pk_t1<MODE><<<blocks_for(nkeys * PM::K * 16), kBlock, 0, side>>>(d_pk, pk_cache, pk_pitch, nn));
         CUDIL_CK_LAUNCH();
         CUDIL_LAUNCH(KID_EXPAND_A, st,
-                     k_expand_a_keys<MODE><<<blocks_for(nkeys * PM::K * PM::L), kBlock, 0, st>>>(d_pk, PM::PK_BYTES, pk_cache, pk_pitch,
+                     k_expand_a_keys<MODE><<<blocks_for(nkeys * PM::K * PM::L, kItemBlock), kItemBlock, 0, st>>>(d_pk, PM::PK_BYTES, pk_cache, pk_pitch,
                                                                                              C::PK_MAT, nn));
         CUDIL_CK_LAUNCH();
         CUDIL_CK(cudaEventRecord(join_ev, side));
